@@ -18,20 +18,29 @@
 //      scale, and for the certificate |[X | Z]| and the FP64 diagonal
 //      R_aa = |X|^2 - |Z|^2 + left.right.
 //
-// K3s  crt_syrk_kernel  (persistent, one CTA per SM, 18 warps)
+// K3s  crt_syrk_kernel  (persistent, one CTA per SM, 20 warps)
 //      warp 0: TMA producer — 128x128-byte boxes (SWIZZLE_128B) of the A and B
 //              residue matrices into a STAGES-deep ring;
 //      warp 1: TMEM owner + MMA issuer — tcgen05.mma.kind::i8, M=N=128, K=32,
 //              int32 accumulators in a double-buffered TMEM tile;
-//      warps 2-17: epilogue (4 TMEM lane quarters x 4 column groups; four
-//              warps per SM sub-partition hide the TMEM and ALU latency) — per
-//              modulus: TMEM -> registers, reduce to [0, m) with integer
-//              operations, merge each even/odd pair of moduli into a 16-bit
-//              digit mod m_e m_o (two digits per 32-bit word; words of four
-//              moduli parked in TMEM columns 256..511, the last word kept in
-//              registers); per tile: CRT over the digits in FP64 (exact split
-//              constants), scale, add the core correction when it is not
-//              screened out, store the tile and its transpose.
+//      warps 2, 3: the next tile's record (row scales, screen bounds, table) into
+//              shared memory: beside the TMA feed an L2 read takes over a thousand
+//              cycles, and the epilogue makes none;
+//      warps 4-19: epilogue (4 TMEM lane quarters x 4 column groups).  Per modulus
+//              one IMAD.WIDE an entry folds the int32 accumulator, unreduced, into
+//              the open digit's 64-bit sum; three times a tile the digit is reduced
+//              (FP64 quotient) and its CRT weight added to the entry's 64-bit
+//              fraction x / M in TMEM columns 256..511.  A finished tile's scaling,
+//              core correction (when it is not screened out) and stores (the tile and
+//              its transpose) run in four chunks between the next tile's first moduli,
+//              so that the MMAs do not wait for them.
+//      The epilogue's instructions were the limit: reducing every accumulator to its
+//      residue and merging residues in pairs took about 13 instructions per entry and
+//      modulus (IMAD.HI issues at a quarter rate), spilled registers went through L2,
+//      and the MMAs stood still during the final phase.  Z=70 table (kdim 1024): 2.88
+//      ms before, 2.35 ms now; N=2112 table (kdim 2176): 2.58 and 2.41 ms.
+//      The fraction's rounding, 2^-64 of M, is 2^-50 or less of an entry's Schwarz
+//      scale at the default widths, some 4000 times below the split's own error.
 //      Every mbarrier wait is bounded; on timeout the kernel records
 //      RKB_ETIMEDOUT in *status and every role drains and returns.
 #include <cuda.h>
@@ -738,10 +747,25 @@ constexpr int STAGES = 5;
 constexpr int STAGE_BYTES = (BM + BN) * BKB;  // 32 KB
 constexpr int EPI_WARPS = 16;                 // 4 TMEM lane quarters x 4 column groups
 constexpr int EPI_COLS = BN / (EPI_WARPS / 4);  // columns per epilogue thread
-constexpr int THREADS = 32 * (2 + EPI_WARPS);
-constexpr int STG_LD = 9;   // doubles per staged row (8 + pad)
+constexpr int CTL_WARPS = 4;                  // one warpgroup: TMA, MMA, tile records (rows, columns)
+constexpr int THREADS = 32 * (CTL_WARPS + EPI_WARPS);
+// 640 threads launch with 96 registers each; the control warpgroup keeps 32, which
+// gives the four epilogue warpgroups 112 (4 x 112 + 32 = 5 x 96).
+constexpr int CTL_REGS = 32, EPI_REGS = 112;
+constexpr int NACC = 2;     // int32 accumulator tiles in TMEM (128 columns each; the rest parks digits 0 and 1)
+constexpr int NDIG = 3;     // CRT digits, of up to four moduli each
+constexpr int FC = 8;       // columns per chunk of the final phase
+constexpr int STG_LD = FC + 1;  // doubles per staged row
+// What the epilogue needs to know of a tile, fetched ahead of it by two control warps.
+struct __align__(16) TileInfo {
+    double rs_row[BM], rs_col[BN];         // row scales
+    double row_max[4][3], col_max[4][3];   // screen bounds of each 32-row / 32-column group
+    double *out;                           // the tile's table
+    long row0;
+    int n, ti, tj, pad;
+};
 constexpr size_t SMEM_BYTES = 1024 /*align slack*/ + (size_t)STAGES * STAGE_BYTES +
-                              (size_t)EPI_WARPS * 32 * STG_LD * sizeof(double) + 256 /*barriers*/;
+                              (size_t)EPI_WARPS * 32 * STG_LD * sizeof(double) + 2 * sizeof(TileInfo) + 256 /*barriers*/;
 constexpr long long WAIT_LIMIT = 4000000000LL;  // clock64 ticks (~2 s)
 constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                            ((uint32_t)(BM >> 4) << 24);
@@ -756,12 +780,12 @@ struct CrtArgs {
     double *out;
     int *status;
     int n_mod;
-    int mod[MAXMOD];
-    uint32_t magic[MAXMOD];   // floor(2^32 / m) + 1
-    uint32_t bias[MAXMOD];    // m * 2^18: makes every accumulator nonnegative
-    uint32_t pinv[MAXMOD / 2];  // m_2p^-1 mod m_2p+1
-    double f_hi[MAXMOD], f_lo[MAXMOD];  // per merged digit
-    double M;
+    // The CRT in two steps. Consecutive moduli (up to dig_end[g]) make a digit modulo
+    // D_g < 2^32: d_g = sum_i x_i coef_i mod D_g. Then x / M = sum_g d_g F_g mod 1 with
+    // F_g = f_hi 2^-32 + f_mid 2^-64 + f_lo 2^-96.
+    int dig_end[NDIG], coef[MAXMOD], D[NDIG], f_hi[NDIG], f_mid[NDIG], f_lo[NDIG];
+    double inv_D[NDIG], inv_D32[NDIG];  // 1/D, 2^32/D
+    double M;  // the product of the moduli, times 2^-32
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -783,15 +807,17 @@ __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
 // Bounded wait: false (and status = ETIMEDOUT) after WAIT_LIMIT clock ticks,
 // or as soon as another role has recorded a failure.
 __device__ __forceinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, int *status) {
-    long long t0 = clock64();
-    while (!mbar_try(bar, parity)) {
+    const long long t0 = clock64();
+    while (true) {
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i)  // the status word is an L2 read: looked at between tries only
+            if (mbar_try(bar, parity)) return true;
         if (*(volatile int *)status != 0) return false;
         if (clock64() - t0 > WAIT_LIMIT) {
             atomicExch(status, (int)RKB_ETIMEDOUT);
             return false;
         }
     }
-    return true;
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *status) {
     if (mbar_try(bar, parity)) return true;
@@ -834,43 +860,56 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, int (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                  : "r"(taddr));
 }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t *v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::
-            "r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-        : "memory");
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, int (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const int (&v)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
+                 "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const int (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-template <int NMOD>
+// Exact int -> double by the 2^52 trick (ALU and FP64 pipes; cvt runs at a quarter of their rate).
+__device__ __forceinline__ double int_to_double(int v) {
+    return __dadd_rn(__hiloint2double(0x43300000, (int)((uint32_t)v ^ 0x80000000u)),
+                     -(4503599627370496.0 + 2147483648.0));
+}
+__device__ __forceinline__ double uint_to_double(uint32_t v) {
+    return __dadd_rn(__hiloint2double(0x43300000, (int)v), -4503599627370496.0);
+}
+// acc mod D nearest zero. |acc| < 2^59 and D < 2^32, so the quotient's rounding error is
+// far below 1 and |result| <= D/2 (1 + 2^-25).
+__device__ __forceinline__ int mod_near(long long acc, int D, double inv_D, double inv_D32) {
+    const double q = __fma_rn(int_to_double((int)(acc >> 32)), inv_D32, __dmul_rn(uint_to_double((uint32_t)acc), inv_D));
+    return (int)((uint32_t)acc - (uint32_t)__double2loint(__dadd_rn(q, 6755399441055744.0)) * (uint32_t)D);
+}
+
 __global__ void __launch_bounds__(THREADS, 1)
     crt_syrk_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                     const __grid_constant__ CrtArgs p) {
-    constexpr int PARKED = (NMOD - 1) >> 2;  // groups of four moduli parked in TMEM (0..2)
-    constexpr int LASTG = PARKED;            // group kept in registers
-    constexpr int NDIG = (NMOD + 1) / 2;     // merged CRT digits
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char *ring = base;
     double *stage_out = (double *)(ring + (size_t)STAGES * STAGE_BYTES);
-    uint64_t *bars = (uint64_t *)(stage_out + EPI_WARPS * 32 * STG_LD);
-    uint64_t *full = bars, *empty = bars + STAGES, *accf = bars + 2 * STAGES, *acce = accf + 2;
-    uint32_t *tmem_slot = (uint32_t *)(acce + 2);
+    TileInfo *info = (TileInfo *)(stage_out + EPI_WARPS * 32 * STG_LD);
+    uint64_t *bars = (uint64_t *)(info + 2);
+    uint64_t *full = bars, *empty = full + STAGES, *accf = empty + STAGES, *acce = accf + NACC;
+    uint64_t *inff = acce + NACC, *infe = inff + 2;
+    uint32_t *tmem_slot = (uint32_t *)(infe + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -878,9 +917,13 @@ __global__ void __launch_bounds__(THREADS, 1)
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
-        for (int b = 0; b < 2; ++b) {
+        for (int b = 0; b < NACC; ++b) {
             mbar_init(&accf[b], 1);
             mbar_init(&acce[b], EPI_WARPS);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&inff[b], 2);
+            mbar_init(&infe[b], EPI_WARPS);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -893,238 +936,251 @@ __global__ void __launch_bounds__(THREADS, 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     int *status = p.status;
+    const int n_mod = p.n_mod;
 
-    if (warp == 0) {
-        // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (long t = blockIdx.x; t < p.n_tasks && ok; t += gridDim.x) {
-                const int g = p.tasks[3 * t], ti = p.tasks[3 * t + 1], tj = p.tasks[3 * t + 2];
-                const long row0 = p.grp_row0[g];
-                const int nk = (int)(p.grp_kdim[g] / BKB);
-                for (int md = 0; md < NMOD && ok; ++md) {
-                    const int ya = (int)(md * p.nrows_total + row0 + (long)ti * BM);
-                    const int yb = (int)(md * p.nrows_total + row0 + (long)tj * BN);
-                    for (int kc = 0; kc < nk; ++kc, ++it) {
-                        const int s = it % STAGES;
-                        const uint32_t ph = (it / STAGES) & 1u;
-                        if (!mbar_wait(&empty[s], ph ^ 1u, status)) { ok = false; break; }
-                        unsigned char *sa = ring + (size_t)s * STAGE_BYTES;
-                        mbar_expect_tx(&full[s], STAGE_BYTES);
-                        tma_load(sa, &mapA, kc * BKB, ya, &full[s]);
-                        tma_load(sa + BM * BKB, &mapB, kc * BKB, yb, &full[s]);
+    if (warp < CTL_WARPS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CTL_REGS));
+        if (warp == 0) {
+            // -------------------------------------------------------- TMA producer
+            if (lane == 0) {
+                uint32_t it = 0;
+                bool ok = true;
+                for (long t = blockIdx.x; t < p.n_tasks && ok; t += gridDim.x) {
+                    const int g = p.tasks[3 * t], ti = p.tasks[3 * t + 1], tj = p.tasks[3 * t + 2];
+                    const long row0 = p.grp_row0[g];
+                    const int nk = (int)(p.grp_kdim[g] / BKB);
+                    for (int md = 0; md < n_mod && ok; ++md) {
+                        const int ya = (int)(md * p.nrows_total + row0 + (long)ti * BM);
+                        const int yb = (int)(md * p.nrows_total + row0 + (long)tj * BN);
+                        for (int kc = 0; kc < nk; ++kc, ++it) {
+                            const int s = it % STAGES;
+                            const uint32_t ph = (it / STAGES) & 1u;
+                            if (!mbar_wait(&empty[s], ph ^ 1u, status)) { ok = false; break; }
+                            unsigned char *sa = ring + (size_t)s * STAGE_BYTES;
+                            mbar_expect_tx(&full[s], STAGE_BYTES);
+                            tma_load(sa, &mapA, kc * BKB, ya, &full[s]);
+                            tma_load(sa + BM * BKB, &mapB, kc * BKB, yb, &full[s]);
+                        }
                     }
                 }
             }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            uint32_t it = 0, acc_it = 0;
-            bool ok = true;
-            for (long t = blockIdx.x; t < p.n_tasks && ok; t += gridDim.x) {
-                const int g = p.tasks[3 * t];
-                const int nk = (int)(p.grp_kdim[g] / BKB);
-                for (int md = 0; md < NMOD && ok; ++md, ++acc_it) {
-                    const int buf = acc_it & 1;
-                    const uint32_t aph = (acc_it >> 1) & 1u;
-                    if (!mbar_wait(&acce[buf], aph ^ 1u, status)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t dt = tmem + (uint32_t)(buf * BN);
-                    for (int kc = 0; kc < nk; ++kc, ++it) {
-                        const int s = it % STAGES;
-                        const uint32_t ph = (it / STAGES) & 1u;
-                        if (!mbar_wait(&full[s], ph, status)) { ok = false; break; }
+        } else if (warp == 1) {
+            // -------------------------------------------------------- MMA issuer
+            if (lane == 0) {
+                uint32_t it = 0, buf = 0, aph = 0;  // accumulator buffer and its phase
+                bool ok = true;
+                for (long t = blockIdx.x; t < p.n_tasks && ok; t += gridDim.x) {
+                    const int nk = (int)(p.grp_kdim[p.tasks[3 * t]] / BKB);
+                    for (int md = 0; md < n_mod && ok; ++md) {
+                        if (!mbar_wait(&acce[buf], aph ^ 1u, status)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t sa = smem_u32(ring + (size_t)s * STAGE_BYTES);
-                        const uint64_t ad = sw128_desc(sa), bd = sw128_desc(sa + BM * BKB);
+                        const uint32_t dt = tmem + buf * (uint32_t)BN;
+                        for (int kc = 0; kc < nk; ++kc, ++it) {
+                            const int s = it % STAGES;
+                            const uint32_t ph = (it / STAGES) & 1u;
+                            if (!mbar_wait(&full[s], ph, status)) { ok = false; break; }
+                            tc_fence_after();
+                            const uint32_t sa = smem_u32(ring + (size_t)s * STAGE_BYTES);
+                            const uint64_t ad = sw128_desc(sa), bd = sw128_desc(sa + BM * BKB);
 #pragma unroll
-                        for (int kk = 0; kk < BKB / 32; ++kk)
-                            mma_i8(dt, ad + (uint64_t)(2 * kk), bd + (uint64_t)(2 * kk), (kc | kk) != 0 ? 1u : 0u);
-                        mma_commit(&empty[s]);
+                            for (int kk = 0; kk < BKB / 32; ++kk)
+                                mma_i8(dt, ad + (uint64_t)(2 * kk), bd + (uint64_t)(2 * kk), (kc | kk) != 0 ? 1u : 0u);
+                            mma_commit(&empty[s]);
+                        }
+                        if (ok) mma_commit(&accf[buf]);
+                        if (++buf == NACC) { buf = 0; aph ^= 1u; }
                     }
-                    if (ok) mma_commit(&accf[buf]);
                 }
+            }
+        } else {
+            // -------------------------------------------------------- tile records: warp 2 rows, warp 3 columns
+            const bool rows = warp == 2;
+            uint32_t buf = 0, ph = 0;
+            for (long t = blockIdx.x; t < p.n_tasks; t += gridDim.x) {
+                const int g = p.tasks[3 * t], ti = p.tasks[3 * t + 1], tj = p.tasks[3 * t + 2];
+                const long row0 = p.grp_row0[g];
+                const int n = (int)p.grp_n[g];
+                if (!mbar_wait(&infe[buf], ph ^ 1u, status)) break;
+                TileInfo &I = info[buf];
+                double *rs = rows ? I.rs_row : I.rs_col, *mx = rows ? I.row_max[0] : I.col_max[0];
+                int i = (rows ? ti : tj) * BM + lane;
+#pragma unroll 1
+                for (int q = 0; q < 4; ++q, i += 32, mx += 3) {
+                    const bool in = i < n;
+                    rs[32 * q + lane] = in ? __ldg(p.rowscale + row0 + i) * (rows ? p.M : 1.0) : 0.0;
+#pragma unroll 1
+                    for (int v = 0; v < 3; ++v) {  // |g0| or |G00 g0|, |alpha sx|, |q/sx|
+                        const int f = v ? v + 1 : !rows;
+                        double m = in ? __ldg(p.cbound + (row0 + i) * CB_STRIDE + f) : 0.0;
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+                        if (lane == 0) mx[v] = m;
+                    }
+                }
+                if (rows && lane == 0) {
+                    I.out = p.out + p.grp_out[g];
+                    I.row0 = row0;
+                    I.n = n;
+                    I.ti = ti;
+                    I.tj = tj;
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&inff[buf]);
+                if ((buf ^= 1u) == 0u) ph ^= 1u;
             }
         }
     } else {
         // ------------------------------------------------------------ epilogue
-        const int ew = warp - 2;
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPI_REGS));
+        const int ew = warp - CTL_WARPS;
         const int quarter = warp & 3;       // TMEM lane quarter this warp may access
         const int cgrp = ew >> 2;           // column group of the tile
-        const int rloc = quarter * 32 + lane;
-        const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
-        const uint32_t col0 = (uint32_t)(cgrp * EPI_COLS);
+        const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cgrp * EPI_COLS);
         double *stg = stage_out + (size_t)ew * 32 * STG_LD;
-        uint32_t acc_it = 0;
-        bool ok = true;
-        for (long t = blockIdx.x; t < p.n_tasks && ok; t += gridDim.x) {
-            const int g = p.tasks[3 * t], ti = p.tasks[3 * t + 1], tj = p.tasks[3 * t + 2];
-            const long row0 = p.grp_row0[g], n = p.grp_n[g];
-            const long a = (long)ti * BM + rloc;  // table row of this thread
-            const long b0 = (long)tj * BN + col0;
-            uint32_t pk[EPI_COLS];
+        const int tiles = (int)((p.n_tasks - blockIdx.x + gridDim.x - 1) / gridDim.x);
+        const uint32_t park = tbase + (uint32_t)(NACC * BN);  // x / M mod 1: low words, high words BN columns on
+        double *row = stg + lane * STG_LD;
+        // One chunk of FC columns of a finished tile: scaling, correction and stores.
+        auto finish = [&](const TileInfo &I, int c) {
+            const int a0 = I.ti * BM + quarter * 32, bc = I.tj * BN + cgrp * EPI_COLS + c, a = a0 + lane;
+            const double rs_a = I.rs_row[quarter * 32 + lane];  // with M folded in
+            const double *rs_b = I.rs_col + cgrp * EPI_COLS + c;
+            tmem_wait_st();
 #pragma unroll
-            for (int c = 0; c < EPI_COLS; ++c) pk[c] = 0u;
-#pragma unroll 1
-            for (int md = 0; md < NMOD; ++md, ++acc_it) {
-                const int buf = acc_it & 1;
-                const uint32_t aph = (acc_it >> 1) & 1u;
-                if (!mbar_wait(&accf[buf], aph, status)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t m = (uint32_t)p.mod[md], magic = p.magic[md], bias = p.bias[md];
-                const int fsh = 16 * ((md >> 1) & 1);  // 16-bit field of this pair in the word
-                if ((md & 1) == 0) {
-                    // even modulus: park r_e in its pair field
+            for (int h = 0; h < FC; h += 4) {
+                int lo[4], hi[4];
+                tmem_ld4(park + (uint32_t)(c + h), lo);
+                tmem_ld4(park + (uint32_t)(BN + c + h), hi);
+                tmem_wait_ld();
 #pragma unroll
-                    for (int c = 0; c < EPI_COLS / 16; ++c) {
-                        uint32_t v[16];
-                        tmem_ld16(tmem + lane_off + (uint32_t)(buf * BN) + col0 + (uint32_t)(c * 16), v);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) pk[c * 16 + j] |= umod_small(v[j] + bias, m, magic) << fsh;
-                    }
-                } else {
-                    // odd modulus: merge with the parked r_e into a digit mod m_e m_o
-                    const uint32_t me = (uint32_t)p.mod[md - 1], inv = p.pinv[md >> 1];
-#pragma unroll
-                    for (int c = 0; c < EPI_COLS / 16; ++c) {
-                        uint32_t v[16];
-                        tmem_ld16(tmem + lane_off + (uint32_t)(buf * BN) + col0 + (uint32_t)(c * 16), v);
-                        tmem_wait_ld();
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const uint32_t ro = umod_small(v[j] + bias, m, magic);
-                            const uint32_t word = pk[c * 16 + j];
-                            const uint32_t re = (word >> fsh) & 0xffffu;
-                            const uint32_t t = umod_small((ro + 2u * m - re) * inv, m, magic);
-                            pk[c * 16 + j] = (word & ~(0xffffu << fsh)) | ((re + me * t) << fsh);
-                        }
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acce[buf]);
-                if ((md & 3) == 3 && (md >> 2) < PARKED) {
-                    // park a completed group of four moduli in TMEM columns 256 + 128*group
-                    const uint32_t col = 256u + 128u * (uint32_t)(md >> 2) + col0;
-#pragma unroll
-                    for (int c = 0; c < EPI_COLS / 16; ++c) tmem_st16(tmem + lane_off + col + (uint32_t)(c * 16), &pk[c * 16]);
-                    tmem_wait_st();
-#pragma unroll
-                    for (int c = 0; c < EPI_COLS; ++c) pk[c] = 0u;
-                }
+                for (int j = 0; j < 4; ++j)
+                    row[h + j] = __fma_rn(uint_to_double((uint32_t)lo[j]), 0x1p-32, int_to_double(hi[j])) *
+                                 (rs_a * rs_b[h + j]);
             }
-            if (!ok) break;
-            // ---- CRT, scaling, correction and stores
-            const bool arow = a < n;
-            const double rs_a = arow ? __ldg(p.rowscale + row0 + a) : 0.0;
-            const double *la = p.left + (row0 + (arow ? a : 0)) * p.cwp;
-            const bool mirror = ti != tj;
-            double *R = p.out + p.grp_out[g];
             // Correction screen for this warp's 32 x EPI_COLS block: with per-row bounds
             // relative to each row's scale, |left_a . right_b| <= 2^(e_a+e_b) *
             // (|g0_a| |G00 g0_b| + |alpha_a sx| |q_b/sx| + |q_a/sx| |alpha_b sx|).
             // Below corr_floor the term is far under the split's own error and is skipped.
-            double ra0 = 0.0, ra2 = 0.0, ra3 = 0.0, cb1 = 0.0, cb2 = 0.0, cb3 = 0.0;
-            if (arow) {
-                const double *cr = p.cbound + (row0 + a) * CB_STRIDE;
-                ra0 = __ldg(cr);
-                ra2 = __ldg(cr + 2);
-                ra3 = __ldg(cr + 3);
-            }
-#pragma unroll
-            for (int h = 0; h < EPI_COLS / 32; ++h) {
-                const long bcol = b0 + lane + 32 * h;
-                if (bcol < n) {
-                    const double *cc = p.cbound + (row0 + bcol) * CB_STRIDE;
-                    cb1 = fmax(cb1, __ldg(cc + 1));
-                    cb2 = fmax(cb2, __ldg(cc + 2));
-                    cb3 = fmax(cb3, __ldg(cc + 3));
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                ra0 = fmax(ra0, __shfl_xor_sync(0xffffffffu, ra0, o));
-                ra2 = fmax(ra2, __shfl_xor_sync(0xffffffffu, ra2, o));
-                ra3 = fmax(ra3, __shfl_xor_sync(0xffffffffu, ra3, o));
-                cb1 = fmax(cb1, __shfl_xor_sync(0xffffffffu, cb1, o));
-                cb2 = fmax(cb2, __shfl_xor_sync(0xffffffffu, cb2, o));
-                cb3 = fmax(cb3, __shfl_xor_sync(0xffffffffu, cb3, o));
-            }
-            const bool need_corr = !(ra0 * cb1 + ra2 * cb3 + ra3 * cb2 <= p.corr_floor);
-            constexpr int FC = 8;  // columns per final-phase chunk
-            // The final phase runs once per tile: a rolled loop keeps its code
-            // small enough to stay in the instruction cache beside the
-            // per-modulus code, so the register-resident last group is first
-            // copied to a (cached) local array that the loop can index.
-            uint32_t pk_l[EPI_COLS];
-#pragma unroll
-            for (int c = 0; c < EPI_COLS; ++c) pk_l[c] = pk[c];
+            const double *rm = I.row_max[quarter], *cm = I.col_max[cgrp];
+            const int n = I.n;
+            if (!(rm[0] * cm[0] + rm[1] * cm[2] + rm[2] * cm[1] <= p.corr_floor) && a < n) {
+                const double *la = p.left + (I.row0 + a) * p.cwp;
+                const double *rb = p.right + (I.row0 + bc) * p.cwp;
 #pragma unroll 1
-            for (int c = 0; c < EPI_COLS / FC; ++c) {
-                uint32_t w0[FC], w1[FC], w2[FC];
-                if (PARKED >= 1) tmem_ld8(tmem + lane_off + 256u + col0 + (uint32_t)(c * FC), w0);
-                if (PARKED >= 2) tmem_ld8(tmem + lane_off + 384u + col0 + (uint32_t)(c * FC), w1);
-#pragma unroll
-                for (int j = 0; j < FC; ++j) w2[j] = pk_l[c * FC + j];
-                tmem_wait_ld();
-                double xs[FC];
-#pragma unroll
-                for (int j = 0; j < FC; ++j) {
-                    double yh = 0.0, yl = 0.0;
-#pragma unroll
-                    for (int dg = 0; dg < NDIG; ++dg) {
-                        const int md = 2 * dg;              // first modulus of the digit
-                        const int grp = md >> 2;
-                        const uint32_t word = grp == LASTG ? w2[j] : (grp == 0 ? w0[j] : w1[j]);
-                        const uint32_t dv = (word >> (16 * ((md >> 1) & 1))) & 0xffffu;
-                        // exact int -> double: (2^52 + dv) - 2^52
-                        const double r = __hiloint2double(0x43300000, (int)dv) - 4503599627370496.0;
-                        yh = fma(r, p.f_hi[dg], yh);
-                        yl = fma(r, p.f_lo[dg], yl);
-                    }
-                    const long b = b0 + c * FC + j;
-                    const double rs_b = b < n ? __ldg(p.rowscale + row0 + b) : 0.0;
-                    xs[j] = ((yh - rint(yh)) * p.M + yl * p.M) * (rs_a * rs_b);
-                }
-                if (need_corr && arow) {  // warp-uniform except for the row guard
-                    for (int j = 0; j < FC; ++j) {
-                        const long b = b0 + c * FC + j;
-                        if (b < n) {
-                            const double *rb = p.right + (row0 + b) * p.cwp;
-                            double corr = 0.0;
-                            for (int i = 0; i < p.cw; ++i) corr = fma(__ldg(la + i), __ldg(rb + i), corr);
-                            xs[j] += corr;
-                        }
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < FC; ++j) {
-                    const long b = b0 + c * FC + j;
-                    const bool valid = arow && b < n;
-                    const double v = valid ? xs[j] : 0.0;
-                    if (valid) {
-                        if (!isfinite(v)) atomicExch(status, (int)RKB_ENONFINITE);
-                        if (mirror) R[b * n + a] = v;  // lanes hold consecutive a: coalesced
-                    }
-                    stg[lane * STG_LD + j] = v;
-                }
-                {
-                    // direct tile row segments of 8 columns through shared memory (coalesced rows)
-                    __syncwarp();
-                    const long a0 = (long)ti * BM + quarter * 32;
-                    const long bc = b0 + c * FC;
-#pragma unroll 4
-                    for (int rr = 0; rr < 32; rr += 4) {
-                        const int row = rr + (lane >> 3), col = lane & 7;
-                        const long aa = a0 + row, bb = bc + col;
-                        if (aa < n && bb < n) R[aa * n + bb] = stg[row * STG_LD + col];
-                    }
-                    __syncwarp();
+                for (int j = 0; j < min(FC, n - bc); ++j, rb += p.cwp) {
+                    double corr = 0.0;
+#pragma unroll 2
+                    for (int i = 0; i < p.cw; ++i) corr = fma(__ldg(la + i), __ldg(rb + i), corr);
+                    row[j] += corr;
                 }
             }
+            __syncwarp();
+            uint32_t top = 0u;  // largest exponent field of this thread's entries
+            const int sub = lane / FC, col = lane % FC;
+            const double *seg = stg + sub * STG_LD + col;
+            if (a0 + 32 <= n && bc + FC <= n) {
+                // the transposed tile: lanes hold consecutive a, 256 contiguous bytes a store;
+                // the tile itself: row segments of FC columns, 32 / FC rows a store
+                double *T = I.out + (long)bc * n + a, *R = I.out + (long)(a0 + sub) * n + bc + col;
+                const bool mirror = I.ti != I.tj;
+#pragma unroll
+                for (int j = 0; j < FC; ++j, T += n) {
+                    const double v = row[j];
+                    top = max(top, (uint32_t)__double2hiint(v) & 0x7ff00000u);
+                    if (mirror) *T = v;
+                }
+#pragma unroll
+                for (int rr = 0; rr < 32; rr += 32 / FC, R += (long)(32 / FC) * n) *R = seg[rr * STG_LD];
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < FC; ++j)
+                    if (a < n && bc + j < n) {
+                        const double v = row[j];
+                        top = max(top, (uint32_t)__double2hiint(v) & 0x7ff00000u);
+                        if (I.ti != I.tj) I.out[(long)(bc + j) * n + a] = v;
+                    }
+#pragma unroll 1
+                for (int rr = 0; rr < 32; rr += 32 / FC)
+                    if (a0 + rr + sub < n && bc + col < n)
+                        I.out[(long)(a0 + rr + sub) * n + bc + col] = seg[rr * STG_LD];
+            }
+            if (top == 0x7ff00000u) atomicExch(status, (int)RKB_ENONFINITE);
+            __syncwarp();
+        };
+        uint32_t it = 0;  // accumulators taken
+        bool ok = true;
+#pragma unroll 1
+        for (int k = 0; k < tiles; ++k) {
+            // The chunks of the tile before wait for the first digit of this one, in whose
+            // shadow (the MMAs run on) they are finished.
+            int late = k ? 0 : EPI_COLS;
+            if (k && !mbar_wait(&inff[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, status)) break;
+#pragma unroll 1
+            for (int dg = 0, md = 0; dg < NDIG; ++dg) {
+                long long acc[EPI_COLS];  // the open digit's sum
+#pragma unroll
+                for (int c = 0; c < EPI_COLS; ++c) acc[c] = 0;
+                const int end = p.dig_end[dg];
+#pragma unroll 1
+                for (; md < end; ++md, ++it) {
+                    if (!mbar_wait(&accf[it & 1u], (it >> 1) & 1u, status)) { ok = false; break; }
+                    tc_fence_after();
+                    const int coef = p.coef[md];
+                    const uint32_t src = tbase + (it & 1u) * (uint32_t)BN;
+#pragma unroll
+                    for (int c = 0; c < EPI_COLS; c += 8) {
+                        int v[8];
+                        tmem_ld8(src + (uint32_t)c, v);
+                        tmem_wait_ld();
+                        if (c + 8 == EPI_COLS) {  // the accumulator is read: the next modulus may overwrite it
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(&acce[it & 1u]);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc[c + j] += (long long)v[j] * coef;
+                    }
+                    if (late < EPI_COLS) {
+                        finish(info[(k - 1) & 1], late);
+                        late += FC;
+                    }
+                }
+                if (!ok) break;
+                if (dg == 0 && k) {
+#pragma unroll 1
+                    for (; late < EPI_COLS; late += FC) finish(info[(k - 1) & 1], late);
+                    if (lane == 0) mbar_arrive(&infe[(k - 1) & 1]);
+                }
+                // f += d F mod 1, rounded to 2^-64
+                const int D = p.D[dg], fh = p.f_hi[dg], fm = p.f_mid[dg], fl = p.f_lo[dg];
+                const double inv_D = p.inv_D[dg], inv_D32 = p.inv_D32[dg];
+                tmem_wait_st();
+#pragma unroll
+                for (int c = 0; c < EPI_COLS; c += 4) {
+                    int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+                    if (dg) {
+                        tmem_ld4(park + (uint32_t)c, lo);
+                        tmem_ld4(park + (uint32_t)(BN + c), hi);
+                        tmem_wait_ld();
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int d = mod_near(acc[c + j], D, inv_D, inv_D32);
+                        long long f = ((long long)hi[j] << 32) | (uint32_t)lo[j];
+                        f += (long long)d * fm + ((long long)((uint32_t)d * (uint32_t)fh) << 32) +
+                             (((long long)d * fl + 0x80000000LL) >> 32);
+                        lo[j] = (int)f;
+                        hi[j] = (int)(f >> 32);
+                    }
+                    tmem_st4(park + (uint32_t)c, lo);
+                    tmem_st4(park + (uint32_t)(BN + c), hi);
+                }
+            }
+            if (!ok) break;
+        }
+        if (ok && tiles > 0 && mbar_wait(&inff[(tiles - 1) & 1], (uint32_t)((tiles - 1) >> 1) & 1u, status)) {
+#pragma unroll 1
+            for (int c = 0; c < EPI_COLS; c += FC) finish(info[(tiles - 1) & 1], c);
         }
     }
     tc_fence_before();
@@ -1150,6 +1206,44 @@ static EncodeTiledFn encode_fn() {
             fn = (EncodeTiledFn)f;
     }
     return fn;
+}
+
+static int inverse_mod(int a, int m) {  // by trial (m <= 256); 0 when there is none
+    for (int x = 1; x < m; ++x)
+        if (a % m * x % m == 1 % m) return x;
+    return 0;
+}
+
+// The CRT constants of the contraction (CrtArgs).
+static void crt_weights(const int *moduli, int n_mod, CrtArgs &p) {
+    const __int128 one = (__int128)1 << 126;
+    for (int g = 0, i0 = 0; g < NDIG; ++g) {
+        const int i1 = i0 + (n_mod - i0 + NDIG - g - 1) / (NDIG - g);  // 4 to 12 moduli in three even parts
+        unsigned long long D = 1, c = 0;
+        for (int i = i0; i < i1; ++i) D *= moduli[i];
+        for (int i = i0; i < i1; ++i) {
+            // coef_i = (D/m_i) ((D/m_i)^-1 mod m_i), nearest zero: 1 mod m_i, 0 mod the digit's others
+            const int m = moduli[i];
+            const unsigned long long r = D / m, e = r * inverse_mod((int)(r % m), m) % D;
+            p.coef[i] = (int)(2 * e >= D ? (long long)e - (long long)D : (long long)e);
+            int rest = 1 % m;  // M/D mod m
+            for (int j = 0; j < n_mod; ++j)
+                if (j < i0 || j >= i1) rest = rest * (moduli[j] % m) % m;
+            c = (c + e * inverse_mod(rest, m)) % D;
+        }
+        // F = ((M/D)^-1 mod D) / D in [-1/2, 1/2)
+        const __int128 cs = 2 * c >= D ? (__int128)c - (__int128)D : (__int128)c, Ds = (__int128)D;
+        const __int128 f = one / Ds * cs + one % Ds * cs / Ds;
+        const __int128 w = (f + ((__int128)1 << 29)) >> 30;  // 96 bits; the two lower words are read as signed
+        p.f_lo[g] = (int)(uint32_t)w;
+        const uint64_t t = (uint64_t)(w >> 32) + ((uint32_t)w >> 31);
+        p.f_mid[g] = (int)(uint32_t)t;
+        p.f_hi[g] = (int)((uint32_t)(t >> 32) + ((uint32_t)t >> 31));
+        p.D[g] = (int)(uint32_t)D;
+        p.inv_D[g] = 1.0 / (double)D;
+        p.inv_D32[g] = 4294967296.0 / (double)D;
+        p.dig_end[g] = i0 = i1;
+    }
 }
 
 static int make_map(CUtensorMap *map, const void *ptr, long kpad, long rows) {
@@ -1378,34 +1472,14 @@ extern "C" int rkb_split_contract(const signed char *d_resA, const signed char *
     p.cwp = cwp; p.cw = cw;
     p.grp_row0 = d_grp_row0; p.grp_n = d_grp_n; p.grp_kdim = d_grp_kdim; p.grp_out = d_grp_out;
     p.tasks = d_tasks; p.n_tasks = n_tasks; p.nrows_total = nrows_total; p.out = d_out; p.status = d_status;
-    p.n_mod = n_mod; p.M = M;
-    const int ndig = (n_mod + 1) / 2;
-    for (int i = 0; i < MAXMOD; ++i) {
-        const int m = i < n_mod ? moduli[i] : 256;
-        RKB_CHECK_ARG(m >= 2 && m <= 256, "moduli must lie in [2, 256]");
-        p.mod[i] = m;
-        p.magic[i] = (uint32_t)((1ULL << 32) / (unsigned long long)m + 1ULL);
-        p.bias[i] = (uint32_t)m << 18;
-        p.f_hi[i] = i < ndig ? f_hi[i] : 0.0;
-        p.f_lo[i] = i < ndig ? f_lo[i] : 0.0;
-    }
-    for (int i = 0; i < MAXMOD / 2; ++i) p.pinv[i] = i < n_mod / 2 ? (uint32_t)pair_inv[i] : 1u;
+    p.n_mod = n_mod; p.M = M * 0x1p-32;
+    for (int i = 0; i < n_mod; ++i) RKB_CHECK_ARG(moduli[i] >= 2 && moduli[i] <= 256, "moduli must lie in [2, 256]");
+    crt_weights(moduli, n_mod, p);
     long grid = n_tasks < sm_count() ? n_tasks : sm_count();
     cudaStream_t st = as_stream(stream);
-#define RKB_CRT_CASE(NM)                                                                                     \
-    case NM: {                                                                                               \
-        RKB_CUDA(set_smem(crt_syrk_kernel<NM>, (int)SMEM_BYTES));                                            \
-        crt_syrk_kernel<NM><<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(mA, mB, p);                         \
-        break;                                                                                               \
-    }
-    switch (n_mod) {
-        RKB_CRT_CASE(4) RKB_CRT_CASE(5) RKB_CRT_CASE(6) RKB_CRT_CASE(7) RKB_CRT_CASE(8) RKB_CRT_CASE(9)
-        RKB_CRT_CASE(10) RKB_CRT_CASE(11) RKB_CRT_CASE(12)
-        default:
-            set_error("split contraction compiled for 4..12 moduli (got %d)", n_mod);
-            return RKB_EINVAL;
-    }
-#undef RKB_CRT_CASE
+    RKB_CHECK_ARG(n_mod >= 4, "split contraction takes 4..%d moduli (got %d)", MAXMOD, n_mod);
+    RKB_CUDA(set_smem(crt_syrk_kernel, (int)SMEM_BYTES));
+    crt_syrk_kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(mA, mB, p);
     RKB_LAUNCHED("crt_syrk_kernel");
     return RKB_OK;
 }

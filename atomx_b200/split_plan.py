@@ -51,8 +51,10 @@ FP64.
 CRT constants
 -------------
 Pairwise-coprime moduli m_i <= 256 (int8 residues in [-128, 127]), M = prod m_i.
-The device reduces each int32 accumulator to r_i in [0, m_i) and merges the
-residues of consecutive moduli into one digit d_p = r_2p + m_2p t,
+The contraction kernel derives its weights from the moduli and M alone
+(``crt_weights`` in csrc/rkb_split.cu).  ``crt_constants`` also gives the
+constants of an equivalent recombination in doubles, used on the CPU: residues
+r_i in [0, m_i) of consecutive moduli merge into one digit d_p = r_2p + m_2p t,
 t = (r_2p+1 - r_2p) m_2p^-1 mod m_2p+1, a residue mod D_p = m_2p m_2p+1
 (< 2^16); an odd last modulus stays a digit of its own.  An integer x with
 |x| < M/2 is rebuilt from the digits as x = M * frac(sum_p d_p f_p),

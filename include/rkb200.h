@@ -232,9 +232,9 @@ int rkb_exchange_matrix(const double *d_fb, const double *d_bsp, const double *d
  * rkb_split_contract: for every task (group, tile_i, tile_j >= tile_i) the
  * 128 x 128 tile of R_g is computed as n_mod residue GEMMs of length
  * d_grp_kdim[g] (multiple of 128, <= 3456) on the tensor cores, CRT-recombined
- * in FP64 from digits merged over consecutive moduli pairs with the HOST
- * constants pair_inv (m_2p^-1 mod m_2p+1) and per-digit f_hi/f_lo/M (see
- * atomx_b200/split_plan.py), scaled and corrected, and written (and
+ * to 64 bits of x / M (M, the product of the moduli, as a double; the CRT
+ * weights follow from the moduli, and pair_inv, f_hi and f_lo are not read),
+ * scaled and corrected, and written (and
  * mirrored) into the n x n block at d_out + d_grp_out[g], as
  * rkb_table_contract_fp64 does.  The FP64 core correction of a 32 x 64 block
  * is skipped when its bound from d_cbound (relative to 2^(e_a + e_b), which
