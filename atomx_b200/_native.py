@@ -44,6 +44,8 @@ _SIGNATURES = {
                              _l, _l, _vp, _vp, _vp, _vp, _i, _vp],
     "rkb_split_rows_cells": [_vp, _vp, _l, _vp, _vp, _vp, _l, _vp, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp,
                              _vp, _l, _l, _l, _vp, _vp, _vp, _vp, _i, _vp],
+    "rkb_split_rows_cells_z": [_vp, _vp, _l, _vp, _vp, _vp, _l, _vp, _i, _i, _vp, _vp, _vp, _vp, _i, _i, _i, _vp, _vp,
+                               _vp, _l, _l, _l, _l, _l, _vp, _vp, _vp, _vp, _i, _vp],
     "rkb_split_fused_body_width": [_i, _i],
     "rkb_green_factor": [_vp, _i, _i, _i, _d, _vp, _vp, _vp, _l],
     "rkb_green_tables": [_vp, _i, _i, _vp, _i, _d, _vp, _vp, _i, _i, _vp, _l, _vp, _vp, _l, _vp, _vp],
@@ -67,6 +69,8 @@ _SIGNATURES = {
     "rkb_cell_fock_finish": [_vp, _vp, _i, _i, _l, _vp, _vp],
     "rkb_split_contract": [_vp, _vp, _l, _l, _i, _vp, _vp, _vp, _vp, _d, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _vp,
                            _vp, _vp, _vp, _l, _vp, _vp, _vp],
+    "rkb_split_contract_z": [_vp, _vp, _l, _l, _l, _i, _vp, _d, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _vp, _vp, _vp,
+                             _vp, _vp, _l, _vp, _vp, _vp],
 }
 _RESTYPE = {"rkb_last_error": _c.c_char_p, "rkb_version": _c.c_char_p, "rkb_split_fused_body_width": _c.c_long,
             "rkb_green_factor": _c.c_long, "rkb_green_tables": _c.c_long, "rkb_table_plan": _c.c_long, "rkb_gauss_legendre_01": None}

@@ -179,9 +179,14 @@ class SplitBatch(_Graphable):
         nrows = int(self.row_base[-1])
         self.rows_alloc = _round_up(max(nrows, 1), TILE)
         ws = workspace
-        res_shape = (self.n_mod, self.rows_alloc, self.kpad)
-        self.resA = _alloc(ws, res_shape, torch.int8, d)
-        self.resB = _alloc(ws, res_shape, torch.int8, d) if any(r.has_z for r in self.ions) else None
+        # With every ion on the cell kernel, B holds only the columns from each
+        # ion's first Z chunk on (IonRows.b_col0); else it is written whole.
+        cells = all(r.kind == "cells" for r in self.ions)
+        self.b_col0 = [r.b_col0 if cells else 0 for r in self.ions]
+        self.b_ld = max(r.kmax_dim - c for r, c in zip(self.ions, self.b_col0)) if cells else self.kpad
+        self.resA = _alloc(ws, (self.n_mod, self.rows_alloc, self.kpad), torch.int8, d)
+        self.resB = (_alloc(ws, (self.n_mod, self.rows_alloc, self.b_ld), torch.int8, d)
+                     if any(r.has_z for r in self.ions) and self.b_ld > 0 else None)
         # The cell and two-kernel row paths write every column of their rows;
         # the fused kernel only its own.  Padding rows are read by the last
         # tiles (their entries are never stored) and are zeroed all the same.
@@ -200,12 +205,13 @@ class SplitBatch(_Graphable):
         self.xwork = _alloc(ws, (max(two), self.kpad), torch.float64, d) if two else None
         self.corr_floor = 2.0 ** -(self.bits + 10) if corr_floor is None else float(corr_floor)
         # groups: (ion, k)
-        g_row0, g_n, g_kdim, self.group_of = [], [], [], []
+        g_row0, g_n, g_kdim, g_zc, self.group_of = [], [], [], [], []
         for i, (dv, r) in enumerate(zip(self.devs, self.ions)):
             for k in dv.plan.ks:
                 g_row0.append(int(self.row_base[i]) + dv.plan.k_row_offset[k])
                 g_n.append(dv.plan.n_of_k(k))
                 g_kdim.append(r.kdim[k])
+                g_zc.append(self.b_col0[i] // TILE)
                 self.group_of.append((i, k))
         offs = np.concatenate([[0], np.cumsum(np.asarray(g_n, dtype=np.int64) ** 2)])
         self.offsets = {gk: int(offs[j]) for j, gk in enumerate(self.group_of)}
@@ -214,12 +220,15 @@ class SplitBatch(_Graphable):
         self.n_tasks = int(tasks.shape[0])
         # the group records and the task list in one host-to-device copy
         ng_ = len(g_n)
-        host = np.empty(4 * ng_ + (tasks.size + 1) // 2, dtype=np.int64)
+        host = np.empty(4 * ng_ + (tasks.size + ng_ + 1) // 2, dtype=np.int64)
         host[:4 * ng_] = np.concatenate([g_row0, g_n, g_kdim, offs[:-1]]).astype(np.int64)
-        host[4 * ng_:].view(np.int32)[:tasks.size] = tasks.reshape(-1)
+        words = host[4 * ng_:].view(np.int32)
+        words[:tasks.size] = tasks.reshape(-1)
+        words[tasks.size:tasks.size + ng_] = g_zc
         arr = torch.from_numpy(host).to(d)
         self.grp_row0, self.grp_n, self.grp_kdim, self.grp_out = (arr[i * ng_:(i + 1) * ng_] for i in range(4))
-        self.tasks = arr[4 * ng_:].view(torch.int32)[:tasks.size]
+        words_d = arr[4 * ng_:].view(torch.int32)
+        self.tasks, self.grp_zc = words_d[:tasks.size], words_d[tasks.size:tasks.size + ng_]
         #: [contraction status, number of tables whose certificate failed]
         self.status = torch.zeros(2, dtype=torch.int32, device=d)
         self.est = torch.zeros(len(g_n), dtype=torch.float64, device=d)
@@ -228,10 +237,7 @@ class SplitBatch(_Graphable):
         self.escalated: list = []
         self._stream = None
         self.out = _alloc(ws, (self.total,), torch.float64, d)
-        self._c = (np.ctypeslib.as_ctypes(np.ascontiguousarray(self.moduli, dtype=np.int32)),
-                   np.ctypeslib.as_ctypes(np.ascontiguousarray(self.f_hi)),
-                   np.ctypeslib.as_ctypes(np.ascontiguousarray(self.f_lo)),
-                   np.ctypeslib.as_ctypes(np.ascontiguousarray(np.concatenate([self.pair_inv, [1]]).astype(np.int32))))
+        self._c = np.ctypeslib.as_ctypes(np.ascontiguousarray(self.moduli, dtype=np.int32))
 
     @property
     def launches_per_step(self) -> int:
@@ -271,8 +277,9 @@ class SplitBatch(_Graphable):
                 if ls not in used:
                     ls.wait_event(fork)
                     used.add(ls)
-            r.launch(self.ion_bits[i], self.n_mod, self._c[0], self.resA, self.resB, self.kpad, int(self.row_base[i]),
-                     self.rows_alloc, self.rowscale, self.left, self.right, self.cbound, self.cwp, self.xwork, ls)
+            r.launch(self.ion_bits[i], self.n_mod, self._c, self.resA, self.resB, self.kpad, int(self.row_base[i]),
+                     self.rows_alloc, self.rowscale, self.left, self.right, self.cbound, self.cwp, self.xwork, ls,
+                     self.b_col0[i], self.b_ld)
         for ls in used:
             join = torch.cuda.Event()
             join.record(ls)
@@ -281,15 +288,16 @@ class SplitBatch(_Graphable):
 
     def contract(self, stream=None) -> None:
         L = _native.load()
-        _native.check(L.rkb_split_contract(self.resA.data_ptr(), _native.ptr(self.resB), self.kpad, self.rows_alloc,
-                                           self.n_mod, self._c[0], self._c[3], self._c[1], self._c[2], self.M,
-                                           self.rowscale.data_ptr(), self.left.data_ptr(), self.right.data_ptr(),
-                                           self.cbound.data_ptr(), self.corr_floor, self.cw, self.cwp,
-                                           self.grp_row0.data_ptr(), self.grp_n.data_ptr(),
-                                           self.grp_kdim.data_ptr(), self.grp_out.data_ptr(), self.tasks.data_ptr(),
-                                           self.n_tasks, self.out.data_ptr(), self.status.data_ptr(),
-                                           _native.stream_handle(stream)),
-                      "rkb_split_contract")
+        _native.check(L.rkb_split_contract_z(self.resA.data_ptr(), _native.ptr(self.resB), self.kpad, self.b_ld,
+                                             self.rows_alloc, self.n_mod, self._c, self.M,
+                                             self.rowscale.data_ptr(), self.left.data_ptr(), self.right.data_ptr(),
+                                             self.cbound.data_ptr(), self.corr_floor, self.cw, self.cwp,
+                                             self.grp_row0.data_ptr(), self.grp_n.data_ptr(),
+                                             self.grp_kdim.data_ptr(), self.grp_zc.data_ptr(),
+                                             self.grp_out.data_ptr(), self.tasks.data_ptr(), self.n_tasks,
+                                             self.out.data_ptr(), self.status.data_ptr(),
+                                             _native.stream_handle(stream)),
+                      "rkb_split_contract_z")
 
     def step(self, stream=None, side_streams=None) -> None:
         """Enqueue every row launch and the one contraction (no host sync)."""

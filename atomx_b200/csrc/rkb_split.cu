@@ -93,6 +93,8 @@ struct RowsArgs {
     double inv_mod[MAXMOD];    // RN(1/m)
     signed char *resA, *resB;  // [n_mod][nrows_total][kpad]; resB may be null
     long kpad, row_base, nrows_total;
+    long b_ld;   // row stride and width of resB
+    int b_col0;  // first column that resB holds (cell kernel; a multiple of 128)
     double *rowscale, *left, *right, *cbound;
     double *xwork;  // scratch rows [X | Z | 0] (row stride kpad)
     int cwp;
@@ -525,219 +527,330 @@ __global__ void __launch_bounds__(128) split_rows_fused_kernel(RowsArgs a) {
 
 
 // ---------------------------------------------------------------------------
-// Cell-parallel row kernel: one block per row, one thread per cell.  Thread t
+// Cell-parallel row kernel: one block per R rows, one thread per cell.  Thread t
 // owns cell m = nv-1-t (cells last to first), so a forward exclusive block
 // scan of the cell dots u_m.g_m gives each cell its suffix sum t_m directly.
-// The block first forms g = w*rho for the whole row with coalesced loads
-// (consecutive threads, consecutive nodes) into a padded shared-memory image;
-// each thread then reads its cell's g and the cell-minor factor copy
-// (entry i of every cell contiguous, so a warp's reads are consecutive) and
-// forms X = L_m^T g_m + C_m t_m in registers, without shuffles.
-// Threads past the cells compute the Z columns.  After a block maximum fixes
-// the row's power-of-two scale, every thread writes its int8 residues into
-// per-modulus row images in shared memory, and the block copies them out with
-// 16-byte stores.  Columns are in natural order: (m-1)*ng + node, then Z.
+// The block first forms g = w*rho of its rows with coalesced loads into a
+// padded shared-memory image; each thread then reads its cell's g and the
+// cell-minor factor copy (entry i of every cell contiguous, so a warp's reads
+// are consecutive), once for all R rows, and forms X = L_m^T g_m + C_m t_m in
+// registers, in place of g.  Threads past the cells compute the Z columns.  X
+// and Z go back to the image in column order, and once a block maximum has
+// fixed each row's power-of-two scale, the residues are written: a thread takes
+// four consecutive columns, so that a warp stores 128 contiguous bytes per
+// modulus and the work is even whatever the number of cells.  Columns are in
+// natural order: (m-1)*ng + node, then Z.
+//
+// Bound by instruction issue.  A residue costs six FP32 operations (an integer
+// of 41 bits as three exact limbs; FP32 issues at twice the rate of FP64 and
+// integer multiplies), and the factor tables, R rows per read, stay off L2.  One
+// row per block with FP64 residues, byte stores to shared images and a copy
+// out took 0.856 ms for the Z=70 rows (56 209 x 896) and 2.06 ms for N = 2112
+// (44 900 rows); this form takes 0.732 and 1.25 ms.  R = 1, 2, 4 took 0.753, 0.759,
+// 0.732 ms for the first and 1.37, 1.25, 1.35 ms for the second: four rows fit the
+// registers up to eight nodes a cell, two beyond.
 //
 // Cell-minor factor table of one multipole (doubles), nv cells:
 //   u[NG][nv] | C[NG][nv] | L[NG][NG][nv] (L[i][node][m])
 constexpr int CELL_ZMAX = 128;  // Z columns per row of the cell kernel (one thread each, nv + Z <= 256)
+__host__ __device__ constexpr int cell_rows(int ng) { return ng <= 8 ? 4 : 2; }  // R: R x ng doubles a thread
+// doubles from one cell to the next in the image: odd, so that cell-strided reads do not conflict
+__host__ __device__ constexpr int cell_stride(int ng) { return ng | 1; }
+__host__ __device__ constexpr long cell_image(int ng, long nv, long z) {  // doubles of one row's image
+    return (nv + (z + ng - 1) / ng) * cell_stride(ng);
+}
 
-template <int NG>
-__global__ void __launch_bounds__(256) split_rows_cell_kernel(RowsArgs a, const double *__restrict__ ktab_t,
-                                                              const long *__restrict__ koff_t) {
-    constexpr int GS = NG | 1;  // padded cell stride of the g image (odd: 2-way bank conflicts at most)
-    extern __shared__ __align__(16) unsigned char smc[];
+struct ResidueArgs {
+    float4 mod[MAXMOD];  // m, 1/m, 2^14 mod m and 2^28 mod m (nearest zero)
+};
+
+template <int NG, int R>
+__device__ __forceinline__ void cell_rows_body(const RowsArgs &a, const ResidueArgs &f,
+                                               const double *__restrict__ ktab_t, const long *__restrict__ koff_t,
+                                               long q, long zmax, double *img, double *red) {
+    constexpr int GS = cell_stride(NG);
     const int nv = a.nv;
-    const long q = blockIdx.x;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nwarp = blockDim.x >> 5;
-    const long kpad = a.kpad;
-    const size_t ndbl = ((size_t)nv * GS + 64 + 1) & ~(size_t)1;     // doubles before the images (even: 16-B aligned)
-    double *gimg = reinterpret_cast<double *>(smc);                  // [nv][GS]
-    double *red = gimg + (size_t)nv * GS;                              // [64] block scratch
-    unsigned char *lines = smc + ndbl * sizeof(double);               // [n_mod][kpad]
-    unsigned char *zneg = lines + (size_t)a.n_mod * kpad;             // [n_mod][CELL_ZMAX]: B's Z bytes
+    const long ld = cell_image(NG, nv, zmax);
     const int k = a.row_k[q];
-    const long pr = a.row_pair[q];
-    const double *Pa = a.P + a.pairs[2 * pr] * a.orb_ld, *Pc = a.P + a.pairs[2 * pr + 1] * a.orb_ld;
-    const double *Qa = a.Q + a.pairs[2 * pr] * a.orb_ld, *Qc = a.Q + a.pairs[2 * pr + 1] * a.orb_ld;
     const long n = (long)nv * NG;
     const double *tab = a.ktab + a.koff[k];
     const double *v0 = tab + n + (long)nv * NG * NG + (long)nv * NG;
     const double *G00 = v0 + NG;
     const double sx = G00[NG * NG];
-    const int nz = (int)G00[NG * NG + 1];
+    const int nz = min((int)G00[NG * NG + 1], (int)zmax);
     const double *zt = G00 + NG * NG + 2;
     const double *tt = ktab_t + koff_t[k];
     const double *ut = tt, *Ct = tt + n, *Lt = tt + 2 * n;
-    const long kbody = (long)(nv - 1) * NG;
+    const int kbody = (nv - 1) * NG, zend = kbody + nz;
     const long grow = a.row_base + q;
-    // g = w * (P_a P_c + Q_a Q_c) for the whole row, coalesced
-    for (long j = tid; j < n; j += blockDim.x) {
-        const long cell = j / NG, node = j - cell * NG;
-        gimg[cell * GS + node] =
-            __dmul_rn(a.w[j], __dadd_rn(__dmul_rn(Pa[j], Pc[j]), __dmul_rn(Qa[j], Qc[j])));
+    // g = w * (P_a P_c + Q_a Q_c) of the rows, coalesced
+    {
+        const double *Pa[R], *Pc[R], *Qa[R], *Qc[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const long pr = a.row_pair[q + r];
+            const long x = a.pairs[2 * pr] * a.orb_ld, c = a.pairs[2 * pr + 1] * a.orb_ld;
+            Pa[r] = a.P + x;
+            Qa[r] = a.Q + x;
+            Pc[r] = a.P + c;
+            Qc[r] = a.Q + c;
+        }
+        for (int j = tid; j < (int)n; j += blockDim.x) {
+            const int cell = j / NG, at = cell * GS + (j - cell * NG);
+            const double w = __ldg(a.w + j);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                img[r * ld + at] = __dmul_rn(w, __dadd_rn(__dmul_rn(__ldg(Pa[r] + j), __ldg(Pc[r] + j)),
+                                                          __dmul_rn(__ldg(Qa[r] + j), __ldg(Qc[r] + j))));
+        }
     }
     __syncthreads();
     const int m = nv - 1 - tid;  // this thread's cell (m < 0: a Z column or idle)
-    double g[NG], x[NG];
-    double d = 0.0;
+    double g[R][NG], d[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) d[r] = 0.0;
     if (m >= 0) {
 #pragma unroll
-        for (int i = 0; i < NG; ++i) g[i] = gimg[(long)m * GS + i];
-        if (m >= 1) {
-#pragma unroll
-            for (int i = 0; i < NG; ++i) d = fma(ut[(long)i * nv + m], g[i], d);
-        }
-    }
-    // cell 0: alpha = v_0 . g_0, G_00 g_0 and their norms (one thread)
-    double n1 = 0.0, n2 = 0.0, gg = 0.0, alpha = 0.0;
-    if (m == 0) {
-#pragma unroll
-        for (int i = 0; i < NG; ++i) alpha = fma(v0[i], g[i], alpha);
-#pragma unroll
         for (int i = 0; i < NG; ++i) {
-            double sacc = 0.0;
+            const double u = m >= 1 ? __ldg(ut + (long)i * nv + m) : 0.0;
 #pragma unroll
-            for (int j = 0; j < NG; ++j) sacc = fma(G00[i * NG + j], g[j], sacc);
-            a.left[grow * a.cwp + i] = g[i];
-            a.right[grow * a.cwp + i] = sacc;
-            n1 = fma(g[i], g[i], n1);
-            n2 = fma(sacc, sacc, n2);
-            gg = fma(g[i], sacc, gg);
+            for (int r = 0; r < R; ++r) {
+                g[r][i] = img[r * ld + m * GS + i];
+                d[r] = fma(u, g[r][i], d[r]);
+            }
         }
-        for (int i = NG + 2; i < a.cwp; ++i) a.left[grow * a.cwp + i] = a.right[grow * a.cwp + i] = 0.0;
-    }
-    // exclusive scan of d over threads (= suffix sums over cells)
-    const double incl = warp_inclusive_scan(d, lane);
-    if (lane == 31) red[wid] = incl;
-    __syncthreads();
-    double before = 0.0;
-    for (int w = 0; w < wid; ++w) before += red[w];
-    const double up = __shfl_up_sync(0xffffffffu, incl, 1);
-    const double t_m = lane == 0 ? before : before + up;
-    double amax = 0.0, xsq = 0.0, zsq = 0.0;
-    bool bad = false;
-    if (m >= 1) {
-#pragma unroll
-        for (int node = 0; node < NG; ++node) {
-            double xv = Ct[(long)node * nv + m] * t_m;
-#pragma unroll
-            for (int i = node; i < NG; ++i) xv = fma(Lt[((long)i * NG + node) * nv + m], g[i], xv);
-            x[node] = xv;
-            amax = fmax(amax, fabs(xv));
-            xsq = fma(xv, xv, xsq);
-            bad |= !isfinite(xv);
-        }
-    }
-    // cell 0: the core-body coupling columns (t_0 = q = u_b . g_b)
-    double a_sx = 0.0, q_sx = 0.0;
-    if (m == 0) {
-        a_sx = alpha * sx;
-        q_sx = t_m / sx;
-        bad |= !isfinite(a_sx) || !isfinite(q_sx);
-        a.left[grow * a.cwp + NG] = a_sx;
-        a.left[grow * a.cwp + NG + 1] = q_sx;
-        a.right[grow * a.cwp + NG] = q_sx;
-        a.right[grow * a.cwp + NG + 1] = a_sx;
     }
     // Z columns: thread nv + e
     const int e = tid - nv;
-    double zx = 0.0;
+    double zx[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) zx[r] = 0.0;
     if (e >= 0 && e < nz) {
         const double *ze = zt + (long)e * (NG + 1);
-        const long cz = (long)ze[0];
+        const int cz = (int)ze[0] * GS;
 #pragma unroll
-        for (int i = 0; i < NG; ++i) zx = fma(ze[1 + i], gimg[cz * GS + i], zx);
-        amax = fmax(amax, fabs(zx));
-        zsq = zx * zx;
-        bad |= !isfinite(zx);
-    }
-    // block maximum, sums of squares and non-finite flag (red[]: 8 warps at most)
+        for (int i = 0; i < NG; ++i) {
+            const double z = ze[1 + i];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    xsq = warp_sum(xsq);
-    zsq = warp_sum(zsq);
-    const int badw = __any_sync(0xffffffffu, bad);
-    __syncthreads();  // red[] reused
-    if (lane == 0) {
-        red[wid] = amax;
-        red[8 + wid] = xsq;
-        red[16 + wid] = zsq;
-        red[32 + wid] = badw ? 1.0 : 0.0;
+            for (int r = 0; r < R; ++r) zx[r] = fma(z, img[r * ld + cz + i], zx[r]);
+        }
     }
-    __syncthreads();
-    amax = 0.0;
-    xsq = 0.0;
-    zsq = 0.0;
-    bool anybad = false;
-    for (int w = 0; w < nwarp; ++w) {
-        amax = fmax(amax, red[w]);
-        xsq += red[8 + w];
-        zsq += red[16 + w];
-        anybad |= red[32 + w] != 0.0;
+    // the core cell: lane (r, i) of the block's last warp forms G_00 g_0 (row i)
+    double *core = red + 8 * 4 * R;  // [R][2 * NG]: g_0, G_00 g_0
+    for (int o = wid == nwarp - 1 ? lane : R * NG; o < R * NG; o += 32) {
+        const int r = o / NG, i = o - r * NG;
+        const double *g0 = img + r * ld;
+        double sacc = 0.0;
+#pragma unroll
+        for (int j = 0; j < NG; ++j) sacc = fma(__ldg(G00 + i * NG + j), g0[j], sacc);
+        a.left[(grow + r) * a.cwp + i] = g0[i];
+        a.right[(grow + r) * a.cwp + i] = sacc;
+        core[r * 2 * NG + i] = g0[i];
+        core[r * 2 * NG + NG + i] = sacc;
     }
-    int ex = 0;
-    double scale = 0.0, inv_scale = 0.0;
-    if (!anybad && amax > 0.0) {
-        frexp(amax, &ex);  // amax < 2^ex
-        scale = ldexp(1.0, a.bits - ex);
-        inv_scale = ldexp(1.0, ex - a.bits);
+    // exclusive scan of d over threads (= suffix sums over cells)
+    double t_m[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const double incl = warp_inclusive_scan(d[r], lane);
+        if (lane == 31) red[wid * R + r] = incl;
+        t_m[r] = __shfl_up_sync(0xffffffffu, incl, 1);
+        if (lane == 0) t_m[r] = 0.0;
     }
-    if (m == 0) {
-        a.rowscale[grow] = anybad ? __longlong_as_double(0x7ff8000000000000LL) : inv_scale;
-        write_row_record(a.cbound + grow * CB_STRIDE, amax, ex, n1, n2, a_sx, q_sx, xsq, zsq, gg);
+    __syncthreads();  // from here on nothing reads g from the image
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        double before = 0.0;
+        for (int w = 0; w < wid; ++w) before += red[w * R + r];
+        t_m[r] = lane == 0 ? before : before + t_m[r];
     }
-    // residues into the row images (natural column order), zero tails
-    const double rc = 6755399441055744.0;  // 1.5 * 2^52
-    const long zend = kbody + nz;
-    for (long c = zend + tid; c < kpad; c += blockDim.x)
-        for (int md = 0; md < a.n_mod; ++md) lines[(size_t)md * kpad + c] = 0;
+    uint32_t top[R];  // largest exponent field
+    double xsq[R], zsq[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        top[r] = 0u;
+        xsq[r] = zsq[r] = 0.0;
+    }
     if (m >= 1) {
 #pragma unroll
-        for (int node = 0; node < NG; ++node) x[node] = __dadd_rn(__fma_rn(x[node], scale, rc), -rc);
-        for (int md = 0; md < a.n_mod; ++md) {
-            const double mm = (double)a.mod[md], im = a.inv_mod[md];
-            unsigned char *ln = lines + (size_t)md * kpad + (long)(m - 1) * NG;
+        for (int node = 0; node < NG; ++node) {
+            const double C = __ldg(Ct + (long)node * nv + m);
+            double xv[R];
 #pragma unroll
-            for (int node = 0; node < NG; ++node) ln[node] = (unsigned char)residue_f64(x[node], mm, im);
+            for (int r = 0; r < R; ++r) xv[r] = C * t_m[r];
+#pragma unroll
+            for (int i = node; i < NG; ++i) {
+                const double L = __ldg(Lt + ((long)i * NG + node) * nv + m);
+#pragma unroll
+                for (int r = 0; r < R; ++r) xv[r] = fma(L, g[r][i], xv[r]);
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                img[r * ld + m * GS + node] = xv[r];
+                top[r] = max(top[r], (uint32_t)__double2hiint(xv[r]) & 0x7ff00000u);
+                xsq[r] = fma(xv[r], xv[r], xsq[r]);
+            }
         }
     }
     if (e >= 0 && e < nz) {
-        zx = __dadd_rn(__fma_rn(zx, scale, rc), -rc);
-        for (int md = 0; md < a.n_mod; ++md) {
-            const uint32_t r = residue_f64(zx, (double)a.mod[md], a.inv_mod[md]);
-            lines[(size_t)md * kpad + kbody + e] = (unsigned char)r;
-            int nr = -(int)(int8_t)(uint8_t)r;  // residue of -x, centred again
-            nr -= nr > 127 ? a.mod[md] : 0;
-            zneg[md * CELL_ZMAX + e] = (unsigned char)nr;
+        const int cell = nv + e / NG, at = cell * GS + e % NG;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            img[r * ld + at] = zx[r];
+            top[r] = max(top[r], (uint32_t)__double2hiint(zx[r]) & 0x7ff00000u);
+            zsq[r] = zx[r] * zx[r];
+        }
+    }
+    // the coupling moments (cell 0's thread: t_0 = q = u_b . g_b)
+    double *mom = core + 2 * NG * R;  // [R][2]: alpha sx, q / sx
+    if (m == 0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            double alpha = 0.0;
+#pragma unroll
+            for (int i = 0; i < NG; ++i) alpha = fma(__ldg(v0 + i), g[r][i], alpha);
+            const double a_sx = alpha * sx, q_sx = t_m[r] / sx;
+            if (!isfinite(a_sx) || !isfinite(q_sx)) top[r] = 0x7ff00000u;
+            mom[2 * r] = a_sx;
+            mom[2 * r + 1] = q_sx;
+        }
+    }
+    // block maximum and sums of squares (8 warps at most)
+    __syncthreads();  // red[] reused
+    double *rsum = red;
+    uint32_t *rtop = reinterpret_cast<uint32_t *>(red + 8 * 2 * R);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint32_t t = __reduce_max_sync(0xffffffffu, top[r]);
+        const double xs = warp_sum(xsq[r]), zs = warp_sum(zsq[r]);
+        if (lane == 0) {
+            rsum[(wid * R + r) * 2] = xs;
+            rsum[(wid * R + r) * 2 + 1] = zs;
+            rtop[wid * R + r] = t;
         }
     }
     __syncthreads();
-    // copy the row images out: 16-byte chunks; B's chunks that hold Z columns
-    // take their bytes from the negated copy
-    const long chunks = kpad / 16;
-    const long zc0 = kbody / 16, zc1 = (zend + 15) / 16;
-    for (long it = tid; it < (long)a.n_mod * chunks; it += blockDim.x) {
-        const int md = (int)(it / chunks);
-        const long ch = it - (long)md * chunks;
-        const uint4 v = *reinterpret_cast<const uint4 *>(lines + (size_t)md * kpad + ch * 16);
-        const long o = ((long)md * a.nrows_total + grow) * kpad + ch * 16;
-        *reinterpret_cast<uint4 *>(a.resA + o) = v;
-        if (a.resB) {
-            if (nz > 0 && ch >= zc0 && ch < zc1) {
-                unsigned char tmp[16];
-                *reinterpret_cast<uint4 *>(tmp) = v;
-                for (int b = 0; b < 16; ++b) {
-                    const long c = ch * 16 + b;
-                    if (c >= kbody && c < zend) tmp[b] = zneg[md * CELL_ZMAX + (c - kbody)];
-                }
-                *reinterpret_cast<uint4 *>(a.resB + o) = *reinterpret_cast<const uint4 *>(tmp);
-            } else {
-                *reinterpret_cast<uint4 *>(a.resB + o) = v;
+    double *scl = mom + 2 * R;  // [R]: the rows' scales 2^(bits - e)
+    if (tid < R) {
+        const int r = tid;
+        uint32_t t = 0u;
+        double xs = 0.0, zs = 0.0;
+        for (int w = 0; w < nwarp; ++w) {
+            t = max(t, rtop[w * R + r]);
+            xs += rsum[(w * R + r) * 2];
+            zs += rsum[(w * R + r) * 2 + 1];
+        }
+        // every |x| < 2^ex; a row below the normal range counts as zero
+        const bool bad = t == 0x7ff00000u, some = t != 0u && !bad;
+        const int ex = some ? (int)(t >> 20) - 1022 : 0;
+        scl[r] = some ? ldexp(1.0, a.bits - ex) : 0.0;
+        // a non-finite row gets a NaN scale: its residues are zero and every
+        // entry it reaches is NaN, which the contraction reports
+        a.rowscale[grow + r] =
+            bad ? __longlong_as_double(0x7ff8000000000000LL) : (some ? ldexp(1.0, ex - a.bits) : 0.0);
+        const double *g0 = core + r * 2 * NG, *gg0 = g0 + NG;
+        double n1 = 0.0, n2 = 0.0, gg = 0.0;
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            n1 = fma(g0[i], g0[i], n1);
+            n2 = fma(gg0[i], gg0[i], n2);
+            gg = fma(g0[i], gg0[i], gg);
+        }
+        const double a_sx = mom[2 * r], q_sx = mom[2 * r + 1];
+        double *lf = a.left + (grow + r) * a.cwp, *rt = a.right + (grow + r) * a.cwp;
+        lf[NG] = rt[NG + 1] = a_sx;
+        lf[NG + 1] = rt[NG] = q_sx;
+        for (int i = NG + 2; i < a.cwp; ++i) lf[i] = rt[i] = 0.0;
+        write_row_record(a.cbound + (grow + r) * CB_STRIDE, some ? 1.0 : 0.0, ex, n1, n2, a_sx, q_sx, xs, zs, gg);
+    }
+    __syncthreads();
+    // residues: item = (row, four columns)
+    const int words = (int)(a.kpad / 4);
+    for (int it = tid; it < R * words; it += blockDim.x) {
+        const int r = it / words, c0 = (it - r * words) * 4;
+        const double scale = scl[r];
+        const double *x = img + r * ld + GS;
+        const int zlive = scale != 0.0 ? zend : 0;
+        float l0[4], l1[4], l2[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const int c = c0 + s;
+            // the scaled value rounded to an integer of at most bits + 1 bits: the low bits of the sum;
+            // a zero scale (an empty or non-finite row) gives zero
+            const double v = c < zlive ? x[GS == NG ? c : c + c / NG] : 0.0;
+            const double y = __fma_rn(v, scale, 6755399441055744.0);  // 1.5 * 2^52
+            const uint32_t lo = (uint32_t)__double2loint(y), hi = (uint32_t)__double2hiint(y);
+            l0[s] = __fadd_rn(__uint_as_float((lo & 0x3fffu) | 0x4b000000u), -8388608.0f);
+            l1[s] = __fadd_rn(__uint_as_float(((lo >> 14) & 0x3fffu) | 0x4b000000u), -8388608.0f);
+            // (hi : lo) >> 28, signed: the sum's exponent and leading bit are 0x43380000 in hi
+            l2[s] = __fadd_rn(__uint_as_float(__funnelshift_r(lo, hi, 28) + (0x4b400000u - 0x33800000u)), -12582912.0f);
+        }
+        signed char *pa = a.resA + (grow + r) * a.kpad + c0;
+        const long slab = a.nrows_total * a.kpad;
+        auto residues = [&](int md, float (&t)[4]) {
+            const float4 v = f.mod[md];  // m, 1/m, 2^14 mod m, 2^28 mod m
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                // |u| < 2^22: exact; the quotient rounds to the nearest integer (or either, at a tie of an even m)
+                const float u = __fmaf_rn(l2[s], v.w, __fmaf_rn(l1[s], v.z, l0[s]));
+                const float qf = __fadd_rn(__fmaf_rn(u, v.y, 12582912.0f), -12582912.0f);
+                t[s] = __fmaf_rn(-qf, v.x, u);  // in [-128, 128]
+            }
+        };
+        auto byte = [](float t) { return __float_as_uint(__fadd_rn(t, 12582912.0f)); };  // in the low eight bits
+        auto word = [&](const float (&t)[4]) {
+            return __byte_perm(__byte_perm(byte(t[0]), byte(t[1]), 0x0040), __byte_perm(byte(t[2]), byte(t[3]), 0x0040),
+                               0x5410);
+        };
+        if (!a.resB || c0 < a.b_col0 || c0 >= a.b_col0 + a.b_ld) {
+#pragma unroll 2
+            for (int md = 0; md < a.n_mod; ++md, pa += slab) {
+                float t[4];
+                residues(md, t);
+                *reinterpret_cast<uint32_t *>(pa) = word(t);
+            }
+        } else {
+            signed char *pb = a.resB + (grow + r) * a.b_ld + (c0 - a.b_col0);
+            const long slab_b = a.nrows_total * a.b_ld;
+#pragma unroll 1
+            for (int md = 0; md < a.n_mod; ++md, pa += slab, pb += slab_b) {
+                float t[4];
+                residues(md, t);
+                *reinterpret_cast<uint32_t *>(pa) = word(t);
+#pragma unroll
+                for (int s = 0; s < 4; ++s)  // B holds the residues of -z
+                    if (c0 + s >= kbody) t[s] = -t[s];
+                *reinterpret_cast<uint32_t *>(pb) = word(t);
             }
         }
     }
 }
+
+template <int NG>
+__global__ void __launch_bounds__(256, 2) split_rows_cell_kernel(const __grid_constant__ RowsArgs a,
+                                                              const __grid_constant__ ResidueArgs f,
+                                                              const double *__restrict__ ktab_t,
+                                                              const long *__restrict__ koff_t, int zmax) {
+    constexpr int R = cell_rows(NG);
+    extern __shared__ __align__(16) double sm[];
+    double *img = sm;                                          // [R][cell_image]
+    double *red = sm + R * cell_image(NG, a.nv, zmax);           // block scratch (cell_scratch doubles)
+    const long q0 = (long)blockIdx.x * R;
+    bool same = q0 + R <= a.nrows;
+    for (int r = 1; same && r < R; ++r) same = a.row_k[q0 + r] == a.row_k[q0];
+    if (same) {
+        cell_rows_body<NG, R>(a, f, ktab_t, koff_t, q0, zmax, img, red);
+        return;
+    }
+    // the last rows, and rows at a change of multipole: one at a time
+    for (long q = q0; q < a.nrows && q < q0 + R; ++q) {
+        cell_rows_body<NG, 1>(a, f, ktab_t, koff_t, q, zmax, img, red);
+        __syncthreads();
+    }
+}
+// doubles of block scratch: warp sums and maxima, the core vectors and moments, the scales
+constexpr int cell_scratch(int ng) { return cell_rows(ng) * (8 * 4 + 2 * ng + 2 + 1); }
 
 // =========================================================================
 // K3s — tcgen05 INT8 residue SYRK with CRT epilogue
@@ -775,6 +888,7 @@ struct CrtArgs {
     double corr_floor;  // skip the FP64 core correction of a warp block when its bound is below this
     int cwp, cw;
     const long *grp_row0, *grp_n, *grp_kdim, *grp_out;
+    const int *grp_zc;  // first 128-column chunk that B holds for itself (null: all)
     const int *tasks;
     long n_tasks, nrows_total;
     double *out;
@@ -948,7 +1062,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 for (long t = blockIdx.x; t < p.n_tasks && ok; t += gridDim.x) {
                     const int g = p.tasks[3 * t], ti = p.tasks[3 * t + 1], tj = p.tasks[3 * t + 2];
                     const long row0 = p.grp_row0[g];
-                    const int nk = (int)(p.grp_kdim[g] / BKB);
+                    const int nk = (int)(p.grp_kdim[g] / BKB), zc = p.grp_zc ? p.grp_zc[g] : 0;
                     for (int md = 0; md < n_mod && ok; ++md) {
                         const int ya = (int)(md * p.nrows_total + row0 + (long)ti * BM);
                         const int yb = (int)(md * p.nrows_total + row0 + (long)tj * BN);
@@ -959,7 +1073,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                             unsigned char *sa = ring + (size_t)s * STAGE_BYTES;
                             mbar_expect_tx(&full[s], STAGE_BYTES);
                             tma_load(sa, &mapA, kc * BKB, ya, &full[s]);
-                            tma_load(sa + BM * BKB, &mapB, kc * BKB, yb, &full[s]);
+                            if (kc < zc) tma_load(sa + BM * BKB, &mapA, kc * BKB, yb, &full[s]);
+                            else tma_load(sa + BM * BKB, &mapB, (kc - zc) * BKB, yb, &full[s]);
                         }
                     }
                 }
@@ -1337,13 +1452,14 @@ extern "C" int rkb_split_rows(const double *d_Pv, const double *d_Qv, long orb_l
     return RKB_OK;
 }
 
-extern "C" int rkb_split_rows_cells(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
-                                    const long *d_row_pair, const int *d_row_k, long nrows, const double *d_w,
-                                    int nv, int ng, const double *d_ktab, const long *d_koff,
-                                    const double *d_ktab_t, const long *d_koff_t, int max_z, int bits,
-                                    int n_mod, const int *moduli, signed char *d_resA, signed char *d_resB,
-                                    long kpad, long row_base, long nrows_total, double *d_rowscale, double *d_left,
-                                    double *d_right, double *d_cbound, int cwp, void *stream) {
+extern "C" int rkb_split_rows_cells_z(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
+                                      const long *d_row_pair, const int *d_row_k, long nrows, const double *d_w,
+                                      int nv, int ng, const double *d_ktab, const long *d_koff,
+                                      const double *d_ktab_t, const long *d_koff_t, int max_z, int bits,
+                                      int n_mod, const int *moduli, signed char *d_resA, signed char *d_resB,
+                                      long kpad, long b_col0, long b_ld, long row_base, long nrows_total,
+                                      double *d_rowscale, double *d_left, double *d_right, double *d_cbound, int cwp,
+                                      void *stream) {
     RKB_CHECK_ARG(nv >= 2 && ng >= 5 && ng <= 11, "the cell row kernel takes 5 <= ng <= 11 (got %d)", ng);
     RKB_CHECK_ARG(max_z >= 0 && max_z <= CELL_ZMAX, "the cell row kernel takes <= %d Z columns (got %d)", CELL_ZMAX,
                   max_z);
@@ -1359,8 +1475,12 @@ extern "C" int rkb_split_rows_cells(const double *d_Pv, const double *d_Qv, long
     RKB_CHECK_ARG(row_base >= 0 && row_base + nrows <= nrows_total, "row range outside the residue matrices");
     RKB_CHECK_ARG(((uintptr_t)d_resA % 16) == 0 && (d_resB == nullptr || ((uintptr_t)d_resB % 16) == 0),
                   "residue buffers must be 16-byte aligned");
+    RKB_CHECK_ARG(d_resB == nullptr || (b_col0 % BKB == 0 && b_col0 >= 0 && b_col0 <= (long)(nv - 1) * ng &&
+                                        b_ld % BKB == 0 && b_ld >= (long)(nv - 1) * ng + max_z - b_col0),
+                  "B must start at a multiple of %d columns within the body and hold every Z column", BKB);
     if (nrows == 0) return RKB_OK;
     RowsArgs a = {};
+    a.b_col0 = (int)b_col0; a.b_ld = b_ld;
     a.P = d_Pv; a.Q = d_Qv; a.orb_ld = orb_ld; a.pairs = d_pairs; a.row_pair = d_row_pair; a.row_k = d_row_k;
     a.nrows = nrows; a.w = d_w; a.nv = nv; a.ng = ng; a.ktab = d_ktab; a.koff = d_koff; a.bits = bits;
     a.n_mod = n_mod;
@@ -1373,14 +1493,21 @@ extern "C" int rkb_split_rows_cells(const double *d_Pv, const double *d_Qv, long
     a.resA = d_resA; a.resB = d_resB; a.kpad = kpad; a.row_base = row_base; a.nrows_total = nrows_total;
     a.rowscale = d_rowscale; a.left = d_left; a.right = d_right; a.cbound = d_cbound; a.cwp = cwp;
     RKB_CHECK_ARG(d_ktab_t != nullptr && d_koff_t != nullptr, "the cell-minor factor tables are required");
-    const size_t smem = ((((size_t)nv * (ng | 1) + 64 + 1) & ~(size_t)1) * sizeof(double)) + (size_t)n_mod * (kpad + CELL_ZMAX);
+    const int rows = cell_rows(ng);
+    const size_t smem = sizeof(double) * (size_t)(rows * cell_image(ng, nv, max_z) + cell_scratch(ng));
     RKB_CHECK_ARG(smem <= 200 * 1024, "row images too large for shared memory");
+    ResidueArgs f = {};
+    for (int i = 0; i < n_mod; ++i) {
+        const int m = moduli[i];
+        auto near = [m](long v) { return (float)(2 * (v % m) > m ? v % m - m : v % m); };
+        f.mod[i] = make_float4((float)m, 1.0f / (float)m, near(1L << 14), near(1L << 28));
+    }
     cudaStream_t st = as_stream(stream);
-    const dim3 grid((unsigned)nrows), block((unsigned)threads);
-#define RKB_CELL_CASE(NGV)                                                         \
-    case NGV:                                                                      \
-        RKB_CUDA(set_smem(split_rows_cell_kernel<NGV>, (int)smem));                \
-        split_rows_cell_kernel<NGV><<<grid, block, smem, st>>>(a, d_ktab_t, d_koff_t); \
+    const dim3 grid((unsigned)ceil_div(nrows, rows)), block((unsigned)threads);
+#define RKB_CELL_CASE(NGV)                                                                      \
+    case NGV:                                                                                   \
+        RKB_CUDA(set_smem(split_rows_cell_kernel<NGV>, (int)smem));                             \
+        split_rows_cell_kernel<NGV><<<grid, block, smem, st>>>(a, f, d_ktab_t, d_koff_t, max_z); \
         break;
     switch (ng) {
         RKB_CELL_CASE(5) RKB_CELL_CASE(6) RKB_CELL_CASE(7) RKB_CELL_CASE(8) RKB_CELL_CASE(9) RKB_CELL_CASE(10)
@@ -1390,6 +1517,18 @@ extern "C" int rkb_split_rows_cells(const double *d_Pv, const double *d_Qv, long
 #undef RKB_CELL_CASE
     RKB_LAUNCHED("split_rows_cell_kernel");
     return RKB_OK;
+}
+
+extern "C" int rkb_split_rows_cells(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
+                                    const long *d_row_pair, const int *d_row_k, long nrows, const double *d_w,
+                                    int nv, int ng, const double *d_ktab, const long *d_koff,
+                                    const double *d_ktab_t, const long *d_koff_t, int max_z, int bits,
+                                    int n_mod, const int *moduli, signed char *d_resA, signed char *d_resB,
+                                    long kpad, long row_base, long nrows_total, double *d_rowscale, double *d_left,
+                                    double *d_right, double *d_cbound, int cwp, void *stream) {
+    return rkb_split_rows_cells_z(d_Pv, d_Qv, orb_ld, d_pairs, d_row_pair, d_row_k, nrows, d_w, nv, ng, d_ktab, d_koff,
+                                  d_ktab_t, d_koff_t, max_z, bits, n_mod, moduli, d_resA, d_resB, kpad, 0, kpad,
+                                  row_base, nrows_total, d_rowscale, d_left, d_right, d_cbound, cwp, stream);
 }
 
 extern "C" long rkb_split_fused_body_width(int nv, int ng) {
@@ -1446,14 +1585,15 @@ extern "C" int rkb_split_rows_fused(const double *d_Pv, const double *d_Qv, long
     return RKB_OK;
 }
 
-extern "C" int rkb_split_contract(const signed char *d_resA, const signed char *d_resB, long kpad,
-                                  long nrows_total, int n_mod, const int *moduli, const int *pair_inv,
-                                  const double *f_hi,
-                                  const double *f_lo, double M, const double *d_rowscale, const double *d_left,
-                                  const double *d_right, const double *d_cbound, double corr_floor, int cw,
-                                  int cwp, const long *d_grp_row0,
-                                  const long *d_grp_n, const long *d_grp_kdim, const long *d_grp_out,
-                                  const int *d_tasks, long n_tasks, double *d_out, int *d_status, void *stream) {
+extern "C" int rkb_split_contract_z(const signed char *d_resA, const signed char *d_resB, long kpad, long b_ld,
+                                    long nrows_total, int n_mod, const int *moduli, double M,
+                                    const double *d_rowscale, const double *d_left, const double *d_right,
+                                    const double *d_cbound, double corr_floor, int cw, int cwp,
+                                    const long *d_grp_row0, const long *d_grp_n, const long *d_grp_kdim,
+                                    const int *d_grp_zchunk, const long *d_grp_out, const int *d_tasks,
+                                    long n_tasks, double *d_out, int *d_status, void *stream) {
+    RKB_CHECK_ARG(d_resB == nullptr || (b_ld % BKB == 0 && b_ld > 0 && b_ld <= kpad),
+                  "B's width must be a positive multiple of %d, <= kpad", BKB);
     RKB_CHECK_ARG(n_mod >= 1 && n_mod <= MAXMOD, "1..%d moduli supported (got %d)", MAXMOD, n_mod);
     RKB_CHECK_ARG(kpad % BKB == 0 && kpad > 0 && kpad <= 3456, "kpad must be a positive multiple of %d, <= 3456",
                   BKB);
@@ -1465,12 +1605,13 @@ extern "C" int rkb_split_contract(const signed char *d_resA, const signed char *
     CUtensorMap mA, mB;
     int rc = make_map(&mA, d_resA, kpad, (long)n_mod * nrows_total);
     if (rc) return rc;
-    rc = make_map(&mB, d_resB ? d_resB : d_resA, kpad, (long)n_mod * nrows_total);
+    rc = d_resB ? make_map(&mB, d_resB, b_ld, (long)n_mod * nrows_total) : make_map(&mB, d_resA, kpad, (long)n_mod * nrows_total);
     if (rc) return rc;
     CrtArgs p;
     p.rowscale = d_rowscale; p.left = d_left; p.right = d_right; p.cbound = d_cbound; p.corr_floor = corr_floor;
     p.cwp = cwp; p.cw = cw;
     p.grp_row0 = d_grp_row0; p.grp_n = d_grp_n; p.grp_kdim = d_grp_kdim; p.grp_out = d_grp_out;
+    p.grp_zc = d_resB ? d_grp_zchunk : nullptr;
     p.tasks = d_tasks; p.n_tasks = n_tasks; p.nrows_total = nrows_total; p.out = d_out; p.status = d_status;
     p.n_mod = n_mod; p.M = M * 0x1p-32;
     for (int i = 0; i < n_mod; ++i) RKB_CHECK_ARG(moduli[i] >= 2 && moduli[i] <= 256, "moduli must lie in [2, 256]");
@@ -1482,6 +1623,20 @@ extern "C" int rkb_split_contract(const signed char *d_resA, const signed char *
     crt_syrk_kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(mA, mB, p);
     RKB_LAUNCHED("crt_syrk_kernel");
     return RKB_OK;
+}
+
+extern "C" int rkb_split_contract(const signed char *d_resA, const signed char *d_resB, long kpad,
+                                  long nrows_total, int n_mod, const int *moduli, const int *pair_inv,
+                                  const double *f_hi,
+                                  const double *f_lo, double M, const double *d_rowscale, const double *d_left,
+                                  const double *d_right, const double *d_cbound, double corr_floor, int cw,
+                                  int cwp, const long *d_grp_row0,
+                                  const long *d_grp_n, const long *d_grp_kdim, const long *d_grp_out,
+                                  const int *d_tasks, long n_tasks, double *d_out, int *d_status, void *stream) {
+    (void)pair_inv, (void)f_hi, (void)f_lo;
+    return rkb_split_contract_z(d_resA, d_resB, kpad, kpad, nrows_total, n_mod, moduli, M, d_rowscale, d_left, d_right,
+                                d_cbound, corr_floor, cw, cwp, d_grp_row0, d_grp_n, d_grp_kdim, nullptr, d_grp_out,
+                                d_tasks, n_tasks, d_out, d_status, stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -306,6 +306,10 @@ class IonRows:
         self.kdim = {k: _round_up(self.body_w + self.nz[k], self.KCHUNK) for k in plan.ks}
         self.kmax_dim = max(self.kdim.values())
         self.has_z = max_z > 0
+        #: first column that the B residues hold for themselves: the columns
+        #: before it have no Z and are read from A (cell kernel; the other row
+        #: kernels write B whole)
+        self.b_col0 = self.kbody // self.KCHUNK * self.KCHUNK if kind == "cells" else 0
         if dt:
             self.zcount = dt["zcount"]
         else:
@@ -322,27 +326,30 @@ class IonRows:
         return np.concatenate([fused_body_positions(nv, ng), self.body_w + np.arange(self.nz[k])])
 
     def launch(self, bits: int, n_mod: int, moduli_c, resA, resB, kpad: int, row_base: int, nrows_total: int,
-               rowscale, left, right, cbound, cwp: int, xwork, stream) -> None:
+               rowscale, left, right, cbound, cwp: int, xwork, stream, b_col0: int = 0, b_ld: int | None = None) -> None:
         """Write this ion's rows at rows [row_base, row_base + n_rows) of the
-        [modulus][row][kpad] residue matrices (resA/resB, nrows_total rows)."""
+        [modulus][row][kpad] residue matrices (resA/resB, nrows_total rows);
+        ``b_col0``, ``b_ld``: resB holds the b_ld columns from b_col0 on only
+        (cell kernel)."""
         L = _native.load()
         dev, plan = self.dev, self.dev.plan
         rb = int(row_base)
         # the row range is folded into the base pointers (every modulus slab
         # shifts by the same row offset), so each launch sees rows from 0
         a_ptr = resA.data_ptr() + rb * kpad
-        b_ptr = resB.data_ptr() + rb * kpad if resB is not None else 0
+        b_ld = kpad if b_ld is None else int(b_ld)
+        b_ptr = resB.data_ptr() + rb * b_ld if resB is not None else 0
         rs, lf = rowscale.data_ptr() + 8 * rb, left.data_ptr() + 8 * rb * cwp
         rt, cb = right.data_ptr() + 8 * rb * cwp, cbound.data_ptr() + 8 * CB_STRIDE * rb
         if self.kind == "cells":
-            _native.check(L.rkb_split_rows_cells(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
-                                                 dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows,
-                                                 dev.w.data_ptr(), dev.nv, dev.ng, self.ktab.data_ptr(),
-                                                 self.koff.data_ptr(), self.ktab_t.data_ptr(), self.koff_t.data_ptr(),
-                                                 self.max_z, bits, n_mod, moduli_c, a_ptr,
-                                                 b_ptr, kpad, 0, nrows_total, rs, lf, rt, cb, cwp,
-                                                 _native.stream_handle(stream)),
-                          "rkb_split_rows_cells")
+            _native.check(L.rkb_split_rows_cells_z(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
+                                                   dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows,
+                                                   dev.w.data_ptr(), dev.nv, dev.ng, self.ktab.data_ptr(),
+                                                   self.koff.data_ptr(), self.ktab_t.data_ptr(),
+                                                   self.koff_t.data_ptr(), self.max_z, bits, n_mod, moduli_c, a_ptr,
+                                                   b_ptr, kpad, b_col0, b_ld, 0, nrows_total, rs, lf, rt, cb, cwp,
+                                                   _native.stream_handle(stream)),
+                          "rkb_split_rows_cells_z")
             return
         if self.fused:
             _native.check(L.rkb_split_rows_fused(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
@@ -386,9 +393,15 @@ class SplitEngine:
         nrows = plan.n_rows
         # rows padded to whole 128-row TMA boxes (zero rows never reach a stored entry)
         self.rows_alloc = _round_up(max(nrows, 1), 128)
-        self.resA = torch.zeros((self.n_mod, self.rows_alloc, self.kpad), dtype=torch.int8, device=d)
         self.has_z = any(self.nz[k] > 0 for k in plan.ks)
-        self.resB = torch.zeros_like(self.resA) if self.has_z else None
+        self.b_col0, self.b_ld = R.b_col0, self.kpad - R.b_col0
+        self.resA = torch.empty((self.n_mod, self.rows_alloc, self.kpad), dtype=torch.int8, device=d)
+        self._resB = (torch.empty((self.n_mod, self.rows_alloc, self.b_ld), dtype=torch.int8, device=d)
+                      if self.has_z and self.b_ld > 0 else None)
+        # the cell and two-kernel row paths write every column of their rows
+        for res in (self.resA, self._resB):
+            if res is not None:
+                (res if R.kind == "fused" else res[:, nrows:]).zero_()
         self.rowscale = torch.empty(nrows, dtype=torch.float64, device=d)
         self.left = torch.empty((nrows, self.cwp), dtype=torch.float64, device=d)
         self.right = torch.empty_like(self.left)
@@ -400,20 +413,28 @@ class SplitEngine:
         #: more than that; the split's own error is ~2^-bits of the same scale)
         self.corr_floor = 2.0 ** -(self.bits + 10) if corr_floor is None else float(corr_floor)
         sizes = [plan.n_of_k(k) for k in plan.ks]
-        self.grp_row0 = torch.as_tensor([plan.k_row_offset[k] for k in plan.ks], dtype=torch.int64, device=d)
-        self.grp_n = torch.as_tensor(sizes, dtype=torch.int64, device=d)
-        self.grp_kdim = torch.as_tensor([self.kdim[k] for k in plan.ks], dtype=torch.int64, device=d)
         offs_out = np.concatenate([[0], np.cumsum(np.asarray(sizes, dtype=np.int64) ** 2)])
-        self.grp_out = torch.as_tensor(offs_out[:-1], dtype=torch.int64, device=d)
         self.offsets = {k: int(offs_out[i]) for i, k in enumerate(plan.ks)}
         self.total = int(offs_out[-1])
         tasks = tile_tasks(sizes, block=TASK_BLOCK)
         self.n_tasks = int(tasks.shape[0])
-        self.tasks = torch.as_tensor(tasks.reshape(-1), device=d)
         # task range of each group (tasks are grouped by multipole) for streaming
         bounds = np.searchsorted(tasks[:, 0], np.arange(len(sizes) + 1))
         self.task_range = [(int(bounds[i]), int(bounds[i + 1])) for i in range(len(sizes))]
-        self.grp_out_zero = torch.zeros(len(sizes), dtype=torch.int64, device=d)
+        # the group records (and the zero offsets of the streaming path) and the
+        # task list, in one host-to-device copy
+        ng_ = len(sizes)
+        host = np.zeros(5 * ng_ + (tasks.size + ng_ + 1) // 2, dtype=np.int64)
+        host[:4 * ng_] = np.concatenate([[plan.k_row_offset[k] for k in plan.ks], sizes,
+                                         [self.kdim[k] for k in plan.ks], offs_out[:-1]])
+        words = host[5 * ng_:].view(np.int32)
+        words[:tasks.size] = tasks.reshape(-1)
+        words[tasks.size:tasks.size + ng_] = self.b_col0 // self.KCHUNK
+        arr = torch.from_numpy(host).to(d)
+        self.grp_row0, self.grp_n, self.grp_kdim, self.grp_out, self.grp_out_zero = (
+            arr[i * ng_:(i + 1) * ng_] for i in range(5))
+        words_d = arr[5 * ng_:].view(torch.int32)
+        self.tasks, self.grp_zc = words_d[:tasks.size], words_d[tasks.size:tasks.size + ng_]
         #: [contraction status, number of tables whose certificate failed]
         self.status = torch.zeros(2, dtype=torch.int32, device=d)
         #: certificate estimate of every multipole table (Schwarz-relative error)
@@ -424,12 +445,17 @@ class SplitEngine:
         self._stream = None
         #: the whole table (None when the engine only streams multipole tables)
         self.out = torch.empty(self.total, dtype=torch.float64, device=d) if materialize else None
-        self._mod_c = (np.ctypeslib.as_ctypes(np.ascontiguousarray(self.moduli, dtype=np.int32)),
-                       np.ctypeslib.as_ctypes(np.ascontiguousarray(self.f_hi)),
-                       np.ctypeslib.as_ctypes(np.ascontiguousarray(self.f_lo)),
-                       np.ctypeslib.as_ctypes(np.ascontiguousarray(np.concatenate([self.pair_inv, [1]]).astype(np.int32))))
+        self._mod_c = (np.ctypeslib.as_ctypes(np.ascontiguousarray(self.moduli, dtype=np.int32)),)
 
     dominant_kernel = "split::crt_syrk_kernel"
+
+    @property
+    def resB(self) -> torch.Tensor | None:
+        """The whole B operand (a copy of A's columns before ``b_col0``, then
+        what the row kernel wrote), assembled for inspection."""
+        if self._resB is None or self.b_col0 == 0:
+            return self._resB
+        return torch.cat([self.resA[:, :, :self.b_col0], self._resB], dim=2)
 
     @property
     def launches_per_step(self) -> int:
@@ -452,9 +478,9 @@ class SplitEngine:
             s = stream if stream is not None else torch.cuda.current_stream()
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record(s)
-        self.ion_rows.launch(self.bits, self.n_mod, self._mod_c[0], self.resA, self.resB, self.kpad, 0,
+        self.ion_rows.launch(self.bits, self.n_mod, self._mod_c[0], self.resA, self._resB, self.kpad, 0,
                              self.rows_alloc, self.rowscale, self.left, self.right, self.cbound, self.cwp,
-                             self.xwork, stream)
+                             self.xwork, stream, self.b_col0, self.b_ld)
         if ev is not None:
             ev[1].record(s)
             self.row_events.append(ev)
@@ -481,16 +507,15 @@ class SplitEngine:
 
     def _contract(self, grp_out, t0, t1, out, stream) -> None:
         L = _native.load()
-        _native.check(L.rkb_split_contract(self.resA.data_ptr(), _native.ptr(self.resB), self.kpad, self.rows_alloc,
-                                           self.n_mod, self._mod_c[0], self._mod_c[3], self._mod_c[1], self._mod_c[2],
-                                           self.M,
-                                           self.rowscale.data_ptr(), self.left.data_ptr(), self.right.data_ptr(),
-                                           self.cbound.data_ptr(), self.corr_floor, self.cw, self.cwp,
-                                           self.grp_row0.data_ptr(), self.grp_n.data_ptr(),
-                                           self.grp_kdim.data_ptr(), grp_out.data_ptr(),
-                                           self.tasks.data_ptr() + 12 * t0, t1 - t0, out.data_ptr(),
-                                           self.status.data_ptr(), _native.stream_handle(stream)),
-                      "rkb_split_contract")
+        _native.check(L.rkb_split_contract_z(self.resA.data_ptr(), _native.ptr(self._resB), self.kpad, self.b_ld,
+                                             self.rows_alloc, self.n_mod, self._mod_c[0], self.M,
+                                             self.rowscale.data_ptr(), self.left.data_ptr(), self.right.data_ptr(),
+                                             self.cbound.data_ptr(), self.corr_floor, self.cw, self.cwp,
+                                             self.grp_row0.data_ptr(), self.grp_n.data_ptr(),
+                                             self.grp_kdim.data_ptr(), self.grp_zc.data_ptr(), grp_out.data_ptr(),
+                                             self.tasks.data_ptr() + 12 * t0, t1 - t0, out.data_ptr(),
+                                             self.status.data_ptr(), _native.stream_handle(stream)),
+                      "rkb_split_contract_z")
 
     def stream_tables(self, sink, stream=None, check: bool = True) -> None:
         """Compute the rows once, then each multipole's table into one of two
@@ -601,7 +626,7 @@ class SplitEngine:
 
     def device_bytes(self) -> int:
         """Bytes of the engine's own device buffers (not the ion's inputs)."""
-        ts = [self.ktab, self.koff, self.resA, self.resB, self.rowscale, self.left, self.right, self.cbound,
+        ts = [self.ktab, self.koff, self.resA, self._resB, self.rowscale, self.left, self.right, self.cbound,
               self.xwork, self.zcount, self.tasks, self.est, self.out]
         return int(sum(t.numel() * t.element_size() for t in ts if t is not None))
 
@@ -672,7 +697,7 @@ class SplitEngine:
         per-row scale, core vectors and row records written."""
         d = self.dev
         reads = (d.Pv.numel() + d.Qv.numel()) * 8
-        res = self.n_mod * self.dev.plan.n_rows * self.kpad * (2 if self.resB is not None else 1)
+        res = self.n_mod * self.dev.plan.n_rows * (self.kpad + (self.b_ld if self._resB is not None else 0))
         per_row = 8 + 2 * 8 * self.cwp + 8 * 8
         return int(reads + res + self.dev.plan.n_rows * per_row)
 

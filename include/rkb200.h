@@ -285,6 +285,22 @@ int rkb_split_rows_cells(const double *d_Pv, const double *d_Qv, long orb_ld, co
                          long kpad, long row_base, long nrows_total, double *d_rowscale,
                          double *d_left, double *d_right, double *d_cbound, int cwp, void *stream);
 
+/* The same with a B matrix that holds only what differs from A.  B equals A
+ * but for the negated Z columns: with d_resB of n_mod x nrows_total rows of
+ * b_ld columns starting at column b_col0 (a multiple of 128, at most the body
+ * width (nv-1)*ng, and b_ld, a multiple of 128, wide enough for every Z
+ * column), only columns b_col0 .. b_col0 + b_ld - 1 (below kpad) are written
+ * there, and rkb_split_contract_z takes the chunks before b_col0 / 128 from A.  Half the
+ * bytes written and held; b_col0 = 0, b_ld = kpad is rkb_split_rows_cells. */
+int rkb_split_rows_cells_z(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
+                         const long *d_row_pair, const int *d_row_k, long nrows, const double *d_w,
+                         int nv, int ng, const double *d_ktab, const long *d_koff,
+                         const double *d_ktab_t, const long *d_koff_t, int max_z, int bits,
+                         int n_mod, const int *moduli, signed char *d_resA, signed char *d_resB,
+                         long kpad, long b_col0, long b_ld,
+                           long row_base, long nrows_total, double *d_rowscale,
+                         double *d_left, double *d_right, double *d_cbound, int cwp, void *stream);
+
 /* Host-only planning (no device work): the packed factored Green operator of
  * multipole k on the grid r (nv cells x ng nodes, mo/mi the ng x ng partial
  * matrices of atomx numerics/yk.py:65 yk_partial_matrices) with eigenvalue
@@ -337,6 +353,17 @@ int rkb_split_contract(const signed char *d_resA, const signed char *d_resB, lon
                        const long *d_grp_row0, const long *d_grp_n, const long *d_grp_kdim,
                        const long *d_grp_out, const int *d_tasks, long n_tasks, double *d_out,
                        int *d_status, void *stream);
+/* rkb_split_contract on the residues of rkb_split_rows_cells_z: group g's
+ * 128-column chunks before d_grp_zchunk[g] = b_col0 / 128 come from d_resA on
+ * both sides, the rest of B from d_resB (rows of b_ld columns).  Without
+ * d_resB, or with d_grp_zchunk null, as rkb_split_contract. */
+int rkb_split_contract_z(const signed char *d_resA, const signed char *d_resB, long kpad, long b_ld,
+                         long nrows_total, int n_mod, const int *moduli, double M,
+                         const double *d_rowscale, const double *d_left, const double *d_right,
+                         const double *d_cbound, double corr_floor, int cw, int cwp,
+                         const long *d_grp_row0, const long *d_grp_n, const long *d_grp_kdim,
+                         const int *d_grp_zchunk, const long *d_grp_out, const int *d_tasks,
+                         long n_tasks, double *d_out, int *d_status, void *stream);
 
 /* rkb_split_certify: per table g (rows d_grp_row0[g] .. + d_grp_n[g]) the
  * estimate d_est[g] = max_a h_a / sqrt|R_aa| * max_b |[X|Z]_b| / sqrt|R_bb|
