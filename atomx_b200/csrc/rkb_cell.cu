@@ -22,7 +22,7 @@
 #include <cmath>
 
 #include "rkb_common.cuh"
-#include "rkb_dmma.cuh"
+#include "rkb_dgemm.cuh"
 
 namespace rkb {
 namespace cell {
@@ -258,89 +258,26 @@ __global__ void densities_kernel(const double *__restrict__ c1, const double *__
 }
 
 // ------------------------------------------------------------- FP64 GEMM NT
-// C[m][n] (+)= sum_x A[m][x] B[n][x]: 128 x 128 tiles, 3-stage cp.async ring,
-// mma.sync m8n8k4 f64, one persistent CTA per SM over the tile list.
-constexpr int BM = 128, BN = 128, BK = 16, PAD = 4, LDS = BK + PAD, STAGES = 3, THREADS = 256;
-constexpr size_t GEMM_SMEM = (size_t)STAGES * (BM + BN) * LDS * sizeof(double);
-
-__device__ __forceinline__ void load_rows(double *s, const double *__restrict__ g, long ld, long row0, long nrows,
-                                          long k0) {
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        const int c = threadIdx.x + it * THREADS;
-        const int row = c >> 3, col = (c & 7) * 2;
-        const long grow = row0 + row;
-        const bool ok = grow < nrows;
-        cp_async16(s + row * LDS + col, g + (ok ? grow : row0) * ld + k0 + col, ok ? 16 : 0);
-    }
-}
-
-__global__ void __launch_bounds__(THREADS, 1)
+// C[m][n] (+)= sum_x A[m][x] B[n][x], a block per tile (rkb_dgemm.cuh).
+template <class T>
+__global__ void __launch_bounds__(dgemm::THREADS, 3)
 gemm_nt_kernel(const double *__restrict__ A, long lda, const double *__restrict__ B, long ldb, double *__restrict__ C,
                long ldc, long M, long N, long K, int accumulate) {
-    extern __shared__ double smem[];
-    double *As = smem, *Bs = smem + STAGES * BM * LDS;
+    extern __shared__ __align__(16) double smem[];
+    const long tn = (N + T::SIDE - 1) / T::SIDE;
+    const long i0 = blockIdx.x / tn * T::SIDE, j0 = blockIdx.x % tn * T::SIDE;
+    const double *o = T::run(A, lda, i0, M, B, ldb, j0, N, (int)(K / dgemm::BK), smem);
+    constexpr int WS = T::SIDE / 2, RPW = 32 / WS;  // rows a warp stores at a time
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = warp >> 2, wn = warp & 3, fr = lane >> 2, fc = lane & 3;
-    const long tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
-    const int nk = (int)(K / BK);
-    for (long t = blockIdx.x; t < tm * tn; t += gridDim.x) {
-        const long i0 = (t / tn) * BM, j0 = (t % tn) * BN;
-        double acc[8][4][2];
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-        __syncthreads();
-#pragma unroll
-        for (int s = 0; s < STAGES - 1; ++s) {
-            if (s < nk) {
-                load_rows(As + s * BM * LDS, A, lda, i0, M, (long)s * BK);
-                load_rows(Bs + s * BN * LDS, B, ldb, j0, N, (long)s * BK);
-            }
-            cp_async_commit();
+    const long j = j0 + warp % 2 * WS + lane % WS, i = i0 + warp / 2 * WS + lane / WS;
+    o += lane / WS * T::OLD + lane % WS;
+    if (j >= N) return;
+#pragma unroll 8
+    for (int r = 0; r < WS; r += RPW)
+        if (i + r < M) {
+            double *c = C + (i + r) * ldc + j;
+            *c = accumulate ? *c + o[r * T::OLD] : o[r * T::OLD];
         }
-        for (int kb = 0; kb < nk; ++kb) {
-            cp_async_wait<STAGES - 2>();
-            __syncthreads();
-            const int pf = kb + STAGES - 1;
-            if (pf < nk) {
-                const int s = pf % STAGES;
-                load_rows(As + s * BM * LDS, A, lda, i0, M, (long)pf * BK);
-                load_rows(Bs + s * BN * LDS, B, ldb, j0, N, (long)pf * BK);
-            }
-            cp_async_commit();
-            const double *a_s = As + (kb % STAGES) * BM * LDS + (wm * 64 + fr) * LDS + fc;
-            const double *b_s = Bs + (kb % STAGES) * BN * LDS + (wn * 32 + fr) * LDS + fc;
-#pragma unroll
-            for (int kk = 0; kk < BK; kk += 4) {
-                double af[8], bf[4];
-#pragma unroll
-                for (int a = 0; a < 8; ++a) af[a] = a_s[a * 8 * LDS + kk];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) bf[b] = b_s[b * 8 * LDS + kk];
-#pragma unroll
-                for (int a = 0; a < 8; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
-            }
-        }
-        cp_async_wait<0>();
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            const long i = i0 + wm * 64 + a * 8 + fr;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const long j = j0 + wn * 32 + b * 8 + fc * 2;
-#pragma unroll
-                for (int e = 0; e < 2; ++e)
-                    if (i < M && j + e < N) {
-                        double *c = C + i * ldc + j + e;
-                        *c = accumulate ? *c + acc[a][b][e] : acc[a][b][e];
-                    }
-            }
-        }
-    }
 }
 
 // ------------------------------------------------------------- gathered dots
@@ -647,16 +584,22 @@ extern "C" int rkb_cell_densities(const double *d_c1, const double *d_c2, long l
 
 extern "C" int rkb_gemm_nt_fp64(const double *d_A, long lda, const double *d_B, long ldb, double *d_C, long ldc,
                                 long M, long N, long K, int accumulate, void *stream) {
-    RKB_CHECK_ARG(M >= 0 && N >= 0 && K >= 0 && K % cell::BK == 0, "K (%ld) must be a multiple of %d", K, cell::BK);
+    RKB_CHECK_ARG(M >= 0 && N >= 0 && K >= 0 && K % dgemm::BK == 0, "K (%ld) must be a multiple of %d", K, dgemm::BK);
     RKB_CHECK_ARG(lda >= K && ldb >= K && ldc >= N && lda % 2 == 0 && ldb % 2 == 0,
                   "leading dimensions must cover the matrices (and lda, ldb be even)");
     RKB_CHECK_ARG(((uintptr_t)d_A % 16) == 0 && ((uintptr_t)d_B % 16) == 0, "A and B must be 16-byte aligned");
     if (M == 0 || N == 0) return RKB_OK;
-    const long tiles = ceil_div(M, cell::BM) * ceil_div(N, cell::BN);
-    const long grid = tiles < sm_count() ? tiles : sm_count();
-    RKB_CUDA(set_smem(cell::gemm_nt_kernel, (int)cell::GEMM_SMEM));
-    cell::gemm_nt_kernel<<<(unsigned)grid, cell::THREADS, cell::GEMM_SMEM, as_stream(stream)>>>(
-        d_A, lda, d_B, ldb, d_C, ldc, M, N, K, accumulate);
+    const long tiles = ceil_div(M, dgemm::Tile64::SIDE) * ceil_div(N, dgemm::Tile64::SIDE);
+    RKB_CHECK_ARG(tiles < (1L << 31), "result too large (%ld x %ld)", M, N);
+    auto launch = [&](auto tile) {
+        using T = decltype(tile);
+        RKB_CUDA(set_smem(cell::gemm_nt_kernel<T>, (int)T::SMEM));
+        cell::gemm_nt_kernel<T><<<(unsigned)(ceil_div(M, T::SIDE) * ceil_div(N, T::SIDE)), dgemm::THREADS, T::SMEM,
+                                  as_stream(stream)>>>(d_A, lda, d_B, ldb, d_C, ldc, M, N, K, accumulate);
+        return (int)RKB_OK;
+    };
+    const int st = dgemm::small_problem(tiles) ? launch(dgemm::Tile32()) : launch(dgemm::Tile64());
+    if (st) return st;
     RKB_LAUNCHED("cell::gemm_nt_kernel");
     return RKB_OK;
 }

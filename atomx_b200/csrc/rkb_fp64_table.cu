@@ -3,117 +3,48 @@
 // Y^k of its j-th pair (the slater_rk_poisson sum of atomx
 // numerics/bspline/slater.py:130 evaluated for a whole table at once).
 //
-// The table is symmetric in (ac)<->(bd), so only 128x128 tiles with
-// tile_j >= tile_i are computed; off-diagonal tiles are stored twice (as
-// computed and transposed).  Arithmetic is FP64 on the FP64 tensor pipe
-// (mma.sync m8n8k4 .f64 — sm_100a has no FP64 tcgen05 kind), operands staged
-// through shared memory by a 3-deep cp.async ring.  One persistent CTA per SM
-// walks a host-built task list (group, tile_i, tile_j).
-#include "rkb_common.cuh"
-#include "rkb_dmma.cuh"
+// The table is symmetric in (ac)<->(bd): the caller lists 128x128 tiles with
+// tile_j >= tile_i, and a block takes one 64x64 quarter of a listed tile
+// (rkb_dgemm.cuh; FP64 tensor pipe, sm_100a has no FP64 tcgen05 kind).  Quarters
+// below the diagonal of a diagonal tile are not computed.  Every entry above the
+// diagonal is stored twice, as computed and transposed, so the tables are symmetric
+// to the bit and do not depend on the tile size.
+#include "rkb_dgemm.cuh"
 
 namespace rkb {
 namespace fp64tab {
 
-constexpr int BM = 128, BN = 128, BK = 16, PAD = 4, LDS = BK + PAD, STAGES = 3;
-constexpr int THREADS = 256;  // 8 warps as 2 (M) x 4 (N); warp tile 64 x 32
-constexpr size_t SMEM = (size_t)STAGES * (BM + BN) * LDS * sizeof(double);
+constexpr int TILE = 128;  // the task list's tiles
 
-
-// Stage rows [row0, row0+128) x cols [k0, k0+BK) of a row-major (nrows x ld)
-// matrix into smem (128 x LDS); rows past nrows are zero-filled.
-__device__ __forceinline__ void load_tile(double *s, const double *__restrict__ g, long ld, long row0, long nrows,
-                                          long k0) {
-    // 128 rows x 16 doubles = 1024 chunks of 16 B; 4 per thread
-#pragma unroll
-    for (int it = 0; it < 4; ++it) {
-        int c = threadIdx.x + it * THREADS;
-        int row = c >> 3, col = (c & 7) * 2;
-        long grow = row0 + row;
-        bool ok = grow < nrows;
-        const double *src = g + (ok ? grow : row0) * ld + k0 + col;
-        cp_async16(s + row * LDS + col, src, ok ? 16 : 0);
-    }
-}
-
-__global__ void __launch_bounds__(THREADS, 1)
+template <class T>
+__global__ void __launch_bounds__(dgemm::THREADS, 3)
 contract_kernel(const double *__restrict__ G, const double *__restrict__ Y, long ld, long kdim,
                 const long *__restrict__ grp_kdim, const long *__restrict__ grp_row0, const long *__restrict__ grp_n,
-                const long *__restrict__ grp_out, const int *__restrict__ tasks, long n_tasks,
-                double *__restrict__ out) {
-    extern __shared__ double smem[];
-    double *As = smem;
-    double *Bs = smem + STAGES * BM * LDS;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wm = warp >> 2, wn = warp & 3;
-    const int fr = lane >> 2, fc = lane & 3;
-    for (long t = blockIdx.x; t < n_tasks; t += gridDim.x) {
-        const int g = tasks[3 * t], ti = tasks[3 * t + 1], tj = tasks[3 * t + 2];
-        const int nk = (int)((grp_kdim ? grp_kdim[g] : kdim) / BK);
-        const long row0 = grp_row0[g], n = grp_n[g];
-        const long i0 = (long)ti * BM, j0 = (long)tj * BN;
-        const double *Ag = G + row0 * ld, *Bg = Y + row0 * ld;
-
-        double acc[8][4][2];
-#pragma unroll
-        for (int a = 0; a < 8; ++a)
-#pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b][0] = acc[a][b][1] = 0.0;
-
-        __syncthreads();  // previous task's readers are done with the ring
-#pragma unroll
-        for (int s = 0; s < STAGES - 1; ++s) {
-            if (s < nk) {
-                load_tile(As + s * BM * LDS, Ag, ld, i0, n, (long)s * BK);
-                load_tile(Bs + s * BN * LDS, Bg, ld, j0, n, (long)s * BK);
-            }
-            cp_async_commit();
-        }
-        for (int kb = 0; kb < nk; ++kb) {
-            cp_async_wait<STAGES - 2>();
-            __syncthreads();
-            int pf = kb + STAGES - 1;
-            if (pf < nk) {
-                int s = pf % STAGES;
-                load_tile(As + s * BM * LDS, Ag, ld, i0, n, (long)pf * BK);
-                load_tile(Bs + s * BN * LDS, Bg, ld, j0, n, (long)pf * BK);
-            }
-            cp_async_commit();
-            const double *a_s = As + (kb % STAGES) * BM * LDS + (wm * 64 + fr) * LDS + fc;
-            const double *b_s = Bs + (kb % STAGES) * BN * LDS + (wn * 32 + fr) * LDS + fc;
-#pragma unroll
-            for (int kk = 0; kk < BK; kk += 4) {
-                double af[8], bf[4];
-#pragma unroll
-                for (int a = 0; a < 8; ++a) af[a] = a_s[a * 8 * LDS + kk];
-#pragma unroll
-                for (int b = 0; b < 4; ++b) bf[b] = b_s[b * 8 * LDS + kk];
-#pragma unroll
-                for (int a = 0; a < 8; ++a)
-#pragma unroll
-                    for (int b = 0; b < 4; ++b) dmma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
-            }
-        }
-        cp_async_wait<0>();
-
-        double *R = out + grp_out[g];
-        const bool mirror = tj != ti;
-#pragma unroll
-        for (int a = 0; a < 8; ++a) {
-            long i = i0 + wm * 64 + a * 8 + fr;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                long j = j0 + wn * 32 + b * 8 + fc * 2;
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    if (i < n && j + e < n) {
-                        R[i * n + j + e] = acc[a][b][e];
-                        if (mirror) R[(j + e) * n + i] = acc[a][b][e];
-                    }
-                }
-            }
-        }
-    }
+                const long *__restrict__ grp_out, const int *__restrict__ tasks, double *__restrict__ out) {
+    extern __shared__ __align__(16) double smem[];
+    constexpr int SUB = TILE / T::SIDE;  // sub-tiles per side
+    const long t = blockIdx.x / (SUB * SUB);
+    const int sub = (int)(blockIdx.x % (SUB * SUB)), si = sub / SUB, sj = sub % SUB;
+    const int g = tasks[3 * t], ti = tasks[3 * t + 1], tj = tasks[3 * t + 2];
+    if (ti == tj && si > sj) return;
+    const long n = grp_n[g];
+    const long i0 = (long)ti * TILE + si * T::SIDE, j0 = (long)tj * TILE + sj * T::SIDE;
+    if (i0 >= n || j0 >= n) return;
+    const long row0 = grp_row0[g];
+    const double *o = T::run(G + row0 * ld, ld, i0, n, Y + row0 * ld, ld, j0, n,
+                             (int)((grp_kdim ? grp_kdim[g] : kdim) / dgemm::BK), smem);
+    constexpr int WS = T::SIDE / 2, RPW = 32 / WS;  // rows a warp stores at a time
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lr = lane / WS, lc = lane % WS;
+    const long i1 = i0 + warp / 2 * WS, j1 = j0 + warp % 2 * WS;
+    double *R = out + grp_out[g];
+    if (j1 + lc < n)
+#pragma unroll 8
+        for (int r = lr; r < WS; r += RPW)
+            if (i1 + r < n && i1 + r <= j1 + lc) R[(i1 + r) * n + j1 + lc] = o[r * T::OLD + lc];
+    if (i1 + lc < n)
+#pragma unroll 8
+        for (int c = lr; c < WS; c += RPW)
+            if (j1 + c < n && i1 + lc < j1 + c) R[(j1 + c) * n + i1 + lc] = o[lc * T::OLD + c];
 }
 
 }  // namespace fp64tab
@@ -125,11 +56,17 @@ static int launch_contract(const double *d_g, const double *d_y, long ld, long k
                            const long *d_grp_row0, const long *d_grp_n, const long *d_grp_out, const int *d_tasks,
                            long n_tasks, double *d_out, void *stream) {
     if (n_tasks == 0) return RKB_OK;
-    auto kern = fp64tab::contract_kernel;
-    RKB_CUDA(set_smem(kern, (int)fp64tab::SMEM));
-    long grid = n_tasks < sm_count() ? n_tasks : sm_count();
-    kern<<<(unsigned)grid, fp64tab::THREADS, fp64tab::SMEM, as_stream(stream)>>>(
-        d_g, d_y, ld, kdim, d_grp_kdim, d_grp_row0, d_grp_n, d_grp_out, d_tasks, n_tasks, d_out);
+    RKB_CHECK_ARG(n_tasks < (1L << 27), "too many tiles (%ld)", n_tasks);
+    auto launch = [&](auto tile) {
+        using T = decltype(tile);
+        constexpr long SUB = fp64tab::TILE / T::SIDE;
+        RKB_CUDA(set_smem(fp64tab::contract_kernel<T>, (int)T::SMEM));
+        fp64tab::contract_kernel<T><<<(unsigned)(SUB * SUB * n_tasks), dgemm::THREADS, T::SMEM, as_stream(stream)>>>(
+            d_g, d_y, ld, kdim, d_grp_kdim, d_grp_row0, d_grp_n, d_grp_out, d_tasks, d_out);
+        return (int)RKB_OK;
+    };
+    const int st = dgemm::small_problem(4 * n_tasks) ? launch(dgemm::Tile32()) : launch(dgemm::Tile64());
+    if (st) return st;
     RKB_LAUNCHED("fp64tab::contract_kernel");
     return RKB_OK;
 }
@@ -137,8 +74,8 @@ static int launch_contract(const double *d_g, const double *d_y, long ld, long k
 extern "C" int rkb_table_contract_fp64(const double *d_g, const double *d_y, long ld, long kdim,
                                        const long *d_grp_row0, const long *d_grp_n, const long *d_grp_out,
                                        const int *d_tasks, long n_tasks, double *d_out, void *stream) {
-    RKB_CHECK_ARG(kdim >= 0 && kdim % fp64tab::BK == 0 && ld >= kdim && ld % 2 == 0,
-                  "contraction length %ld must be a multiple of %d and <= ld (%ld, even)", kdim, fp64tab::BK, ld);
+    RKB_CHECK_ARG(kdim >= 0 && kdim % dgemm::BK == 0 && ld >= kdim && ld % 2 == 0,
+                  "contraction length %ld must be a multiple of %d and <= ld (%ld, even)", kdim, dgemm::BK, ld);
     return launch_contract(d_g, d_y, ld, kdim, nullptr, d_grp_row0, d_grp_n, d_grp_out, d_tasks, n_tasks, d_out,
                            stream);
 }
