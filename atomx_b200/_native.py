@@ -67,6 +67,8 @@ _SIGNATURES = {
     "rkb_cell_exchange_density": [_vp, _vp, _l, _i, _vp, _l, _l, _i, _vp, _vp],
     "rkb_cell_banded_to_full": [_vp, _i, _i, _l, _vp, _vp],
     "rkb_cell_fock_finish": [_vp, _vp, _i, _i, _l, _vp, _vp],
+    "rkb_fock_blocks": [_vp, _vp, _l, _l, _i, _i, _i, _i, _vp, _vp, _l, _i, _vp, _vp, _vp, _i, _vp, _i, _vp, _l, _vp,
+                        _vp, _vp, _vp, _vp],
     "rkb_split_contract": [_vp, _vp, _l, _l, _i, _vp, _vp, _vp, _vp, _d, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _vp,
                            _vp, _vp, _vp, _l, _vp, _vp, _vp],
     "rkb_split_contract_z": [_vp, _vp, _l, _l, _l, _i, _vp, _d, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _vp, _vp, _vp,

@@ -557,6 +557,10 @@ def compute_exchange_matrix_cell(orb_a_P, orb_a_Q, orb_b_P, orb_b_Q, bsp_data, k
 
 
 # ------------------------------------------------------ DBSR Fock blocks
+#: device bytes of exchange densities one launch of the Fock kernels works on
+_FOCK_BYTES = 512 << 20
+
+
 def build_hf_matrices_dbsr(targets, P_stack, Q_stack, angular_direct, angular_exchange, k_values, norms, bsp_data,
                            cache=None, skip_pq_exchange=False, stream=None):
     """Fock blocks (PP, QQ, PQ, QP) of several target orbitals at once, the
@@ -577,55 +581,49 @@ def build_hf_matrices_dbsr(targets, P_stack, Q_stack, angular_direct, angular_ex
     n_orb = int(np.asarray(P_stack).shape[0])
     P = _stack(list(np.asarray(P_stack)), ns, dev)
     Q = _stack(list(np.asarray(Q_stack)), ns, dev)
-    ld = P.shape[1]
-    comp = {1: P, 2: Q}
-    ad = np.asarray(angular_direct, dtype=np.float64)
-    ax = np.asarray(angular_exchange, dtype=np.float64)
-    H = torch.zeros((nt, 4, ns, ns), dtype=torch.float64, device=dev)
+    ks = [int(k) for k in k_values]
+    nk = len(ks)
+    banks = [cache.bank(k, stream) for k in ks]
     s = _native.stream_handle(stream)
-    tgt = torch.as_tensor(targets.astype(np.int32), device=dev)
-    slot = {(1, 1): 0, (2, 2): 1, (1, 2): 2, (2, 1): 3}
-    for ii, jj in ((1, 1), (1, 2), (2, 1), (2, 2)):
-        itype = {(1, 1): "pppp", (1, 2): "pqpq", (2, 1): "qpqp", (2, 2): "qqqq"}[ii, jj]
-        for k in k_values:
-            k = int(k)
-            bank = cache.bank(k, stream)
-            r0, c0, ks_bra, ks_ket = bank.offsets(itype)
-            a = np.ascontiguousarray(ad[targets, :, k])
-            b = np.ascontiguousarray(ax[targets, :, k])
-            if np.any(a):
-                coef = torch.as_tensor(a, device=dev)
-                kp = _round16(ks_ket * ns)
-                dd = torch.zeros((nt, kp), dtype=torch.float64, device=dev)
-                _native.check(L.rkb_cell_direct_density(comp[jj].data_ptr(), ld, n_orb, coef.data_ptr(), n_orb,
-                                                        tgt.data_ptr(), nt, ns, ks_ket, dd.data_ptr(), kp, s),
-                              "rkb_cell_direct_density")
-                v = torch.empty((nt, ks_bra * ns), dtype=torch.float64, device=dev)
-                kb = bank.K[r0:r0 + ks_bra * ns, c0:]
-                _native.check(L.rkb_gemm_nt_fp64(dd.data_ptr(), kp, kb.data_ptr(), bank.kdim, v.data_ptr(),
-                                                 ks_bra * ns, nt, ks_bra * ns, kp, 0, s), "rkb_gemm_nt_fp64")
-                tmp = torch.zeros((nt, ns, ns), dtype=torch.float64, device=dev)
-                _native.check(L.rkb_cell_banded_to_full(v.data_ptr(), ns, ks_bra, nt, tmp.data_ptr(), s),
-                              "rkb_cell_banded_to_full")
-                H[:, 0 if ii == 1 else 1] += tmp
-            if skip_pq_exchange and ii == 1 and jj == 2:
-                continue
-            if np.any(b):
-                coef = torch.as_tensor(b, device=dev)
-                xx = torch.empty((nt, ns, ns), dtype=torch.float64, device=dev)
-                _native.check(L.rkb_cell_exchange_density(comp[ii].data_ptr(), comp[jj].data_ptr(), ld, n_orb,
-                                                          coef.data_ptr(), n_orb, nt, ns, xx.data_ptr(), s),
-                              "rkb_cell_exchange_density")
-                kofs = torch.full((nt,), r0 * bank.kdim + c0, dtype=torch.int64, device=dev)
-                Kk = torch.empty((nt, ns, ns), dtype=torch.float64, device=dev)
-                _native.check(L.rkb_cell_exchange(bank.K.data_ptr(), bank.kdim, kofs.data_ptr(), xx.data_ptr(), nt, ns,
-                                                  ks_bra, ks_ket, int(ii == jj), 0, Kk.data_ptr(), s),
-                              "rkb_cell_exchange")
-                H[:, slot[ii, jj]] += Kk
-    out = torch.empty_like(H)
-    nrm = torch.as_tensor(np.asarray(norms, dtype=np.float64).reshape(-1), device=dev)
-    _native.check(L.rkb_cell_fock_finish(H.data_ptr(), nrm.data_ptr(), ns, int(bool(skip_pq_exchange)), nt,
-                                         out.data_ptr(), s), "rkb_cell_fock_finish")
+    out = torch.empty((nt, 4, ns, ns), dtype=torch.float64, device=dev)
+    if nt == 0:
+        return out
+    norms = np.asarray(norms, dtype=np.float64).reshape(-1)
+    if norms.shape[0] < nt:
+        raise ValueError(f"{nt} targets need as many norms (got {norms.shape[0]})")
+    # [multipole][target][orbital], as the kernels read them
+    ad = np.asarray(angular_direct, dtype=np.float64)[targets][:, :, ks].transpose(2, 0, 1)
+    ax = np.asarray(angular_exchange, dtype=np.float64)[targets][:, :, ks].transpose(2, 0, 1)
+    if banks:
+        ld, q_off, ks_p, ks_q = banks[0].kdim, banks[0].kp_pad, banks[0].ksp, banks[0].ksq
+    else:
+        ld, q_off, ks_p, ks_q = 2 * _round16(ns), _round16(ns), 1, 1
+    dd_ld = max(q_off, ld - q_off)
+    # targets in groups whose exchange densities stay below _FOCK_BYTES
+    group = min(nt, max(1, min(_FOCK_BYTES // (32 * max(nk, 1) * ns * ns), 65535 // (4 * max(nk, 1)))))
+    work = torch.empty(group * nk * (2 * dd_ld + 2 * ld + 4 * ns * ns) + group * 4 * ns * ns, dtype=torch.float64,
+                       device=dev)
+    kptr = np.array([b.K.data_ptr() for b in banks] + [0], dtype=np.int64)
+    for g0 in range(0, nt, group):
+        g1 = min(nt, g0 + group)
+        m = g1 - g0
+        # angular coefficients, norms, targets and bank addresses in one copy
+        parts = [ad[:, g0:g1], ax[:, g0:g1], norms[g0:g1], kptr.view(np.float64),
+                 np.concatenate([targets[g0:g1].astype(np.int32), np.zeros(m % 2, dtype=np.int32)]).view(np.float64)]
+        host = np.concatenate([np.ascontiguousarray(x).reshape(-1) for x in parts])
+        d = torch.from_numpy(host).to(dev)
+        p = [d.data_ptr() + 8 * int(x) for x in np.concatenate([[0], np.cumsum([x.size for x in parts])])]
+        w = [work.data_ptr() + 8 * int(x) for x in np.cumsum([0, 2 * m * nk * dd_ld, 2 * m * nk * ld,
+                                                               4 * m * nk * ns * ns])]
+        _native.check(L.rkb_fock_blocks(kptr.ctypes.data, p[3], ld, q_off, nk, ns, ks_p, ks_q, P.data_ptr(),
+                                        Q.data_ptr(), P.shape[1], n_orb, p[0], p[1], p[4], m, p[2],
+                                        int(bool(skip_pq_exchange)), w[0], dd_ld, w[1], w[2], w[3],
+                                        out[g0:g1].data_ptr(), s), "rkb_fock_blocks")
+        if stream is not None:  # the copy's memory is in use there
+            d.record_stream(stream)
+    if stream is not None:
+        for x in (work, P, Q):
+            x.record_stream(stream)
     return out
 
 

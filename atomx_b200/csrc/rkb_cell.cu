@@ -480,6 +480,144 @@ __global__ void fock_finish_kernel(const double *__restrict__ h, const double *_
     O[3 * per + ij] = fin(qp);
 }
 
+// ------------------------------------------------- Fock blocks of many targets
+// All the densities, and then all the exchange contractions, of a DBSR Fock step
+// in one launch each: component blocks (PP, QQ, PQ, QP), multipoles and targets
+// together.  Launched one (block, multipole) at a time they were 226 launches a step,
+// each too small for the chip.
+struct FockArgs {
+    const double *const *K;  // bank matrices of the nk multipoles (device array of device pointers)
+    long ld, q_off;          // their leading dimension, and the Q block's row and column offset
+    int nk, nt, n_orb, ns, ks[2];  // spline orders of P, Q
+    const double *comp[2];   // coefficient stacks P, Q
+    long c_ld;
+    const double *ad, *ax;   // angular coefficients [nk][nt][n_orb]
+    const int *target;
+    double *dd;              // direct densities [Q or P][nk][nt][dd_ld], zero padded
+    long dd_ld;
+    const double *v;         // their potentials [P or Q source][nk][nt][ld]
+    double *xx;              // exchange densities [block][nk][nt][ns][ns]
+    double *h;               // blocks [nt][4][ns][ns]
+    int skip_pq;
+};
+__global__ void fock_direct_density_kernel(const __grid_constant__ FockArgs f) {
+    const long x = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= f.dd_ld) return;
+    const int t = blockIdx.y % f.nt, kc = blockIdx.y / f.nt;  // kc = source component * nk + multipole
+    const int src = kc / f.nk, k = kc % f.nk;
+    const int s = (int)(x / f.ns), i = (int)(x % f.ns);
+    const double *c = f.ad + ((long)k * f.nt + t) * f.n_orb, *comp = f.comp[src];
+    double v = 0.0;
+    if (s < f.ks[src] && i + s < f.ns)
+        for (int j = 0; j < f.n_orb; ++j) {
+            double cj = c[j];
+            if (cj == 0.0) continue;
+            if (j == f.target[t]) cj = add(cj, cj);
+            const double pi = comp[(long)j * f.c_ld + i];
+            if (s == 0) v = add(v, mul(mul(cj, pi), pi));
+            else {
+                const double ps = comp[(long)j * f.c_ld + i + s];
+                v = add(v, mul(cj, add(mul(pi, ps), mul(ps, pi))));
+            }
+        }
+    f.dd[((long)kc * f.nt + t) * f.dd_ld + x] = v;
+}
+
+__global__ void fock_exchange_density_kernel(const __grid_constant__ FockArgs f) {
+    const int per = f.ns * f.ns;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= per) return;
+    const int t = blockIdx.y % f.nt, bk = blockIdx.y / f.nt;  // bk = block * nk + multipole
+    const int blk = bk / f.nk, k = bk % f.nk;
+    if (f.skip_pq && blk == 1) return;
+    const int i = e / f.ns, j2 = e % f.ns;
+    const double *c = f.ax + ((long)k * f.nt + t) * f.n_orb;
+    const double *pl = f.comp[blk >> 1] + i, *pr = f.comp[blk & 1] + j2;
+    double v = 0.0;
+    for (int j = 0; j < f.n_orb; ++j) {
+        const double cj = __ldg(c + j);
+        if (cj == 0.0) continue;
+        v = add(v, mul(mul(cj, __ldg(pl + j * f.c_ld)), __ldg(pr + j * f.c_ld)));
+    }
+    f.xx[((long)bk * f.nt + t) * per + e] = v;
+}
+
+// One thread per (row, column) entry of BT targets, which share each bank element
+// read.  The summation order of exchange_kernel is kept for every entry, and the sums
+// over blocks and multipoles are those of one block and multipole at a time.
+// Bound by the latency of the bank reads from L2.  A whole Fock step of 24 targets and
+// 8 multipoles at 120 splines took 6.0 ms in 226 launches, one target a thread (3.5 ms
+// of it in 32 exchange launches), and takes 2.67 ms with eight targets a thread; four
+// targets 3.07, twelve 3.65, four targets of two rows 4.1.
+constexpr int FOCK_THREADS = 128;  // columns a block
+template <int BT>
+__global__ void __launch_bounds__(FOCK_THREADS, 5) fock_exchange_kernel(const __grid_constant__ FockArgs f) {
+    const int ns = f.ns, blk = blockIdx.z & 3, t0 = (blockIdx.z >> 2) * BT;
+    const int left = blk >> 1, right = blk & 1, row = blockIdx.y, col = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool symmetric = left == right;
+    if ((f.skip_pq && blk == 1) || col >= ns || (symmetric && col > row)) return;
+    const int ks = f.ks[left], ks_r = f.ks[right];
+    const long per = (long)ns * ns, ld = f.ld;
+    double h[BT];
+#pragma unroll
+    for (int b = 0; b < BT; ++b) h[b] = 0.0;
+    // the banded direct potential of source component src through this block's bra component
+    auto direct = [&](int src, int k) {
+        const int s = row > col ? row - col : col - row;
+        if (s >= ks) return;
+        const long at = (left ? f.q_off : 0) + (long)s * ns + (row < col ? row : col);
+#pragma unroll
+        for (int b = 0; b < BT; ++b)
+            h[b] = add(h[b], __ldg(f.v + (((long)src * f.nk + k) * f.nt + min(t0 + b, f.nt - 1)) * ld + at));
+    };
+    if (blk == 3)
+        for (int k = 0; k < f.nk; ++k) direct(0, k);
+    for (int k = 0; k < f.nk; ++k) {
+        if (symmetric) direct(left, k);
+        const double *Kb = f.K[k] + (left ? f.q_off * ld : 0) + (right ? f.q_off : 0) + col;
+        const double *d[BT];
+        double s[BT];
+#pragma unroll
+        for (int b = 0; b < BT; ++b) {
+            d[b] = f.xx + (((long)blk * f.nk + k) * f.nt + min(t0 + b, f.nt - 1)) * per + col;
+            s[b] = 0.0;
+        }
+        // one step: density entry (i, col + off), bank element of the left pair of i and row
+        auto step = [&](int i, int jp, int off) {
+            if (col + off < 0 || col + off >= ns) return;
+            const int ip = row >= i ? row - i : i - row;
+            const double kv = __ldg(Kb + ((long)ip * ns + min(i, row)) * ld + (long)jp * ns + min(off, 0));
+#pragma unroll
+            for (int b = 0; b < BT; ++b) s[b] = add(s[b], mul(kv, __ldg(d[b] + (long)i * ns + off)));
+        };
+        const int i_lo = max(row - ks + 1, 0), i_hi = min(row + ks - 1, ns - 1);
+        for (int i = row; i >= i_lo; --i)
+#pragma unroll 2
+            for (int jp = 0; jp < ks_r; ++jp) step(i, jp, jp);
+        for (int i = row + 1; i <= i_hi; ++i)
+#pragma unroll 2
+            for (int jp = 0; jp < ks_r; ++jp) step(i, jp, jp);
+        for (int jp = 1; jp < ks_r; ++jp)
+#pragma unroll 2
+            for (int i = row; i >= i_lo; --i) step(i, jp, -jp);
+        for (int i = row + 1; i <= i_hi; ++i)
+#pragma unroll 2
+            for (int jp = 1; jp < ks_r; ++jp) step(i, jp, -jp);
+#pragma unroll
+        for (int b = 0; b < BT; ++b) h[b] = add(h[b], s[b]);
+    }
+    if (blk == 0)
+        for (int k = 0; k < f.nk; ++k) direct(1, k);
+    const int slot = blk == 0 ? 0 : blk == 1 ? 2 : blk == 2 ? 3 : 1;
+#pragma unroll
+    for (int b = 0; b < BT; ++b)
+        if (t0 + b < f.nt) {
+            double *o = f.h + ((long)(t0 + b) * 4 + slot) * per;
+            o[(long)row * ns + col] = h[b];
+            if (symmetric && col < row) o[(long)col * ns + row] = h[b];
+        }
+}
+
 }  // namespace cell
 }  // namespace rkb
 
@@ -686,6 +824,52 @@ extern "C" int rkb_cell_fock_finish(const double *d_h, const double *d_norm, int
     if (nbatch == 0) return RKB_OK;
     const long n = (long)ns * ns * nbatch;
     cell::fock_finish_kernel<<<blocks_for(n), 256, 0, as_stream(stream)>>>(d_h, d_norm, ns, skip_pq, d_out, nbatch);
+    RKB_LAUNCHED("cell::fock_finish_kernel");
+    return RKB_OK;
+}
+
+extern "C" int rkb_fock_blocks(const void *const *K, const void *d_K, long ld, long q_off, int nk, int ns, int ks_p,
+                               int ks_q, const double *d_P, const double *d_Q, long c_ld, int n_orb,
+                               const double *d_ad, const double *d_ax, const int *d_target, int nt,
+                               const double *d_norm, int skip_pq, double *d_dd, long dd_ld, double *d_v, double *d_xx,
+                               double *d_h, double *d_out, void *stream) {
+    RKB_CHECK_ARG(ns >= 1 && nk >= 0 && nt >= 0 && n_orb >= 0 && ks_p >= 1 && ks_q >= 1, "invalid sizes");
+    RKB_CHECK_ARG(q_off >= (long)ks_p * ns && ld >= q_off + (long)ks_q * ns && c_ld >= ns,
+                  "leading dimensions must cover the blocks");
+    RKB_CHECK_ARG(dd_ld % dgemm::BK == 0 && q_off % dgemm::BK == 0 && (ld - q_off) % dgemm::BK == 0 &&
+                      dd_ld >= q_off && dd_ld >= ld - q_off,
+                  "block widths must be multiples of %d, and dd_ld cover them", dgemm::BK);
+    RKB_CHECK_ARG((long)4 * nk * nt <= 65535 && ns <= 65535, "too many targets and multipoles (%d x %d)", nt,
+                  nk);
+    RKB_CHECK_ARG(d_h != d_out, "the output must not alias the blocks");
+    if (nt == 0) return RKB_OK;
+    cudaStream_t st = as_stream(stream);
+    const long per = (long)ns * ns;
+    RKB_CUDA(cudaMemsetAsync(d_h, 0, sizeof(double) * 4 * per * nt, st));
+    if (nk > 0) {
+        cell::FockArgs f = {};
+        f.K = static_cast<const double *const *>(d_K);
+        f.ld = ld; f.q_off = q_off; f.nk = nk; f.nt = nt; f.n_orb = n_orb; f.ns = ns; f.ks[0] = ks_p; f.ks[1] = ks_q;
+        f.comp[0] = d_P; f.comp[1] = d_Q; f.c_ld = c_ld; f.ad = d_ad; f.ax = d_ax; f.target = d_target;
+        f.dd = d_dd; f.dd_ld = dd_ld; f.v = d_v; f.xx = d_xx; f.h = d_h; f.skip_pq = skip_pq;
+        cell::fock_direct_density_kernel<<<dim3(blocks_for(dd_ld), 2u * nk * nt), 256, 0, st>>>(f);
+        RKB_LAUNCHED("cell::fock_direct_density_kernel");
+        for (int src = 0; src < 2; ++src)
+            for (int k = 0; k < nk; ++k) {
+                const long at = ((long)src * nk + k) * nt, width = src ? ld - q_off : q_off;
+                const int rc = rkb_gemm_nt_fp64(d_dd + at * dd_ld, dd_ld,
+                                                static_cast<const double *>(K[k]) + (src ? q_off : 0), ld, d_v + at * ld,
+                                                ld, nt, ld, width, 0, stream);
+                if (rc != RKB_OK) return rc;
+            }
+        cell::fock_exchange_density_kernel<<<dim3(blocks_for(per), 4u * nk * nt), 256, 0, st>>>(f);
+        RKB_LAUNCHED("cell::fock_exchange_density_kernel");
+        constexpr int BT = 8;
+        cell::fock_exchange_kernel<BT><<<dim3((unsigned)ceil_div(ns, cell::FOCK_THREADS), (unsigned)ns,
+                                              4u * (unsigned)ceil_div(nt, BT)), cell::FOCK_THREADS, 0, st>>>(f);
+        RKB_LAUNCHED("cell::fock_exchange_kernel");
+    }
+    cell::fock_finish_kernel<<<blocks_for(per * nt), 256, 0, st>>>(d_h, d_norm, ns, skip_pq, d_out, nt);
     RKB_LAUNCHED("cell::fock_finish_kernel");
     return RKB_OK;
 }

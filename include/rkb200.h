@@ -453,6 +453,19 @@ int rkb_cell_banded_to_full(const double *d_v, int ns, int ks, long nbatch, doub
 int rkb_cell_fock_finish(const double *d_h, const double *d_norm, int ns, int skip_pq, long nbatch, double *d_out,
                          void *stream);
 
+/* The whole of _build_hf_matrix_dbsr for nt targets (what the entry points
+ * above do per component block and multipole): K, nk bank matrices of leading
+ * dimension ld (a HOST array of device pointers, and the same on the device),
+ * Q rows and columns from q_off on; d_ad, d_ax the angular coefficients
+ * [nk][nt][n_orb]; workspaces d_dd (2 nk nt dd_ld doubles, dd_ld >= both block
+ * widths), d_v (2 nk nt ld), d_xx (4 nk nt ns^2) and d_h (4 nt ns^2); d_out
+ * receives (PP, QQ, PQ, QP) of every target, symmetrised and divided by its
+ * norm.  4 nk nt <= 65535. */
+int rkb_fock_blocks(const void *const *K, const void *d_K, long ld, long q_off, int nk, int ns, int ks_p, int ks_q,
+                    const double *d_P, const double *d_Q, long c_ld, int n_orb, const double *d_ad,
+                    const double *d_ax, const int *d_target, int nt, const double *d_norm, int skip_pq, double *d_dd,
+                    long dd_ld, double *d_v, double *d_xx, double *d_h, double *d_out, void *stream);
+
 /* ---------------------------------------------------------------------------
  * rkb_split_rows_noalloc: no counterpart in the reference (an addition of this
  * library).  The same computation and arguments as rkb_split_rows, without
