@@ -14,22 +14,36 @@
 //            a_j = rho_j rk_j, likewise rescaled;
 //            y_i = inner_i inverse_i + rk_i y_i,  y_0 = y_0 rk_0
 //
-// The reference runs both scans serially per row.  Here one CTA owns a row:
-// each frame is scanned in tiles of TILE points with a block-wide exclusive
-// prefix (outward) or suffix (inward) sum, formed without subtractions (a
-// difference of partial sums would cancel on grids whose terms grow along
-// the row), and the carry between tiles and frames is kept in shared memory
-// and rescaled exactly where the reference rescales it.  Rows are independent (persistent CTAs walk the row list).  The
-// summation order inside a frame differs from the serial one, so results
-// agree with the reference to rounding, not bit for bit.
+// With h_i half the interval between points i and i + 1 (h_(-1) = h_(n-1) = 0), w_i = h_(i-1) +
+// h_i, and t_i = 1 except at a frame's first point, where it is the transfer, both
+// are first-order recurrences in one point's value at a time:
+//
+//   inward:  A_i = t_(i+1) A_(i+1) + w_i b_i,   acc_i = t_(i+1) A_(i+1) + h_i b_i
+//   outward: B_i = t_i B_(i-1) + w_i a_i,       inner_i = t_i B_(i-1) + h_(i-1) a_i
+//
+// The reference runs them serially per row.  Here one CTA owns a row and cuts it into
+// tiles of TILE points, a warp per tile: a first pass sums every tile's terms, a scan over
+// the tiles gives each its two carries, and a second pass scans inside the tiles and
+// forms y and its dots with up to FUSED consumers (a row with more takes the second
+// pass again).  No tile waits for another, the batch stores no y, and all loads are
+// coalesced (consecutive lanes, consecutive points).  Sums are formed without
+// subtractions: a difference of partial sums would cancel on grids whose terms grow
+// along the row.  The summation order differs from the serial one, so results agree
+// with the reference to rounding, not bit for bit.
+//
+// Bound by instruction issue (two passes of nine loads and about fifteen FP64
+// operations a point, two warp scans in the second).  4000 rows x 20 000 points with 2
+// consumers: tile after tile with block-wide scans and y in memory 2.87 ms, this form
+// 1.10 ms (tiles of 64, 192, 256 points: 1.2 to 1.4 ms).
 #include "rkb_common.cuh"
 
 namespace rkb {
 namespace grid {
 
-constexpr int THREADS = 256;
-constexpr int ITEMS = 4;
-constexpr int TILE = THREADS * ITEMS;
+constexpr int THREADS = 256, WARPS = THREADS / 32;
+constexpr int CH = 4, TILE = 32 * CH;  // chunks of 32 points per tile
+constexpr int FUSED = 4;               // consumers dotted in one second pass
+constexpr unsigned FULL = 0xffffffffu;
 
 struct Tables {
     const double *r, *rk, *inverse;  // rk / inverse: the row's multipole, n values
@@ -39,137 +53,181 @@ struct Tables {
     long n, i_cut;
 };
 
-// Density of a row: either a sampled rho, or P_a P_b + Q_a Q_b formed on the
+// Density of a row: a sampled rho, or P_a P_b + Q_a Q_b formed on the
 // fly (quadrature.py:313-352 forms it in the same way).
-struct Dens {
-    const double *rho, *Pa, *Qa, *Pb, *Qb;
-    __device__ __forceinline__ double operator()(long i) const {
-        return rho ? rho[i] : __dadd_rn(__dmul_rn(Pa[i], Pb[i]), __dmul_rn(Qa[i], Qb[i]));
+struct DensRow {
+    const double *rho;
+    __device__ __forceinline__ DensRow from(long i) const { return DensRow{rho + i}; }
+    __device__ __forceinline__ double operator()(int i) const { return __ldg(rho + i); }
+};
+struct DensPair {
+    const double *Pa, *Qa, *Pb, *Qb;
+    __device__ __forceinline__ DensPair from(long i) const { return DensPair{Pa + i, Qa + i, Pb + i, Qb + i}; }
+    __device__ __forceinline__ double operator()(int i) const {
+        return __dadd_rn(__dmul_rn(__ldg(Pa + i), __ldg(Pb + i)), __dmul_rn(__ldg(Qa + i), __ldg(Qb + i)));
     }
 };
 
-// Block-wide exclusive scan of one double per thread (sum over lower
-// threadIdx), formed without subtracting: the lane below's inclusive value
-// plus the totals of the lower warps.  *total receives the block's sum.
-__device__ __forceinline__ double block_scan_excl(double v, double *sh, double *total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const double incl = warp_inclusive_scan(v, lane);
-    const double below = __shfl_up_sync(0xffffffffu, incl, 1);
-    if (lane == 31) sh[wid] = incl;
-    __syncthreads();
-    double before = 0.0, all = 0.0;
-    for (int w = 0; w < nw; ++w) {
-        if (w < wid) before += sh[w];
-        all += sh[w];
+// Index of the first frame start (frames 1 .. ncuts-2) at or beyond p, or ncuts - 1.
+__device__ __forceinline__ long frame_from(const Tables &T, long p) {
+    long lo = 1, hi = T.ncuts - 1;
+    while (lo < hi) {
+        const long mid = (lo + hi) / 2;
+        if (T.cuts[mid] >= p) hi = mid;
+        else lo = mid + 1;
     }
-    __syncthreads();
-    *total = all;
-    return lane == 0 ? before : before + below;
+    return lo;
+}
+__device__ __forceinline__ double transfer_at(const Tables &T, long p) {  // of the frame that starts at p, else 1
+    const long q = frame_from(T, p);
+    return q < T.ncuts - 1 && T.cuts[q] == p ? T.transfer[q - 1] : 1.0;
 }
 
-__device__ __forceinline__ double block_total(double v, double *sh) {
-    v = warp_sum(v);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sh[w];
-    __syncthreads();
-    return t;
+// x -> m x + s composed along the lanes: lane l receives the map of lanes 0..l in order
+// (UP), or of lanes 31..l (down).
+template <bool UP>
+__device__ __forceinline__ void scan_maps(double &m, double &s, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double m2 = UP ? __shfl_up_sync(FULL, m, o) : __shfl_down_sync(FULL, m, o);
+        const double s2 = UP ? __shfl_up_sync(FULL, s, o) : __shfl_down_sync(FULL, s, o);
+        if (UP ? lane >= o : lane + o < 32) {
+            s = fma(s2, m, s);
+            m *= m2;
+        }
+    }
+}
+template <bool UP>
+__device__ __forceinline__ double scan_sums(double s, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double s2 = UP ? __shfl_up_sync(FULL, s, o) : __shfl_down_sync(FULL, s, o);
+        if (UP ? lane >= o : lane + o < 32) s += s2;
+    }
+    return s;
 }
 
-// Both scans of one row; y (i_cut + 1 values) receives the result.
-__device__ void row_scan(const Tables &T, const Dens &rho, double *y, double *sh) {
-    const long n = T.n, ic = T.i_cut;
-    const int t = threadIdx.x;
-    double *carry = sh + 32;
-    // ---- inward, frames from the top; intervals j in [cuts[b], min(cuts[b+1]-1, n-2)]
-    if (t == 0) *carry = 0.0;
-    if (ic == n - 1 && t == 0) y[n - 1] = 0.0;
-    __syncthreads();
-    for (long b = T.ncuts - 2; b >= 0; --b) {
-        const long lo = T.cuts[b];
-        const long hi = T.cuts[b + 1] - 1 < n - 2 ? T.cuts[b + 1] - 1 : n - 2;  // top interval of the frame
-        if (b < T.ncuts - 2) {
-            if (t == 0) *carry *= T.transfer[b];
-            __syncthreads();
-        }
-        for (long top = hi; top >= lo; top -= TILE) {
-            // thread t handles intervals top - ITEMS*t - s, s = 0..ITEMS-1 (descending)
-            double term[ITEMS];
-            double local = 0.0;
+// What the recurrences need of the points base + 32 c + lane of a tile (zeros outside the
+// row).  EDGE: the tile may reach beyond the row or hold its first point.
+template <bool EDGE, class Dens>
+__device__ __forceinline__ void tile_points(const Tables &T, const Dens &rho, long base, int lane, double (&a)[CH],
+                                            double (&b)[CH], double (&hl)[CH], double (&hr)[CH], double (&inv)[CH],
+                                            double (&rk)[CH]) {
+    const long p0 = base + lane;
+    const Dens d = rho.from(p0);
+    const double *r = T.r + p0, *pi = T.inverse + p0, *pk = T.rk + p0;
 #pragma unroll
-            for (int s = 0; s < ITEMS; ++s) {
-                const long j = top - (long)ITEMS * t - s;
-                term[s] = 0.0;
-                if (j >= lo) {
-                    const double bj = rho(j) * T.inverse[j];
-                    double bn = rho(j + 1) * T.inverse[j + 1];
-                    if (j + 1 == T.cuts[b + 1] && b < T.ncuts - 2) bn *= T.transfer[b];
-                    term[s] = .5 * (bj + bn) * (T.r[j + 1] - T.r[j]);
-                }
-                local += term[s];
-            }
-            double tile;
-            const double above = block_scan_excl(local, sh, &tile);  // intervals above this thread's
-            const double c0 = *carry;
-            double run = c0 + above;
-#pragma unroll
-            for (int s = 0; s < ITEMS; ++s) {
-                const long j = top - (long)ITEMS * t - s;
-                run += term[s];
-                if (j >= lo && j <= ic) y[j] = run;
-            }
-            __syncthreads();
-            if (t == 0) *carry = c0 + tile;
-            __syncthreads();
+    for (int c = 0; c < CH; ++c) {
+        if (EDGE && p0 + 32 * c >= T.n) {
+            a[c] = b[c] = hl[c] = hr[c] = inv[c] = rk[c] = 0.0;
+            continue;
         }
+        const double x = __ldg(r + 32 * c), v = d(32 * c);
+        inv[c] = __ldg(pi + 32 * c);
+        rk[c] = __ldg(pk + 32 * c);
+        hl[c] = EDGE && p0 + 32 * c == 0 ? 0.0 : .5 * (x - __ldg(r + 32 * c - 1));
+        hr[c] = EDGE && p0 + 32 * c + 1 >= T.n ? 0.0 : .5 * (__ldg(r + 32 * c + 1) - x);
+        b[c] = v * inv[c];
+        a[c] = v * rk[c];
     }
-    __syncthreads();
-    // ---- outward, frames from the bottom; points i in [max(1, cuts[b]), min(cuts[b+1], ic+1))
-    if (t == 0) {
-        *carry = 0.0;
-        y[0] *= T.rk[0];
-    }
-    __syncthreads();
-    for (long b = 0; b < T.ncuts - 1; ++b) {
-        if (T.cuts[b] > ic) break;
-        if (b) {
-            if (t == 0) *carry *= T.transfer[b - 1];
-            __syncthreads();
-        }
-        const long lo = T.cuts[b] > 1 ? T.cuts[b] : 1;
-        const long hi = T.cuts[b + 1] < ic + 1 ? T.cuts[b + 1] : ic + 1;
-        for (long base = lo; base < hi; base += TILE) {
-            double term[ITEMS];
-            double local = 0.0;
+}
+
+// A tile's sums A and B, without its carries.
+template <bool EDGE, class Dens>
+__device__ __forceinline__ void tile_sums(const Tables &T, const Dens &rho, long base, bool cut, int lane, double &si,
+                                          double &so) {
+    double a[CH], b[CH], hl[CH], hr[CH], inv[CH], rk[CH];
+    tile_points<EDGE>(T, rho, base, lane, a, b, hl, hr, inv, rk);
+    si = so = 0.0;
+    if (!EDGE || !cut) {
 #pragma unroll
-            for (int s = 0; s < ITEMS; ++s) {
-                const long i = base + (long)ITEMS * t + s;
-                term[s] = 0.0;
-                if (i < hi) {
-                    const double ai = rho(i) * T.rk[i];
-                    double ap = rho(i - 1) * T.rk[i - 1];
-                    if (i == T.cuts[b] && b > 0) ap *= T.transfer[b - 1];
-                    term[s] = .5 * (ai + ap) * (T.r[i] - T.r[i - 1]);
-                }
-                local += term[s];
-            }
-            double tile;
-            const double below = block_scan_excl(local, sh, &tile);  // points below this thread's
-            const double c0 = *carry;
-            double run = c0 + below;
-#pragma unroll
-            for (int s = 0; s < ITEMS; ++s) {
-                const long i = base + (long)ITEMS * t + s;
-                run += term[s];
-                if (i < hi) y[i] = run * T.inverse[i] + T.rk[i] * y[i];
-            }
-            __syncthreads();
-            if (t == 0) *carry = c0 + tile;
-            __syncthreads();
+        for (int c = 0; c < CH; ++c) {
+            const double w = hl[c] + hr[c];
+            si = fma(b[c], w, si);
+            so = fma(a[c], w, so);
         }
+        si = warp_sum(si);
+        so = warp_sum(so);
+        return;
     }
-    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < CH; ++k) {
+        double bk = 0.0, ak = 0.0;  // chunk CH-1-k from the top, chunk k from the bottom
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            if (c == CH - 1 - k) bk = b[c] * (hl[c] + hr[c]);
+            if (c == k) ak = a[c] * (hl[c] + hr[c]);
+        }
+        double mi = transfer_at(T, base + 32 * (CH - 1 - k) + lane + 1), mo = transfer_at(T, base + 32 * k + lane);
+        scan_maps<false>(mi, bk, lane);
+        si = __shfl_sync(FULL, fma(mi, si, bk), 0);
+        scan_maps<true>(mo, ak, lane);
+        so = __shfl_sync(FULL, fma(mo, so, ak), 31);
+    }
+}
+
+// y at a tile's points from its carries A (at base + TILE) and B (at base - 1).
+template <bool EDGE, class Dens>
+__device__ __forceinline__ void tile_y(const Tables &T, const Dens &rho, long base, bool cut, int lane, double A,
+                                       double B, double (&y)[CH]) {
+    double a[CH], b[CH], hl[CH], hr[CH], inv[CH], rk[CH];
+    tile_points<EDGE>(T, rho, base, lane, a, b, hl, hr, inv, rk);
+#pragma unroll
+    for (int c = CH - 1; c >= 0; --c) {
+        double s = b[c] * (hl[c] + hr[c]), t = 1.0;
+        if (EDGE && cut) {
+            t = transfer_at(T, base + 32 * c + lane + 1);
+            double m = t;
+            scan_maps<false>(m, s, lane);
+            s = fma(m, A, s);
+        } else {
+            s = A + scan_sums<false>(s, lane);
+        }
+        double above = __shfl_down_sync(FULL, s, 1);
+        if (lane == 31) above = A;
+        A = __shfl_sync(FULL, s, 0);
+        y[c] = rk[c] * fma(hr[c], b[c], t * above);
+    }
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+        double s = a[c] * (hl[c] + hr[c]), t = 1.0;
+        if (EDGE && cut) {
+            t = transfer_at(T, base + 32 * c + lane);
+            double m = t;
+            scan_maps<true>(m, s, lane);
+            s = fma(m, B, s);
+        } else {
+            s = B + scan_sums<true>(s, lane);
+        }
+        double below = __shfl_up_sync(FULL, s, 1);
+        if (lane == 0) below = B;
+        B = __shfl_sync(FULL, s, 31);
+        if (!EDGE || base + 32 * c + lane) y[c] = fma(inv[c], fma(hl[c], a[c], t * below), y[c]);
+    }
+}
+
+// Exclusive carries of the tiles' maps x -> m x + s in order of the scan: s[c] is replaced by
+// the value that tile c starts from.  One warp; tiles with a frame start have their
+// multiplier looked up.
+template <bool UP>
+__device__ void carry_scan(const Tables &T, double *sums, int ntiles, int lane) {
+    double carry = 0.0;
+    for (int k = 0; k < ntiles; k += 32) {
+        const int i = UP ? k + lane : ntiles - 1 - k - (31 - lane);
+        double m = 1.0, s = 0.0;
+        if (i >= 0 && i < ntiles) {
+            s = sums[i];
+            // outward: frame starts in [base, base + TILE); inward: in (base, base + TILE]
+            const long first = (long)i * TILE + (UP ? 0 : 1);
+            for (long q = frame_from(T, first); q < T.ncuts - 1 && T.cuts[q] < first + TILE; ++q) m *= T.transfer[q - 1];
+        }
+        scan_maps<UP>(m, s, lane);
+        const double after = fma(m, carry, s);  // the value behind this lane's tile
+        double before = UP ? __shfl_up_sync(FULL, after, 1) : __shfl_down_sync(FULL, after, 1);
+        if (lane == (UP ? 0 : 31)) before = carry;
+        if (i >= 0 && i < ntiles) sums[i] = before;
+        carry = __shfl_sync(FULL, after, UP ? 31 : 0);
+    }
 }
 
 struct BatchArgs {
@@ -184,39 +242,95 @@ struct BatchArgs {
     const double *r, *RK, *inverse, *transfers;
     const long *cuts;
     long n, ncuts, ntr, i_cut;
-    double *val;        // consumer dots
-    double *y, *work;   // y rows (ld y_ld) when W is null, else work rows (one per CTA)
+    double *val;  // consumer dots
+    double *y;    // y rows (ld y_ld) when W is null
     long y_ld;
 };
 
-__global__ void __launch_bounds__(THREADS) grid_rows_kernel(BatchArgs a) {
-    __shared__ double sh[40];
+template <bool DOTS>
+__global__ void __launch_bounds__(THREADS, 3) grid_rows_kernel(const __grid_constant__ BatchArgs a, double *scratch) {
+    extern __shared__ double tiles_sh[];
+    __shared__ double dots_sh[WARPS * FUSED];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ntiles = (int)((a.n + TILE - 1) / TILE), live = (int)(a.i_cut / TILE) + 1;  // tiles with an output
+    double *in = scratch ? scratch + 2L * ntiles * blockIdx.x : tiles_sh, *out = in + ntiles;
     for (long m = blockIdx.x; m < a.nrows; m += gridDim.x) {
         if (a.rows_ok && !a.rows_ok[m]) continue;
-        const bool dots = a.W != nullptr;
-        if (dots && a.cons_ptr[m] == a.cons_ptr[m + 1]) continue;
+        const long s0 = DOTS ? a.cons_ptr[m] : 0, s1 = DOTS ? a.cons_ptr[m + 1] : 1;
+        if (s0 == s1) continue;
         const long k = a.rows_k[m];
-        Tables T{a.r, a.RK + k * a.n, a.inverse + k * a.n, a.cuts, a.ncuts, a.transfers + k * a.ntr, a.n, a.i_cut};
-        Dens d{nullptr, nullptr, nullptr, nullptr, nullptr};
-        if (a.rho) {
-            d.rho = a.rho + m * a.rho_ld;
-        } else {
-            d.Pa = a.PA + a.rows_a[m] * a.ld;
-            d.Qa = a.QA + a.rows_a[m] * a.ld;
-            d.Pb = a.PB + a.rows_b[m] * a.ld;
-            d.Qb = a.QB + a.rows_b[m] * a.ld;
-        }
-        double *y = dots ? a.work + (long)blockIdx.x * a.n : a.y + m * a.y_ld;
-        row_scan(T, d, y, sh);
-        if (!dots) continue;
-        for (long s = a.cons_ptr[m]; s < a.cons_ptr[m + 1]; ++s) {
-            const double *w = a.W + a.cons_rho[s] * a.w_ld;
-            double part = 0.0;
-            for (long i = threadIdx.x; i <= a.i_cut; i += blockDim.x) part = fma(w[i], y[i], part);
-            const double tot = block_total(part, sh);
-            if (threadIdx.x == 0) a.val[s] = tot;
+        const Tables T{a.r, a.RK + k * a.n, a.inverse + k * a.n, a.cuts, a.ncuts, a.transfers + k * a.ntr, a.n, a.i_cut};
+        const auto rho = [&] {
+            if constexpr (DOTS) {
+                const long x = a.rows_a[m] * a.ld, z = a.rows_b[m] * a.ld;
+                return DensPair{a.PA + x, a.QA + x, a.PB + z, a.QB + z};
+            } else {
+                return DensRow{a.rho + m * a.rho_ld};
+            }
+        }();
+        // a tile at the row's ends or with a frame start in [base, base + TILE] takes the general form
+        auto has_cut = [&](long base) {
+            const long q = frame_from(T, base);
+            return q < T.ncuts - 1 && T.cuts[q] <= base + TILE;
+        };
+        // ---- the tiles' sums
+        for (int c = warp; c < ntiles; c += WARPS) {
+            const long base = (long)c * TILE;
+            const bool cut = has_cut(base);
+            double si, so;
+            if (cut || base == 0 || base + TILE >= T.n) tile_sums<true>(T, rho, base, cut, lane, si, so);
+            else tile_sums<false>(T, rho, base, false, lane, si, so);
+            if (lane == 0) {
+                in[c] = si;
+                out[c] = so;
+            }
         }
         __syncthreads();
+        if (warp == 0) carry_scan<false>(T, in, ntiles, lane);
+        if (warp == 1) carry_scan<true>(T, out, ntiles, lane);
+        __syncthreads();
+        // ---- y, and its dots with FUSED consumers at a time
+        for (long s = s0; s < s1; s += FUSED) {
+            const double *w[FUSED];
+            double part[FUSED];
+            if (DOTS)
+#pragma unroll
+                for (int q = 0; q < FUSED; ++q) {
+                    w[q] = a.W + a.cons_rho[s + q < s1 ? s + q : s] * a.w_ld + lane;
+                    part[q] = 0.0;
+                }
+            for (int c = warp; c < live; c += WARPS) {
+                const long base = (long)c * TILE;
+                const bool cut = has_cut(base);
+                double y[CH];
+                if (cut || base == 0 || base + TILE >= T.n) tile_y<true>(T, rho, base, cut, lane, in[c], out[c], y);
+                else tile_y<false>(T, rho, base, false, lane, in[c], out[c], y);
+                const bool whole = base + TILE <= a.i_cut + 1;
+#pragma unroll
+                for (int j = 0; j < CH; ++j) {
+                    if (!whole && base + 32 * j + lane > a.i_cut) continue;
+                    if (!DOTS) a.y[m * a.y_ld + base + 32 * j + lane] = y[j];
+                    else
+#pragma unroll
+                        for (int q = 0; q < FUSED; ++q)
+                            if (q == 0 || s + q < s1) part[q] = fma(__ldg(w[q] + base + 32 * j), y[j], part[q]);
+                }
+            }
+            if (!DOTS) break;
+#pragma unroll
+            for (int q = 0; q < FUSED; ++q) {
+                part[q] = warp_sum(part[q]);
+                if (lane == 0) dots_sh[warp * FUSED + q] = part[q];
+            }
+            __syncthreads();
+            if (threadIdx.x < FUSED && s + threadIdx.x < s1) {
+                double v = 0.0;
+                for (int x = 0; x < WARPS; ++x) v += dots_sh[x * FUSED + threadIdx.x];
+                a.val[s + threadIdx.x] = v;
+            }
+            __syncthreads();
+        }
+        __syncthreads();  // the carries are overwritten by the next row
     }
 }
 
@@ -232,6 +346,22 @@ static int grid_common_checks(long n, long ncuts, long ntr, long i_cut) {
     return RKB_OK;
 }
 
+template <bool DOTS>
+static int launch_rows(const grid::BatchArgs &a, cudaStream_t st) {
+    auto kern = grid::grid_rows_kernel<DOTS>;
+    const long ctas = a.nrows < 8L * sm_count() ? a.nrows : 8L * sm_count();
+    const size_t bytes = sizeof(double) * 2 * (size_t)ceil_div(a.n, grid::TILE);  // the tiles' sums and carries
+    double *scratch = nullptr;
+    const bool fits = bytes <= 200 * 1024;  // above 3.2 million points they go to device memory
+    if (fits) RKB_CUDA(set_smem(kern, (int)bytes));
+    else RKB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&scratch), bytes * ctas, st));
+    kern<<<(unsigned)ctas, grid::THREADS, fits ? bytes : 0, st>>>(a, scratch);
+    const cudaError_t e = cudaGetLastError();
+    if (scratch) cudaFreeAsync(scratch, st);
+    if (e != cudaSuccess) return cuda_status(e, "grid_rows_kernel");
+    return RKB_OK;
+}
+
 extern "C" int rkb_grid_yk_rows(const double *d_rho, long rho_ld, const long *d_rows_k, long nrows,
                                 const double *d_r, long n, const double *d_RK, const double *d_inverse,
                                 const long *d_cuts, long ncuts, const double *d_transfers, long ntr, long i_cut,
@@ -244,10 +374,7 @@ extern "C" int rkb_grid_yk_rows(const double *d_rho, long rho_ld, const long *d_
     a.rho = d_rho; a.rho_ld = rho_ld; a.rows_k = d_rows_k; a.nrows = nrows;
     a.r = d_r; a.RK = d_RK; a.inverse = d_inverse; a.transfers = d_transfers; a.cuts = d_cuts;
     a.n = n; a.ncuts = ncuts; a.ntr = ntr; a.i_cut = i_cut; a.y = d_y; a.y_ld = y_ld;
-    const long grid_n = nrows < 8L * sm_count() ? nrows : 8L * sm_count();
-    grid::grid_rows_kernel<<<(unsigned)grid_n, grid::THREADS, 0, as_stream(stream)>>>(a);
-    RKB_LAUNCHED("grid_rows_kernel");
-    return RKB_OK;
+    return launch_rows<false>(a, as_stream(stream));
 }
 
 extern "C" int rkb_grid_pair_dot_batch(const double *d_PA, const double *d_QA, const double *d_PB,
@@ -268,9 +395,6 @@ extern "C" int rkb_grid_pair_dot_batch(const double *d_PA, const double *d_QA, c
     a.rows_k = d_rows_k; a.rows_ok = d_rows_ok; a.nrows = nrows; a.W = d_W; a.w_ld = w_ld;
     a.cons_ptr = d_cons_ptr; a.cons_rho = d_cons_rho; a.r = d_r; a.RK = d_RK; a.inverse = d_inverse;
     a.transfers = d_transfers; a.cuts = d_cuts; a.n = n; a.ncuts = ncuts; a.ntr = ntr; a.i_cut = i_cut;
-    a.val = d_val; a.work = d_work;
-    const long grid_n = nrows < work_rows ? nrows : work_rows;
-    grid::grid_rows_kernel<<<(unsigned)grid_n, grid::THREADS, 0, as_stream(stream)>>>(a);
-    RKB_LAUNCHED("grid_rows_kernel");
-    return RKB_OK;
+    a.val = d_val;
+    return launch_rows<true>(a, as_stream(stream));
 }

@@ -186,15 +186,13 @@ def yk_pair_dot_batch_on_grid(PA, QA, PB, QB, rows_a, rows_b, rows_k, rows_ok, R
     ok = torch.as_tensor(np.asarray(rows_ok.cpu() if is_device_tensor(rows_ok) else rows_ok, dtype=np.uint8),
                          device=dev)
     nrows = int(rows_k_h.shape[0])
-    work_rows = min(nrows, 8 * torch.cuda.get_device_properties(dev).multi_processor_count)
-    work = torch.empty((work_rows, n), dtype=torch.float64, device=dev)
     _native.check(L.rkb_grid_pair_dot_batch(mats[0].data_ptr(), mats[1].data_ptr(), mats[2].data_ptr(),
                                             mats[3].data_ptr(), ld, idx[0].data_ptr(), idx[1].data_ptr(),
                                             idx[2].data_ptr(), ok.data_ptr(), nrows, W.data_ptr(), W.shape[1],
                                             idx[3].data_ptr(), idx[4].data_ptr(), tab.r.data_ptr(), n,
                                             tab.RK.data_ptr(), tab.inverse.data_ptr(), tab.cuts.data_ptr(),
                                             tab.ncuts, tab.transfers.data_ptr(), tab.ntr, ic, val.data_ptr(),
-                                            work.data_ptr(), work_rows, _native.stream_handle()),
+                                            val.data_ptr(), 1, _native.stream_handle()),
                   "rkb_grid_pair_dot_batch")
     return val if on_dev else val.cpu().numpy()
 

@@ -117,7 +117,7 @@ int rkb_slater_direct(const double *d_rho13, const double *d_rho24, const double
  * 0..i_cut and, for each consumer slot s in [d_cons_ptr[m], d_cons_ptr[m+1]),
  * writes d_val[s] = sum_i W[d_cons_rho[s]][i] Y_i (W rows of stride w_ld).
  * Rows with d_rows_ok[m] == 0 leave their slots untouched (zero them first).
- * d_work: work_rows x n doubles of scratch (one row per concurrent CTA).
+ * d_work (not null) and work_rows (>= 1) are not used: y is not stored.
  * ------------------------------------------------------------------------- */
 int rkb_grid_yk_rows(const double *d_rho, long rho_ld, const long *d_rows_k, long nrows,
                      const double *d_r, long n, const double *d_RK, const double *d_inverse,
