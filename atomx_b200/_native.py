@@ -25,6 +25,8 @@ _SIGNATURES = {
     "rkb_device_supported": [],
     "rkb_yk_flat": [_vp, _vp, _vp, _l, _i, _i, _i, _vp, _vp, _vp, _vp],
     "rkb_yk_rows": [_vp, _l, _vp, _l, _vp, _vp, _i, _i, _vp, _vp, _vp, _l, _vp],
+    "rkb_yk_rows_pow": [_vp, _l, _vp, _l, _vp, _vp, _i, _i, _vp, _vp, _vp, _l, _vp, _i, _vp],
+    "rkb_table_rows_fp64_pow": [_vp, _vp, _l, _vp, _vp, _vp, _l, _vp, _vp, _i, _i, _vp, _vp, _vp, _vp, _l, _vp, _i, _vp],
     "rkb_eval_orbitals": [_vp, _l, _l, _vp, _i, _i, _i, _i, _vp, _l, _vp],
     "rkb_pair_density": [_vp, _vp, _l, _vp, _l, _l, _vp, _l, _vp],
     "rkb_pack_upper": [_vp, _l, _vp, _vp],

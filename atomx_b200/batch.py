@@ -35,6 +35,7 @@ from . import _native
 from .split import (CB_STRIDE, CERT_LIMIT, IonRows, _round_up, certify, check_kdim, choose_width, join_stream,
                     read_status)
 from .split_plan import crt_constants
+from .yk import power_workspace
 from .tables import TILE, Fp64Recompute, IonDevice, RkTables, tile_tasks
 
 __all__ = ["SplitBatch", "Fp64Batch", "Workspace", "batch_tasks"]
@@ -361,6 +362,11 @@ class Fp64Batch(_Graphable):
         nrows = int(self.row_base[-1])
         self.g = _alloc(workspace, (nrows, self.ld), torch.float64, d)
         self.y = _alloc(workspace, (nrows, self.ld), torch.float64, d)
+        # the ions' rows run one after another on one stream and share a power table
+        pows = [power_workspace(dv.plan.n_rows, max(dv.plan.ks), dv.n, "meta") for dv in self.devs]
+        self.pow_of = [p is not None for p in pows]
+        self.pow = (_alloc(workspace, (max(p.numel() for p in pows if p is not None),), torch.float64, d)
+                    if any(self.pow_of) else None)
         g_row0, g_n, g_kdim, self.group_of = [], [], [], []
         for i, dv in enumerate(self.devs):
             for k in dv.plan.ks:
@@ -394,12 +400,13 @@ class Fp64Batch(_Graphable):
         h = _native.stream_handle(stream)
         for i, dv in enumerate(self.devs):
             off = int(self.row_base[i]) * self.ld * 8
-            _native.check(L.rkb_table_rows_fp64(dv.Pv.data_ptr(), dv.Qv.data_ptr(), dv.n, dv.pairs.data_ptr(),
-                                                dv.row_pair.data_ptr(), dv.row_k.data_ptr(), dv.plan.n_rows,
-                                                dv.r.data_ptr(), dv.w.data_ptr(), dv.nv, dv.ng, dv.mo.data_ptr(),
-                                                dv.mi.data_ptr(), self.g.data_ptr() + off, self.y.data_ptr() + off,
-                                                self.ld, h),
-                          "rkb_table_rows_fp64")
+            _native.check(L.rkb_table_rows_fp64_pow(dv.Pv.data_ptr(), dv.Qv.data_ptr(), dv.n, dv.pairs.data_ptr(),
+                                                    dv.row_pair.data_ptr(), dv.row_k.data_ptr(), dv.plan.n_rows,
+                                                    dv.r.data_ptr(), dv.w.data_ptr(), dv.nv, dv.ng,
+                                                    dv.mo.data_ptr(), dv.mi.data_ptr(), self.g.data_ptr() + off,
+                                                    self.y.data_ptr() + off, self.ld,
+                                                    self.pow.data_ptr() if self.pow_of[i] else 0, max(dv.plan.ks), h),
+                          "rkb_table_rows_fp64_pow")
         _native.check(L.rkb_table_contract_fp64_groups(self.g.data_ptr(), self.y.data_ptr(), self.ld, self.max_kdim,
                                                        self.grp_kdim.data_ptr(), self.grp_row0.data_ptr(),
                                                        self.grp_n.data_ptr(), self.grp_out.data_ptr(),

@@ -74,6 +74,7 @@ int sm_count() {
 struct RhoRows {
     const double *rho;
     long ld;
+    static constexpr int BLOCKS = 7;  // of yk_rows_kernel per SM: more rows in flight, or more registers
     struct Row {
         const double *__restrict__ rho;
         __device__ __forceinline__ double at(long i) const { return __ldg(rho + i); }
@@ -84,6 +85,7 @@ struct RhoPairs {
     const double *P, *Q;
     long orb_ld;
     const long *pairs, *row_pair;
+    static constexpr int BLOCKS = 5;
     struct Row {
         const double *__restrict__ pa, *__restrict__ pc, *__restrict__ qa, *__restrict__ qc;
         // rho = P_a P_c + Q_a Q_c (atomx slater_yk.py:193), each product rounded
@@ -98,6 +100,29 @@ struct RhoPairs {
     }
 };
 
+// Powers of the row's multipole: r^k and r^-(k+1) at node i, evaluated, or read from a
+// table of the same values (pow_table_kernel).
+struct PowEval {
+    const double *__restrict__ r;
+    int k;
+    __device__ __forceinline__ double up(long i) const { return int_pow(__ldg(r + i), k); }
+    __device__ __forceinline__ double down(long i) const { return int_pow(__ldg(r + i), -(k + 1)); }
+};
+struct PowRead {
+    const double *__restrict__ u, *__restrict__ d;
+    __device__ __forceinline__ double up(long i) const { return __ldg(u + i); }
+    __device__ __forceinline__ double down(long i) const { return __ldg(d + i); }
+};
+
+// tab[k][0][i] = r_i^k, tab[k][1][i] = r_i^-(k+1)
+__global__ void pow_table_kernel(const double *__restrict__ r, long n, double *__restrict__ tab) {
+    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const PowEval p{r, (int)blockIdx.y};
+    tab[(2L * blockIdx.y) * n + i] = p.up(i);
+    tab[(2L * blockIdx.y + 1) * n + i] = p.down(i);
+}
+
 // One warp per row; NG is the compile-time node count (0 = runtime ng <= RKB_MAX_NG).
 // `gout` (optional) receives g = w*rho for the row (table engine), and columns
 // n..ld-1 of both outputs are zero-filled.
@@ -111,24 +136,22 @@ struct RhoPairs {
 // owning one cell.  I_out waits in the output row between the passes.  Every
 // product and sum is the one the cell-per-lane form evaluates, in the same
 // order, so the rows are bit-identical to it.
-template <int NG, class Src>
-__global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__restrict__ row_k, int k_all, long nrows,
-                                                      const double *__restrict__ r, const double *__restrict__ w,
-                                                      int nv, int ng_rt, const double *__restrict__ mo,
-                                                      const double *__restrict__ mi, double *__restrict__ yk,
-                                                      long yk_ld, double *__restrict__ gout) {
+//
+// Bound by FP64 and instruction issue: ng multiply-adds a node and pass, separately
+// rounded, and the element-wise work.  Evaluating the powers per row and node (three
+// int_pow and a division) was more than half of that: 20 000 rows of 896 nodes with mixed
+// multipoles took 327 us, and 240 us with the powers read from a table that one small
+// launch fills; Z=70 table rows 816 and 755 us.  With the partial matrices in shared
+// memory (they were 2 ng^2 uniform global loads a chunk) 217 and 614 us.
+template <int NG, class Src, class Pow>
+__device__ __forceinline__ void yk_row(const Src &src, const Pow &pw, long q, const double *__restrict__ w, int nv,
+                                       int ng_rt, const double *__restrict__ mo, const double *__restrict__ mi, int ms,
+                                       double *__restrict__ yk, long yk_ld, double *__restrict__ gout, double *cbuf) {
     constexpr int NGMAX = NG > 0 ? NG : RKB_MAX_NG;
-    constexpr int GSMAX = NGMAX | 1;
     const int ng = NG > 0 ? NG : ng_rt;
     const int gs = NG > 0 ? (NG | 1) : (ng_rt | 1);
-    extern __shared__ double smem_chunk[];
     const int lane = threadIdx.x & 31;
-    const int wib = threadIdx.x >> 5;
     const long n = (long)nv * ng;
-    double *cbuf = smem_chunk + (long)wib * (32 * GSMAX);  // [32][gs]: one chunk's per-node terms
-    const long q = (long)blockIdx.x * (blockDim.x >> 5) + wib;
-    if (q >= nrows) return;
-    const int k = row_k ? row_k[q] : k_all;
     const int nchunks = (nv + 31) >> 5;
     const auto sr = src.row(q);  // the row's source pointers, resolved once
     double *yrow = yk + q * yk_ld;
@@ -146,7 +169,7 @@ __global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__rest
             const double g = __dmul_rn(__ldg(w + i), sr.at(i));
             if (grow_) grow_[i] = g;
             const int cl = (int)(t / ng), node = (int)(t - (long)cl * ng);
-            cbuf[cl * gs + node] = __dmul_rn(g, int_pow(__ldg(r + i), k));
+            cbuf[cl * gs + node] = __dmul_rn(g, pw.up(i));
         }
         __syncwarp();
         const int m = m0 + lane;
@@ -173,7 +196,7 @@ __global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__rest
                     double s = base;
 #pragma unroll
                     for (int j = 0; j < NGMAX; ++j)
-                        if (j < ng) s = __dadd_rn(s, __dmul_rn(h[j], __ldg(&mo[i * ng + j])));
+                        if (j < ng) s = __dadd_rn(s, __dmul_rn(h[j], mo[i * ms + j]));
                     cbuf[lane * gs + i] = s;  // own slots only: h is in registers
                 }
             }
@@ -201,7 +224,7 @@ __global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__rest
             if (u < ng && t < ne) {
                 const long i = e0 + t;
                 const double g = __dmul_rn(__ldg(w + i), sr.at(i));
-                rin[u] = int_pow(__ldg(r + i), -(k + 1));
+                rin[u] = pw.down(i);
                 const int cl = (int)(t / ng), node = (int)(t - (long)cl * ng);
                 cbuf[cl * gs + node] = __dmul_rn(g, rin[u]);
             }
@@ -234,7 +257,7 @@ __global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__rest
                     double s = base;
 #pragma unroll
                     for (int j = 0; j < NGMAX; ++j)
-                        if (j < ng) s = __dadd_rn(s, __dmul_rn(e[j], __ldg(&mi[i * ng + j])));
+                        if (j < ng) s = __dadd_rn(s, __dmul_rn(e[j], mi[i * ms + j]));
                     cbuf[cl_m * gs + i] = s;
                 }
             }
@@ -247,7 +270,7 @@ __global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__rest
             if (u < ng && t < ne) {
                 const long i = e0 + t;
                 const int cl = (int)(t / ng), node = (int)(t - (long)cl * ng);
-                yrow[i] = __dadd_rn(__dmul_rn(rin[u], yrow[i]), __dmul_rn(int_pow(__ldg(r + i), k), cbuf[cl * gs + node]));
+                yrow[i] = __dadd_rn(__dmul_rn(rin[u], yrow[i]), __dmul_rn(pw.up(i), cbuf[cl * gs + node]));
             }
         }
         __syncwarp();  // cbuf is rewritten by the next chunk
@@ -259,36 +282,192 @@ __global__ void __launch_bounds__(128) yk_rows_kernel(Src src, const int *__rest
     }
 }
 
+template <int NG, class Src, bool TAB>
+__global__ void __launch_bounds__(128, NG > 0 ? Src::BLOCKS : 1) yk_rows_kernel(Src src, const int *__restrict__ row_k, int k_all, long nrows,
+                                                      const double *__restrict__ r, const double *__restrict__ w,
+                                                      int nv, int ng, const double *__restrict__ mo,
+                                                      const double *__restrict__ mi, double *__restrict__ yk,
+                                                      long yk_ld, double *__restrict__ gout,
+                                                      const double *__restrict__ tab, int tab_k) {
+    constexpr int GSMAX = (NG > 0 ? NG : RKB_MAX_NG) | 1;
+    extern __shared__ double smem_chunk[];
+    // the partial matrices in shared memory, rows of an even length (two entries a load)
+    constexpr int MS = (NG + 1) & ~1;
+    __shared__ __align__(16) double part[NG > 0 ? 2 * NG * MS : 1];
+    if (NG > 0) {
+        for (int i = threadIdx.x; i < NG * NG; i += blockDim.x) {
+            part[i / NG * MS + i % NG] = mo[i];
+            part[NG * MS + i / NG * MS + i % NG] = mi[i];
+        }
+        __syncthreads();
+    }
+    const double *pmo = NG > 0 ? part : mo, *pmi = NG > 0 ? part + NG * MS : mi;
+    const int ms = NG > 0 ? MS : ng;
+    double *cbuf = smem_chunk + (long)(threadIdx.x >> 5) * (32 * GSMAX);  // [32][gs]: one chunk's per-node terms
+    const long q = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (q >= nrows) return;
+    const int k = row_k ? row_k[q] : k_all;
+    if (TAB && k >= 0 && k <= tab_k) {
+        const long n = (long)nv * (NG > 0 ? NG : ng);
+        yk_row<NG>(src, PowRead{tab + 2 * k * n, tab + (2 * k + 1) * n}, q, w, nv, ng, pmo, pmi, ms, yk, yk_ld, gout, cbuf);
+    } else {
+        yk_row<NG>(src, PowEval{r, k}, q, w, nv, ng, pmo, pmi, ms, yk, yk_ld, gout, cbuf);
+    }
+}
+
+// The same for few rows: a block per row and a warp per chunk of 32 cells.  Every chunk
+// is summed at once, the carries follow from the chunk totals in yk_row's order (so the
+// rows are the same to the bit), and both passes go on together.  Latency-bound: the
+// warp-per-row kernel walks 2 x nchunks chunks one after another (a single row of 238
+// nodes 18.5 us from cold caches, 14.9 us here).
+template <int NG, class Src>
+__global__ void __launch_bounds__(512) yk_row_block_kernel(Src src, const int *__restrict__ row_k, int k_all,
+                                                           const double *__restrict__ r, const double *__restrict__ w,
+                                                           int nv, const double *__restrict__ mo,
+                                                           const double *__restrict__ mi, double *__restrict__ yk,
+                                                           long yk_ld, double *__restrict__ gout) {
+    constexpr int GS = NG | 1;
+    extern __shared__ double smem_chunk[];
+    __shared__ double total[2][16];
+    const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
+    double *cbuf = smem_chunk + (long)c * (32 * GS);
+    const long n = (long)nv * NG, q = blockIdx.x;
+    const PowEval pw{r, row_k ? row_k[q] : k_all};
+    const auto sr = src.row(q);
+    double *yrow = yk + q * yk_ld, *grow_ = gout ? gout + q * yk_ld : nullptr;
+    // outward: this warp's cells m0 .. m0 + 31; inward: mhi down to mlo
+    const int m0 = c << 5, mhi = nv - 1 - m0, mlo = max(0, mhi - 31);
+    const int ne_o = min(32, nv - m0) * NG, ne_i = (mhi - mlo + 1) * NG;
+    const long o0 = (long)m0 * NG, i0 = (long)mlo * NG;
+    double rin[NG], rk[NG], h[NG], e[NG], cell = 0.0;
+#pragma unroll
+    for (int u = 0; u < NG; ++u) {
+        const int t = lane + 32 * u;
+        if (t < ne_o) {
+            const double g = __dmul_rn(__ldg(w + o0 + t), sr.at(o0 + t));
+            if (grow_) grow_[o0 + t] = g;
+            cbuf[t / NG * GS + t % NG] = __dmul_rn(g, pw.up(o0 + t));
+        }
+    }
+    __syncwarp();
+    const bool live_o = m0 + lane < nv;
+#pragma unroll
+    for (int j = 0; j < NG; ++j) {
+        h[j] = live_o ? cbuf[lane * GS + j] : 0.0;
+        if (live_o) cell = __dadd_rn(cell, h[j]);
+    }
+    const double incl_o = warp_inclusive_scan(cell, lane);
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < NG; ++u) {
+        const int t = lane + 32 * u;
+        if (t < ne_i) {
+            const double g = __dmul_rn(__ldg(w + i0 + t), sr.at(i0 + t));
+            rk[u] = pw.up(i0 + t);
+            rin[u] = pw.down(i0 + t);
+            cbuf[t / NG * GS + t % NG] = __dmul_rn(g, rin[u]);
+        }
+    }
+    __syncwarp();
+    const int cl = mhi - lane - mlo;  // this lane's inward cell in the buffer
+    const bool live_i = cl >= 0;
+    cell = 0.0;
+#pragma unroll
+    for (int j = 0; j < NG; ++j) {
+        e[j] = live_i ? cbuf[cl * GS + j] : 0.0;
+        if (live_i) cell = __dadd_rn(cell, e[j]);
+    }
+    const double incl_i = warp_inclusive_scan(cell, lane);
+    if (lane == 31) {
+        total[0][c] = incl_o;
+        total[1][c] = incl_i;
+    }
+    __syncthreads();
+    auto base_of = [&](int pass, double incl) {
+        double carry = 0.0;
+        for (int b = 0; b < c; ++b) carry = __dadd_rn(carry, total[pass][b]);
+        const double excl = __shfl_up_sync(0xffffffffu, incl, 1);
+        return lane == 0 ? carry : __dadd_rn(carry, excl);
+    };
+    auto partial = [&](const double *M, const double (&x)[NG], double base, int i) {
+        double s = base;
+#pragma unroll
+        for (int j = 0; j < NG; ++j) s = __dadd_rn(s, __dmul_rn(x[j], __ldg(M + i * NG + j)));
+        return s;
+    };
+    const double base_o = base_of(0, incl_o), base_i = base_of(1, incl_i);
+    if (live_o)
+#pragma unroll
+        for (int i = 0; i < NG; ++i) cbuf[lane * GS + i] = partial(mo, h, base_o, i);
+    __syncwarp();
+    for (int t = lane; t < ne_o; t += 32) yrow[o0 + t] = cbuf[t / NG * GS + t % NG];  // I_out parked
+    __syncwarp();
+    if (live_i)
+#pragma unroll
+        for (int i = 0; i < NG; ++i) cbuf[cl * GS + i] = partial(mi, e, base_i, i);
+    __syncthreads();  // the whole row's I_out is in place
+#pragma unroll
+    for (int u = 0; u < NG; ++u) {
+        const int t = lane + 32 * u;
+        if (t < ne_i)
+            yrow[i0 + t] = __dadd_rn(__dmul_rn(rin[u], yrow[i0 + t]), __dmul_rn(rk[u], cbuf[t / NG * GS + t % NG]));
+    }
+    for (long i = n + threadIdx.x; i < yk_ld; i += blockDim.x) {
+        yrow[i] = 0.0;
+        if (grow_) grow_[i] = 0.0;
+    }
+}
+
+// Rows up to which a block takes a row: the warp-per-row kernel then leaves SMs idle
+// (two blocks of its four rows per SM).
+static long few_rows() { return 8L * sm_count(); }
+
 template <class Src>
 static int launch_yk(Src src, const int *d_row_k, int k_all, long nrows, const double *d_r, const double *d_w, int nv,
                      int ng, const double *d_mo, const double *d_mi, double *d_yk, long yk_ld, double *d_g,
-                     cudaStream_t st) {
-    const int warps = 4;
+                     cudaStream_t st, double *d_pow = nullptr, int pow_k = -1) {
+    const int warps = 4, chunks = (nv + 31) >> 5;
     // the kernel's GSMAX: ng | 1 for the compiled node counts below, RKB_MAX_NG | 1 otherwise
     const bool compiled = (ng >= 2 && ng <= 13) || ng == 16 || ng == 17;
     const int gsmax = compiled ? (ng | 1) : (RKB_MAX_NG | 1);
-    const size_t smem = (size_t)warps * 32 * gsmax * sizeof(double);  // one chunk buffer per warp, any grid length
-    dim3 grid((unsigned)ceil_div(nrows, warps)), block(32 * warps);
-#define RKB_YK_CASE(NGV)                                                                                  \
-    case NGV: {                                                                                           \
-        auto kern = yk_rows_kernel<NGV, Src>;                                                             \
-        RKB_CUDA(set_smem(kern, (int)smem));     \
-        kern<<<grid, block, smem, st>>>(src, d_row_k, k_all, nrows, d_r, d_w, nv, ng, d_mo, d_mi, d_yk,   \
-                                        yk_ld, d_g);                                                      \
-        break;                                                                                            \
+    const size_t chunk = (size_t)32 * gsmax * sizeof(double);  // one chunk buffer per warp, any grid length
+    const bool block = compiled && chunks <= 16 && nrows <= few_rows();
+    // A table of the powers pays for its own launch where rows outnumber multipoles.
+    const bool tab = !block && d_pow != nullptr && pow_k >= 0;
+    if (tab) {
+        const long n = (long)nv * ng;
+        pow_table_kernel<<<dim3((unsigned)ceil_div(n, 128), (unsigned)(pow_k + 1)), 128, 0, st>>>(d_r, n, d_pow);
+        RKB_LAUNCHED("pow_table_kernel");
+    }
+    dim3 grid((unsigned)ceil_div(nrows, warps));
+#define RKB_YK_LAUNCH(NGV, TABV)                                                                             \
+    {                                                                                                        \
+        auto kern = yk_rows_kernel<NGV, Src, TABV>;                                                          \
+        RKB_CUDA(set_smem(kern, (int)(warps * chunk)));                                                      \
+        kern<<<grid, 32 * warps, warps * chunk, st>>>(src, d_row_k, k_all, nrows, d_r, d_w, nv, ng, d_mo, d_mi, \
+                                                      d_yk, yk_ld, d_g, d_pow, pow_k);                       \
+    }
+#define RKB_YK_CASE(NGV)                                                                                     \
+    case NGV: {                                                                                              \
+        if (block) {                                                                                         \
+            auto kern = yk_row_block_kernel<NGV, Src>;                                                       \
+            RKB_CUDA(set_smem(kern, (int)(chunks * chunk)));                                                 \
+            kern<<<(unsigned)nrows, 32 * chunks, chunks * chunk, st>>>(src, d_row_k, k_all, d_r, d_w, nv, d_mo, \
+                                                                       d_mi, d_yk, yk_ld, d_g);              \
+        } else if (tab) RKB_YK_LAUNCH(NGV, true)                                                             \
+        else RKB_YK_LAUNCH(NGV, false)                                                                       \
+        break;                                                                                               \
     }
     switch (ng) {
         RKB_YK_CASE(2) RKB_YK_CASE(3) RKB_YK_CASE(4) RKB_YK_CASE(5) RKB_YK_CASE(6) RKB_YK_CASE(7)
         RKB_YK_CASE(8) RKB_YK_CASE(9) RKB_YK_CASE(10) RKB_YK_CASE(11) RKB_YK_CASE(12) RKB_YK_CASE(13)
         RKB_YK_CASE(16) RKB_YK_CASE(17)
-        default: {
-            auto kern = yk_rows_kernel<0, Src>;
-            RKB_CUDA(set_smem(kern, (int)smem));
-            kern<<<grid, block, smem, st>>>(src, d_row_k, k_all, nrows, d_r, d_w, nv, ng, d_mo, d_mi, d_yk, yk_ld,
-                                            d_g);
-        }
+        default:
+            if (tab) RKB_YK_LAUNCH(0, true)
+            else RKB_YK_LAUNCH(0, false)
     }
 #undef RKB_YK_CASE
+#undef RKB_YK_LAUNCH
     RKB_LAUNCHED("yk_rows_kernel");
     return RKB_OK;
 }
@@ -448,28 +627,45 @@ int rkb_yk_flat(const double *d_rho, const double *d_r, const double *d_w, long 
 int rkb_yk_rows(const double *d_rho, long rho_ld, const int *d_row_k, long nrows, const double *d_r,
                 const double *d_w, int nv, int ng, const double *d_mo, const double *d_mi, double *d_yk,
                 long yk_ld, void *stream) {
-    long n = (long)nv * ng;
-    int st = check_grid(nv, ng, n);
-    if (st) return st;
-    RKB_CHECK_ARG(nrows >= 0, "nrows must be >= 0");
-    RKB_CHECK_ARG(rho_ld >= n && yk_ld >= n, "leading dimensions must be >= nv*ng");
-    if (nrows == 0) return RKB_OK;
-    RKB_CHECK_ARG(!overlaps(d_rho, nrows, rho_ld, d_yk, nrows, yk_ld, n), "d_yk must not overlap d_rho");
-    return launch_yk(RhoRows{d_rho, rho_ld}, d_row_k, 0, nrows, d_r, d_w, nv, ng, d_mo, d_mi, d_yk, yk_ld, nullptr,
-                     as_stream(stream));
+    return rkb_yk_rows_pow(d_rho, rho_ld, d_row_k, nrows, d_r, d_w, nv, ng, d_mo, d_mi, d_yk, yk_ld, nullptr, -1,
+                           stream);
 }
 
 int rkb_table_rows_fp64(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
                         const long *d_row_pair, const int *d_row_k, long nrows, const double *d_r,
                         const double *d_w, int nv, int ng, const double *d_mo, const double *d_mi, double *d_g,
                         double *d_y, long ld, void *stream) {
+    return rkb_table_rows_fp64_pow(d_Pv, d_Qv, orb_ld, d_pairs, d_row_pair, d_row_k, nrows, d_r, d_w, nv, ng, d_mo,
+                                   d_mi, d_g, d_y, ld, nullptr, -1, stream);
+}
+
+int rkb_yk_rows_pow(const double *d_rho, long rho_ld, const int *d_row_k, long nrows, const double *d_r,
+                    const double *d_w, int nv, int ng, const double *d_mo, const double *d_mi, double *d_yk,
+                    long yk_ld, double *d_pow, int pow_k, void *stream) {
+    long n = (long)nv * ng;
+    int st = check_grid(nv, ng, n);
+    if (st) return st;
+    RKB_CHECK_ARG(nrows >= 0, "nrows must be >= 0");
+    RKB_CHECK_ARG(rho_ld >= n && yk_ld >= n, "leading dimensions must be >= nv*ng");
+    RKB_CHECK_ARG(pow_k <= 4096, "power table too long (%d)", pow_k);
+    if (nrows == 0) return RKB_OK;
+    RKB_CHECK_ARG(!overlaps(d_rho, nrows, rho_ld, d_yk, nrows, yk_ld, n), "d_yk must not overlap d_rho");
+    return launch_yk(RhoRows{d_rho, rho_ld}, d_row_k, 0, nrows, d_r, d_w, nv, ng, d_mo, d_mi, d_yk, yk_ld, nullptr,
+                     as_stream(stream), d_pow, pow_k);
+}
+
+int rkb_table_rows_fp64_pow(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
+                            const long *d_row_pair, const int *d_row_k, long nrows, const double *d_r,
+                            const double *d_w, int nv, int ng, const double *d_mo, const double *d_mi, double *d_g,
+                            double *d_y, long ld, double *d_pow, int pow_k, void *stream) {
     long n = (long)nv * ng;
     int st = check_grid(nv, ng, n);
     if (st) return st;
     RKB_CHECK_ARG(ld >= n && orb_ld >= n, "leading dimensions must be >= nv*ng");
+    RKB_CHECK_ARG(pow_k <= 4096, "power table too long (%d)", pow_k);
     if (nrows == 0) return RKB_OK;
     return launch_yk(RhoPairs{d_Pv, d_Qv, orb_ld, d_pairs, d_row_pair}, d_row_k, 0, nrows, d_r, d_w, nv, ng, d_mo,
-                     d_mi, d_y, ld, d_g, as_stream(stream));
+                     d_mi, d_y, ld, d_g, as_stream(stream), d_pow, pow_k);
 }
 
 int rkb_eval_orbitals(const double *d_coeff, long coeff_ld, long n_orb, const double *d_bsp, int nv, int ng,

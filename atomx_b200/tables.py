@@ -26,7 +26,7 @@ import torch
 from . import _native
 from .device import as_device, resident
 from .plan import TablePlan, make_plan
-from .yk import yk_partial_matrices
+from .yk import power_workspace, yk_partial_matrices
 
 __all__ = ["IonDevice", "RkTables", "RkStream", "HostTableSink", "HostPackedTables", "PackedShipper", "packed_offsets", "upload_ion", "stage_ion", "evaluate_staged", "upload_values", "slater_rk_tables",
            "slater_rk_tables_from_values", "tables_for", "stream_tables", "iter_blocks", "tile_tasks", "TILE",
@@ -377,6 +377,8 @@ class Fp64Workspace:
         self.ld = _round_up(dev.n, 32)
         self.g = torch.empty((plan.n_rows, self.ld), device=dev.Pv.device, dtype=torch.float64)
         self.y = torch.empty_like(self.g)
+        self.kmax = max(plan.ks)
+        self.pow = power_workspace(plan.n_rows, self.kmax, dev.n, dev.Pv.device)
         sizes = [plan.n_of_k(k) for k in plan.ks]
         self.row0 = torch.as_tensor(np.array([plan.k_row_offset[k] for k in plan.ks], dtype=np.int64),
                                     device=self.g.device)
@@ -392,16 +394,21 @@ class Fp64Workspace:
         self.task_range = [(int(bounds[i]), int(bounds[i + 1])) for i in range(len(sizes))]
 
 
+def _fp64_rows(dev: IonDevice, ws: Fp64Workspace, h: int) -> None:
+    """The plain engine's g and Y^k rows of the whole plan (K2) on stream handle ``h``."""
+    _native.check(_native.load().rkb_table_rows_fp64_pow(
+        dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(), dev.row_pair.data_ptr(),
+        dev.row_k.data_ptr(), dev.plan.n_rows, dev.r.data_ptr(), dev.w.data_ptr(), dev.nv, dev.ng, dev.mo.data_ptr(),
+        dev.mi.data_ptr(), ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, _native.ptr(ws.pow), ws.kmax, h),
+        "rkb_table_rows_fp64_pow")
+
+
 def run_fp64(dev: IonDevice, ws: Fp64Workspace, out: torch.Tensor, stream=None) -> None:
     """Plain FP64 engine: K2 (density + Y^k rows) then K3 (table contraction)."""
     L = _native.load()
     s = _native.stream_handle(stream)
     plan = dev.plan
-    _native.check(L.rkb_table_rows_fp64(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
-                                        dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows,
-                                        dev.r.data_ptr(), dev.w.data_ptr(), dev.nv, dev.ng, dev.mo.data_ptr(),
-                                        dev.mi.data_ptr(), ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, s),
-                  "rkb_table_rows_fp64")
+    _fp64_rows(dev, ws, s)
     _native.check(L.rkb_table_contract_fp64(ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, ws.ld, ws.row0.data_ptr(),
                                             ws.nk.data_ptr(), ws.out_off.data_ptr(), ws.tasks.data_ptr(),
                                             ws.n_tasks, out.data_ptr(), s), "rkb_table_contract_fp64")
@@ -462,11 +469,7 @@ def fp64_tables_to_host(dev: IonDevice, ws: Fp64Workspace, out: torch.Tensor, ho
     cs = copy_stream if copy_stream is not None else torch.cuda.Stream(device=out.device)
     h = _native.stream_handle(s)
     plan = dev.plan
-    _native.check(L.rkb_table_rows_fp64(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
-                                        dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows,
-                                        dev.r.data_ptr(), dev.w.data_ptr(), dev.nv, dev.ng, dev.mo.data_ptr(),
-                                        dev.mi.data_ptr(), ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, h),
-                  "rkb_table_rows_fp64")
+    _fp64_rows(dev, ws, h)
     shipper = PackedShipper(plan, host, out.device, cs) if packed else None
     for gi, k in enumerate(plan.ks):
         t0, t1 = ws.task_range[gi]
@@ -570,11 +573,7 @@ def stream_tables(dev: IonDevice, sink, precision: str = "fp64", stream=None, **
         L = _native.load()
         ws = Fp64Workspace(dev)
         h = _native.stream_handle(s)
-        _native.check(L.rkb_table_rows_fp64(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
-                                            dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows,
-                                            dev.r.data_ptr(), dev.w.data_ptr(), dev.nv, dev.ng, dev.mo.data_ptr(),
-                                            dev.mi.data_ptr(), ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, h),
-                      "rkb_table_rows_fp64")
+        _fp64_rows(dev, ws, h)
         nmax = max(plan.n_of_k(k) for k in plan.ks)
         bufs = [torch.empty(nmax * nmax, dtype=torch.float64, device=dev.Pv.device) for _ in range(2)]
         zero = torch.zeros(len(plan.ks), dtype=torch.int64, device=dev.Pv.device)

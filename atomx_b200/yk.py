@@ -68,6 +68,18 @@ def _device_partials(ng: int):
     return resident(mo), resident(mi)
 
 
+#: rows per multipole from which the power table of rkb_yk_rows_pow is used
+POWER_TABLE_ROWS = 16
+
+
+def power_workspace(rows: int, kmax: int, n: int, device) -> torch.Tensor | None:
+    """Workspace of the nodes' powers up to ``kmax`` for that many Y^k rows of n
+    nodes, or None where evaluating them row by row costs less."""
+    if not 0 <= kmax <= 4096 or rows < POWER_TABLE_ROWS * (kmax + 1):
+        return None
+    return torch.empty(2 * (kmax + 1) * n, dtype=torch.float64, device=device)
+
+
 def _run_rows(rho2d: torch.Tensor, ks, r: torch.Tensor, w: torch.Tensor, nv: int, ng: int) -> torch.Tensor:
     """rho2d: (rows, nv*ng) float64 device tensor; ks: int or (rows,) ints."""
     L = _native.require_device()
@@ -79,10 +91,14 @@ def _run_rows(rho2d: torch.Tensor, ks, r: torch.Tensor, w: torch.Tensor, nv: int
                                     mo.data_ptr(), mi.data_ptr(), out.data_ptr(), _native.stream_handle()),
                       "rkb_yk_flat")
         return out
-    kt = torch.as_tensor(np.broadcast_to(np.asarray(ks, dtype=np.int32), (rows,)).copy(), device=rho2d.device)
-    _native.check(L.rkb_yk_rows(rho2d.data_ptr(), n, kt.data_ptr(), rows, r.data_ptr(), w.data_ptr(), nv, ng,
-                                mo.data_ptr(), mi.data_ptr(), out.data_ptr(), n, _native.stream_handle()),
-                  "rkb_yk_rows")
+    ks_h = np.broadcast_to(np.asarray(ks, dtype=np.int32), (rows,))
+    kt = torch.as_tensor(ks_h.copy(), device=rho2d.device)
+    kmax = int(ks_h.max()) if rows else -1
+    pw = power_workspace(rows, kmax, n, rho2d.device)
+    _native.check(L.rkb_yk_rows_pow(rho2d.data_ptr(), n, kt.data_ptr(), rows, r.data_ptr(), w.data_ptr(), nv, ng,
+                                    mo.data_ptr(), mi.data_ptr(), out.data_ptr(), n, _native.ptr(pw), kmax,
+                                    _native.stream_handle()),
+                  "rkb_yk_rows_pow")
     return out
 
 

@@ -61,6 +61,12 @@ int rkb_yk_rows(const double *d_rho, long rho_ld, const int *d_row_k, long nrows
                 const double *d_r, const double *d_w, int nv, int ng,
                 const double *d_mo, const double *d_mi, double *d_yk, long yk_ld,
                 void *stream);
+/* The same with a workspace of 2 (pow_k + 1) nv ng doubles, which the call
+ * fills with the nodes' powers r^k and r^-(k+1) of every k <= pow_k, so that
+ * the rows read them (equal rows; rows with a larger k evaluate their own). */
+int rkb_yk_rows_pow(const double *d_rho, long rho_ld, const int *d_row_k, long nrows, const double *d_r,
+                    const double *d_w, int nv, int ng, const double *d_mo, const double *d_mi, double *d_yk,
+                    long yk_ld, double *d_pow, int pow_k, void *stream);
 
 /* ---------------------------------------------------------------------------
  * Orbital values on the grid: out[o, iv*ng+m] = sum_s coeff[o, iv+s] * bsp[iv, m, s],
@@ -153,6 +159,11 @@ int rkb_table_rows_fp64(const double *d_Pv, const double *d_Qv, long orb_ld, con
                         const double *d_r, const double *d_w, int nv, int ng,
                         const double *d_mo, const double *d_mi, double *d_g, double *d_y,
                         long ld, void *stream);
+/* The same with a power table (rkb_yk_rows_pow). */
+int rkb_table_rows_fp64_pow(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
+                            const long *d_row_pair, const int *d_row_k, long nrows, const double *d_r,
+                            const double *d_w, int nv, int ng, const double *d_mo, const double *d_mi, double *d_g,
+                            double *d_y, long ld, double *d_pow, int pow_k, void *stream);
 
 int rkb_table_contract_fp64(const double *d_g, const double *d_y, long ld, long kdim,
                             const long *d_grp_row0, const long *d_grp_n, const long *d_grp_out,
