@@ -308,11 +308,12 @@ def cell_densities(bank: CellBank, P: torch.Tensor, Q: torch.Tensor, pairs, nsp:
     return D[:n]
 
 
-def _potentials(bank: CellBank, D: torch.Tensor, stream=None) -> torch.Tensor:
-    """W = D K_full^T: row r is the pair potential of density r in bank order."""
+def _potentials(bank: CellBank, D: torch.Tensor, stream=None, out: torch.Tensor | None = None) -> torch.Tensor:
+    """W = D K_full^T: row r is the pair potential of density r in bank order
+    (into ``out``, contiguous rows, when given)."""
     L = _native.load()
     n = D.shape[0]
-    W = torch.empty((max(n, 1), bank.kdim), dtype=torch.float64, device=D.device)
+    W = torch.empty((max(n, 1), bank.kdim), dtype=torch.float64, device=D.device) if out is None else out
     _native.check(L.rkb_gemm_nt_fp64(D.data_ptr(), bank.kdim, bank.K.data_ptr(), bank.kdim, W.data_ptr(), bank.kdim,
                                      n, bank.kdim, bank.kdim, 0, _native.stream_handle(stream)), "rkb_gemm_nt_fp64")
     return W[:n]
@@ -335,6 +336,10 @@ def _sizes(bd):
 
 
 # ------------------------------------------------------ cell integrals
+#: device bytes of densities and potentials that one pass over a batch of keys holds
+_CELL_BYTES = 2 << 30
+
+
 def compute_slater_rk_cell_batch(orbital_arrays, keys, bsp_data, cache=None):
     """R^k(ab, cd) for many (a, b, c, d, k) keys (atomx convol.py:2084).
 
@@ -355,20 +360,34 @@ def compute_slater_rk_cell_batch(orbital_arrays, keys, bsp_data, cache=None):
     dev = torch.device("cuda", torch.cuda.current_device())
     P = _stack([orbital_arrays[n][0] for n in names], ns, dev)
     Q = _stack([orbital_arrays[n][1] for n in names], ns, dev)
-    result = np.zeros(len(keys))
-    by_k: dict = {}
-    for e, kk in enumerate(keys):
-        by_k.setdefault(int(kk[4]), []).append(e)
-    for k, ents in by_k.items():
-        bank = cache.bank(k)
-        lp = np.array([(idx[keys[e][0]], idx[keys[e][1]]) for e in ents], dtype=np.int64)
-        rp = np.array([(idx[keys[e][2]], idx[keys[e][3]]) for e in ents], dtype=np.int64)
-        lu, il = np.unique(lp, axis=0, return_inverse=True)
-        ru, ir = np.unique(rp, axis=0, return_inverse=True)
-        Dl = cell_densities(bank, P, Q, lu, nsp, nsq)
-        W = _potentials(bank, cell_densities(bank, P, Q, ru, nsp, nsq))
-        result[np.asarray(ents)] = to_host(_dots(Dl, W, il.reshape(-1), ir.reshape(-1)))
-    return [float(v) for v in result]
+    n = len(names)
+    kk = np.array([int(key[4]) for key in keys], dtype=np.int64)
+    ab, cd = (np.fromiter((idx[key[i]] * n + idx[key[i + 1]] for key in keys), dtype=np.int64, count=len(keys))
+              for i in (0, 2))
+    ks, kpos = np.unique(kk, return_inverse=True)
+    banks = [cache.bank(int(k)) for k in ks]
+    kdim = banks[0].kdim
+    # the distinct (multipole, pair) rows of each side, multipole by multipole
+    lu, il = np.unique(kpos * (n * n) + ab, return_inverse=True)
+    ru, ir = np.unique(kpos * (n * n) + cd, return_inverse=True)
+    lb, rb = (np.searchsorted(u, np.arange(len(ks) + 1) * (n * n)) for u in (lu, ru))
+    result = np.empty(len(keys))
+    g0 = 0
+    while g0 < len(ks):  # multipoles together as long as their rows stay below _CELL_BYTES
+        g1 = g0 + 1
+        while g1 < len(ks) and (lb[g1 + 1] - lb[g0] + 2 * (rb[g1 + 1] - rb[g0])) * kdim * 8 <= _CELL_BYTES:
+            g1 += 1
+        nl, nr = int(lb[g1] - lb[g0]), int(rb[g1] - rb[g0])
+        pairs = np.concatenate([lu[lb[g0]:lb[g1]], ru[rb[g0]:rb[g1]]]) % (n * n)
+        D = cell_densities(banks[g0], P, Q, np.stack([pairs // n, pairs % n], axis=1), nsp, nsq)
+        W = torch.empty((nr, kdim), dtype=torch.float64, device=dev)
+        for g in range(g0, g1):
+            r0, r1 = int(rb[g] - rb[g0]), int(rb[g + 1] - rb[g0])
+            _potentials(banks[g], D[nl + r0:nl + r1], out=W[r0:r1])
+        ents = np.flatnonzero((kpos >= g0) & (kpos < g1))
+        result[ents] = to_host(_dots(D[:nl], W, il[ents] - lb[g0], ir[ents] - rb[g0]))
+        g0 = g1
+    return result.tolist()
 
 
 def compute_slater_rk_cell(Pa, Qa, Pb, Qb, Pc, Qc, Pd, Qd, bsp_data, k, cache=None):

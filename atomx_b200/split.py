@@ -27,7 +27,7 @@ import torch
 
 from . import _native
 from .split_plan import bits_for_moduli, crt_constants, green_factor_packed, moduli_needed
-from .tables import Fp64Recompute, IonDevice, tile_tasks
+from .tables import Fp64Recompute, IonDevice, PackedShipper, ship_groups, tile_tasks
 from .yk import yk_partial_matrices
 
 __all__ = ["SplitEngine", "IonRows", "factors_for_grid", "host_tables", "choose_width", "DEFAULT_BITS"]
@@ -594,23 +594,28 @@ class SplitEngine:
         _, (_, flagged) = read_status(self.status, s)  # which tables go to FP64: one wait
         fp64 = set(self._failing(self.est.cpu().numpy())) if flagged else set()
         self.escalated = sorted(fp64)
-        from .tables import PackedShipper
-        shipper = PackedShipper(plan, host, self.out.device, cs) if packed else None
-        for gi, k in enumerate(plan.ks):
-            nk, o = plan.n_of_k(k), self.offsets[k]
-            if k in fp64:
-                self._recompute(((k, o),)).run(self.out, s)
+        # failing tables go to FP64 before the split ones around them are shipped
+        groups = ship_groups(plan, [t1 - t0 for t0, t1 in self.task_range])
+        shipper = PackedShipper(plan, host, self.out.device, cs, groups) if packed else None
+        for a, b in groups:
+            ks = plan.ks[a:b]
+            if not fp64.intersection(ks):
+                self._contract(self.grp_out, self.task_range[a][0], self.task_range[b - 1][1], self.out, s)
             else:
-                t0, t1 = self.task_range[gi]
-                self._contract(self.grp_out, t0, t1, self.out, s)
+                for gi, k in enumerate(ks, a):
+                    if k in fp64:
+                        self._recompute(((k, self.offsets[k]),)).run(self.out, s)
+                    else:
+                        self._contract(self.grp_out, *self.task_range[gi], self.out, s)
             if shipper is not None:
-                shipper.ship(k, self.out.data_ptr() + 8 * o, s)
+                shipper.ship([(k, self.out.data_ptr() + 8 * self.offsets[k]) for k in ks], s)
                 continue
             ev = torch.cuda.Event()
             ev.record(s)
             cs.wait_event(ev)
+            o, e = self.offsets[ks[0]], self.offsets[ks[-1]] + plan.n_of_k(ks[-1]) ** 2
             with torch.cuda.stream(cs):
-                host[o:o + nk * nk].copy_(self.out[o:o + nk * nk], non_blocking=True)
+                host[o:e].copy_(self.out[o:e], non_blocking=True)
         self._streamed = True  # the per-table route is already taken
         try:
             self.check_status()

@@ -26,7 +26,7 @@ import torch
 from . import _native
 from .device import as_device, resident
 from .plan import TablePlan, make_plan
-from .yk import power_workspace, yk_partial_matrices
+from .yk import _device_partials, power_workspace, yk_partial_matrices
 
 __all__ = ["IonDevice", "RkTables", "RkStream", "HostTableSink", "HostPackedTables", "PackedShipper", "packed_offsets", "upload_ion", "stage_ion", "evaluate_staged", "upload_values", "slater_rk_tables",
            "slater_rk_tables_from_values", "tables_for", "stream_tables", "iter_blocks", "tile_tasks", "TILE",
@@ -67,13 +67,20 @@ def upload_ion(ion, k_max: int | None = None, plan: TablePlan | None = None, str
     if plan is None:
         plan = make_plan(ion.kappa, ion.spec.k_max if k_max is None else k_max)
     s = _native.stream_handle(stream)
-    r = resident(bsp["gr"]).reshape(-1)
-    w = resident(bsp["grw"]).reshape(-1)
-    mo_h, mi_h = yk_partial_matrices(ng)
-    mo, mi = resident(mo_h), resident(mi_h)
-    bp, bq = resident(bsp["bsp_p"]), resident(bsp["bsp_q"])
-    cp = as_device(ion.P)
-    cq = as_device(ion.Q)
+    mo, mi = _device_partials(ng)
+    inputs = (bsp["gr"], bsp["grw"], bsp["bsp_p"], bsp["bsp_q"], ion.P, ion.Q)
+    if any(isinstance(x, torch.Tensor) for x in inputs):
+        r, w, bp, bq = (resident(x) for x in inputs[:4])
+        cp, cq = as_device(ion.P), as_device(ion.Q)
+    else:  # host arrays: in one copy
+        parts = [np.asarray(x, dtype=np.float64) for x in inputs]
+        offs = np.cumsum([0] + [-(-p.size // 32) * 32 for p in parts]).tolist()
+        host = np.empty(offs[-1])
+        for p, o in zip(parts, offs):
+            host[o:o + p.size] = p.reshape(-1)
+        buf = torch.from_numpy(host).to(torch.device("cuda", torch.cuda.current_device()))
+        r, w, bp, bq, cp, cq = (buf[o:o + p.size].view(p.shape) for p, o in zip(parts, offs))
+    r, w = r.reshape(-1), w.reshape(-1)
     n_orb = cp.shape[0]
     Pv = torch.empty((n_orb, n), device=cp.device, dtype=torch.float64)
     Qv = torch.empty_like(Pv)
@@ -231,12 +238,8 @@ def tile_tasks(sizes, tile: int = TILE, order=None, block: int | None = None):
     row and column panels that stay in L2, where row-major order sweeps a
     whole tile row of column panels (more than L2 holds on large tables)."""
     if block is not None:
-        base = tile_tasks(sizes, tile, order)
-        if base.shape[0] == 0:
-            return base
-        g, ti, tj = base[:, 0], base[:, 1], base[:, 2]
-        grank = np.concatenate([[0], np.cumsum(g[1:] != g[:-1])])  # groups are contiguous
-        return base[np.lexsort((tj, ti, tj // block, ti // block, grank))]
+        return _blocked_tasks(tuple(int(s) for s in np.asarray(sizes).reshape(-1)), tile,
+                              None if order is None else tuple(int(o) for o in order), int(block))
     nt = (np.asarray(sizes, dtype=np.int64).reshape(-1) + tile - 1) // tile
     groups = np.arange(nt.shape[0]) if order is None else np.asarray(order, dtype=np.int64)
     groups = groups[nt[groups] > 0]
@@ -246,6 +249,19 @@ def tile_tasks(sizes, tile: int = TILE, order=None, block: int | None = None):
     g = np.repeat(groups.astype(np.int32), [t.shape[1] for t in tri])
     tt = np.concatenate(tri, axis=1)
     return np.stack([g, tt[0], tt[1]], axis=1)
+
+
+@lru_cache(maxsize=128)
+def _blocked_tasks(sizes: tuple, tile: int, order, block: int) -> np.ndarray:
+    """tile_tasks with ``block`` (read-only, kept per set of sizes: a layout that
+    ions of the same plan share)."""
+    base = tile_tasks(sizes, tile, order)
+    if base.shape[0]:
+        g, ti, tj = base[:, 0], base[:, 1], base[:, 2]
+        grank = np.concatenate([[0], np.cumsum(g[1:] != g[:-1])])  # groups are contiguous
+        base = base[np.lexsort((tj, ti, tj // block, ti // block, grank))]
+    base.setflags(write=False)
+    return base
 
 
 @dataclass
@@ -335,33 +351,50 @@ class HostPackedTables:
         return self.plan.unique_entries
 
 
-class PackedShipper:
-    """Ships finished tables to a pinned host buffer in packed form: each
-    table is packed on the compute stream into one of two rotating device
-    buffers and copied on the copy stream while the next table is computed."""
+def ship_groups(plan: TablePlan, n_tasks) -> list:
+    """Runs of consecutive multipoles [(first, stop)] (indices into plan.ks) to
+    contract in one launch and copy together: small tables share a launch that
+    fills the GPU, a large one goes alone so that its copy overlaps the next.
+    ``n_tasks[i]``: 128 x 128 tiles of table i."""
+    full = 2 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    out, first, tiles = [], 0, 0
+    for i, m in enumerate(n_tasks):
+        tiles += int(m)
+        if tiles >= full or i + 1 == len(n_tasks):
+            out.append((first, i + 1))
+            first, tiles = i + 1, 0
+    return out
 
-    def __init__(self, plan: TablePlan, host: torch.Tensor, device, copy_stream):
+
+class PackedShipper:
+    """Ships finished tables to a pinned host buffer in packed form: a run of
+    consecutive tables is packed on the compute stream into one of two rotating
+    device buffers and copied on the copy stream while the next are computed."""
+
+    def __init__(self, plan: TablePlan, host: torch.Tensor, device, copy_stream, groups):
         self.plan, self.host, self.cs = plan, host, copy_stream
         self.offsets = packed_offsets(plan)
-        nmax = max((plan.n_of_k(k) * (plan.n_of_k(k) + 1) // 2 for k in plan.ks), default=1)
+        self.size = {k: plan.n_of_k(k) * (plan.n_of_k(k) + 1) // 2 for k in plan.ks}
+        nmax = max((sum(self.size[k] for k in plan.ks[a:b]) for a, b in groups), default=1)
         self.bufs = [torch.empty(nmax, dtype=torch.float64, device=device) for _ in range(2)]
         self.free = [None, None]
         self.i = 0
 
-    def ship(self, k: int, table_ptr: int, stream) -> None:
+    def ship(self, tables, stream) -> None:
+        """``tables``: [(k, device address)] of consecutive multipoles."""
         L = _native.load()
         b = self.i % 2
         self.i += 1
         if self.free[b] is not None:
             stream.wait_event(self.free[b])
-        n = self.plan.n_of_k(k)
-        m = n * (n + 1) // 2
-        _native.check(L.rkb_pack_upper(table_ptr, n, self.bufs[b].data_ptr(), _native.stream_handle(stream)),
-                      "rkb_pack_upper")
+        h, base, m = _native.stream_handle(stream), self.bufs[b].data_ptr(), 0
+        for k, ptr in tables:
+            _native.check(L.rkb_pack_upper(ptr, self.plan.n_of_k(k), base + 8 * m, h), "rkb_pack_upper")
+            m += self.size[k]
         ev = torch.cuda.Event()
         ev.record(stream)
         self.cs.wait_event(ev)
-        o = self.offsets[k]
+        o = self.offsets[tables[0][0]]
         with torch.cuda.stream(self.cs):
             self.host[o:o + m].copy_(self.bufs[b][:m], non_blocking=True)
             fe = torch.cuda.Event()
@@ -380,18 +413,21 @@ class Fp64Workspace:
         self.kmax = max(plan.ks)
         self.pow = power_workspace(plan.n_rows, self.kmax, dev.n, dev.Pv.device)
         sizes = [plan.n_of_k(k) for k in plan.ks]
-        self.row0 = torch.as_tensor(np.array([plan.k_row_offset[k] for k in plan.ks], dtype=np.int64),
-                                    device=self.g.device)
-        self.nk = torch.as_tensor(np.array(sizes, dtype=np.int64), device=self.g.device)
         offs = np.concatenate([[0], np.cumsum(np.array(sizes, dtype=np.int64) ** 2)])
-        self.out_off = torch.as_tensor(offs[:-1].astype(np.int64), device=self.g.device)
         self.offsets = {k: int(offs[i]) for i, k in enumerate(plan.ks)}
         self.total = int(offs[-1])
         tasks = tile_tasks(sizes)
         self.n_tasks = int(tasks.shape[0])
-        self.tasks = torch.as_tensor(tasks.reshape(-1), device=self.g.device)
         bounds = np.searchsorted(tasks[:, 0], np.arange(len(sizes) + 1))
         self.task_range = [(int(bounds[i]), int(bounds[i + 1])) for i in range(len(sizes))]
+        # the group records and the task list in one copy
+        m = len(sizes)
+        host = np.zeros(3 * m + (tasks.size + 1) // 2, dtype=np.int64)
+        host[:3 * m] = np.concatenate([[plan.k_row_offset[k] for k in plan.ks], sizes, offs[:-1]])
+        host[3 * m:].view(np.int32)[:tasks.size] = tasks.reshape(-1)
+        arr = torch.from_numpy(host).to(self.g.device)
+        self.row0, self.nk, self.out_off = (arr[i * m:(i + 1) * m] for i in range(3))
+        self.tasks = arr[3 * m:].view(torch.int32)[:tasks.size]
 
 
 def _fp64_rows(dev: IonDevice, ws: Fp64Workspace, h: int) -> None:
@@ -470,21 +506,23 @@ def fp64_tables_to_host(dev: IonDevice, ws: Fp64Workspace, out: torch.Tensor, ho
     h = _native.stream_handle(s)
     plan = dev.plan
     _fp64_rows(dev, ws, h)
-    shipper = PackedShipper(plan, host, out.device, cs) if packed else None
-    for gi, k in enumerate(plan.ks):
-        t0, t1 = ws.task_range[gi]
-        nk, o = plan.n_of_k(k), ws.offsets[k]
+    groups = ship_groups(plan, [t1 - t0 for t0, t1 in ws.task_range])
+    shipper = PackedShipper(plan, host, out.device, cs, groups) if packed else None
+    for a, b in groups:
+        t0, t1 = ws.task_range[a][0], ws.task_range[b - 1][1]
+        ks = plan.ks[a:b]
         _native.check(L.rkb_table_contract_fp64(ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, ws.ld, ws.row0.data_ptr(),
                                                 ws.nk.data_ptr(), ws.out_off.data_ptr(), ws.tasks.data_ptr() + 12 * t0,
                                                 t1 - t0, out.data_ptr(), h), "rkb_table_contract_fp64")
         if shipper is not None:
-            shipper.ship(k, out.data_ptr() + 8 * o, s)
+            shipper.ship([(k, out.data_ptr() + 8 * ws.offsets[k]) for k in ks], s)
             continue
         ev = torch.cuda.Event()
         ev.record(s)
         cs.wait_event(ev)
+        o, e = ws.offsets[ks[0]], ws.offsets[ks[-1]] + plan.n_of_k(ks[-1]) ** 2
         with torch.cuda.stream(cs):
-            host[o:o + nk * nk].copy_(out[o:o + nk * nk], non_blocking=True)
+            host[o:e].copy_(out[o:e], non_blocking=True)
     cs.synchronize()
 
 

@@ -63,9 +63,15 @@ def _check_k(k) -> int:
     return int(k)
 
 
-def _device_partials(ng: int):
+@lru_cache(maxsize=64)
+def _partials_on(ng: int, device: int):
     mo, mi = yk_partial_matrices(ng)
     return resident(mo), resident(mi)
+
+
+def _device_partials(ng: int):
+    """Device copies of the partial matrices: constants of the node count."""
+    return _partials_on(int(ng), torch.cuda.current_device())
 
 
 #: rows per multipole from which the power table of rkb_yk_rows_pow is used
