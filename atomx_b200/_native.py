@@ -62,6 +62,7 @@ _SIGNATURES = {
     "rkb_cell_assemble": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp, _l, _l, _l, _vp],
     "rkb_cell_densities": [_vp, _vp, _l, _vp, _l, _i, _i, _i, _i, _i, _vp, _l, _l, _vp],
     "rkb_gemm_nt_fp64": [_vp, _l, _vp, _l, _vp, _l, _l, _l, _l, _i, _vp],
+    "rkb_gemm_nt_fp64_groups": [_vp, _l, _vp, _vp, _i, _l, _vp, _l, _l, _l, _vp],
     "rkb_cell_dots": [_vp, _l, _vp, _l, _l, _vp, _vp, _l, _vp, _vp],
     "rkb_cell_exchange": [_vp, _l, _vp, _vp, _l, _i, _i, _i, _i, _i, _vp, _vp],
     "rkb_cell_bilinear": [_vp, _l, _i, _vp, _vp, _i, _i, _i, _i, _i, _vp, _vp, _vp],

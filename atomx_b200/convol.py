@@ -308,12 +308,24 @@ def cell_densities(bank: CellBank, P: torch.Tensor, Q: torch.Tensor, pairs, nsp:
     return D[:n]
 
 
-def _potentials(bank: CellBank, D: torch.Tensor, stream=None, out: torch.Tensor | None = None) -> torch.Tensor:
-    """W = D K_full^T: row r is the pair potential of density r in bank order
-    (into ``out``, contiguous rows, when given)."""
+def _potentials_of(banks, rows, D: torch.Tensor, stream=None) -> torch.Tensor:
+    """W = D K_full^T, rows [rows[g], rows[g+1]) of D against banks[g], in one launch."""
+    L = _native.load()
+    kdim = banks[0].kdim
+    W = torch.empty((max(D.shape[0], 1), kdim), dtype=torch.float64, device=D.device)
+    ptrs = np.array([b.K.data_ptr() for b in banks], dtype=np.int64)
+    r0 = np.ascontiguousarray(rows, dtype=np.int64)
+    _native.check(L.rkb_gemm_nt_fp64_groups(D.data_ptr(), kdim, ptrs.ctypes.data, r0.ctypes.data, len(banks), kdim,
+                                            W.data_ptr(), kdim, kdim, kdim, _native.stream_handle(stream)),
+                  "rkb_gemm_nt_fp64_groups")
+    return W[:D.shape[0]]
+
+
+def _potentials(bank: CellBank, D: torch.Tensor, stream=None) -> torch.Tensor:
+    """W = D K_full^T: row r is the pair potential of density r in bank order."""
     L = _native.load()
     n = D.shape[0]
-    W = torch.empty((max(n, 1), bank.kdim), dtype=torch.float64, device=D.device) if out is None else out
+    W = torch.empty((max(n, 1), bank.kdim), dtype=torch.float64, device=D.device)
     _native.check(L.rkb_gemm_nt_fp64(D.data_ptr(), bank.kdim, bank.K.data_ptr(), bank.kdim, W.data_ptr(), bank.kdim,
                                      n, bank.kdim, bank.kdim, 0, _native.stream_handle(stream)), "rkb_gemm_nt_fp64")
     return W[:n]
@@ -336,7 +348,7 @@ def _sizes(bd):
 
 
 # ------------------------------------------------------ cell integrals
-#: device bytes of densities and potentials that one pass over a batch of keys holds
+#: device bytes of densities and potentials that one pass over several multipoles holds
 _CELL_BYTES = 2 << 30
 
 
@@ -380,10 +392,7 @@ def compute_slater_rk_cell_batch(orbital_arrays, keys, bsp_data, cache=None):
         nl, nr = int(lb[g1] - lb[g0]), int(rb[g1] - rb[g0])
         pairs = np.concatenate([lu[lb[g0]:lb[g1]], ru[rb[g0]:rb[g1]]]) % (n * n)
         D = cell_densities(banks[g0], P, Q, np.stack([pairs // n, pairs % n], axis=1), nsp, nsq)
-        W = torch.empty((nr, kdim), dtype=torch.float64, device=dev)
-        for g in range(g0, g1):
-            r0, r1 = int(rb[g] - rb[g0]), int(rb[g + 1] - rb[g0])
-            _potentials(banks[g], D[nl + r0:nl + r1], out=W[r0:r1])
+        W = _potentials_of(banks[g0:g1], rb[g0:g1 + 1] - rb[g0], D[nl:nl + nr])
         ents = np.flatnonzero((kpos >= g0) & (kpos < g1))
         result[ents] = to_host(_dots(D[:nl], W, il[ents] - lb[g0], ir[ents] - rb[g0]))
         g0 = g1
@@ -428,15 +437,30 @@ def cell_tables(P, Q, kappa, bsp_data, k_max: int, cache=None, plan=None, stream
     offs = np.concatenate([[0], np.cumsum(np.asarray(sizes, dtype=np.int64) ** 2)])
     values = torch.empty(int(offs[-1]), dtype=torch.float64, device=dev)
     s = _native.stream_handle(stream)
-    for gi, k in enumerate(plan.ks):
-        bank = cache.bank(k, stream)
-        D = cell_densities(bank, Pd, Qd, plan.pairs[plan.pairs_of_k[k]], nsp, nsq, stream)
-        W = _potentials(bank, D, stream)
-        tasks = torch.as_tensor(tile_tasks([sizes[gi]]).reshape(-1), device=dev)
-        meta = torch.as_tensor(np.array([0, sizes[gi], int(offs[gi])], dtype=np.int64), device=dev)
-        _native.check(L.rkb_table_contract_fp64(D.data_ptr(), W.data_ptr(), bank.kdim, bank.kdim, meta[0:].data_ptr(),
-                                                meta[1:].data_ptr(), meta[2:].data_ptr(), tasks.data_ptr(),
-                                                tasks.shape[0] // 3, values.data_ptr(), s), "rkb_table_contract_fp64")
+    banks = [cache.bank(k, stream) for k in plan.ks]
+    g0 = 0
+    while g0 < len(plan.ks):  # multipoles together as long as their rows stay below _CELL_BYTES
+        kdim, g1, rows = banks[g0].kdim, g0 + 1, sizes[g0]
+        while g1 < len(plan.ks) and 2 * (rows + sizes[g1]) * kdim * 8 <= _CELL_BYTES:
+            rows += sizes[g1]
+            g1 += 1
+        row0 = np.concatenate([[0], np.cumsum(sizes[g0:g1])]).astype(np.int64)
+        pairs = np.concatenate([plan.pairs[plan.pairs_of_k[k]] for k in plan.ks[g0:g1]])
+        D = cell_densities(banks[g0], Pd, Qd, pairs, nsp, nsq, stream)
+        W = _potentials_of(banks[g0:g1], row0, D, stream)
+        m, tasks = g1 - g0, tile_tasks(sizes[g0:g1])
+        host = np.zeros(3 * m + (tasks.size + 1) // 2, dtype=np.int64)
+        host[:3 * m] = np.concatenate([row0[:-1], sizes[g0:g1], offs[g0:g1]])
+        host[3 * m:].view(np.int32)[:tasks.size] = tasks.reshape(-1)
+        meta = torch.from_numpy(host).to(dev)
+        p = meta.data_ptr()
+        _native.check(L.rkb_table_contract_fp64(D.data_ptr(), W.data_ptr(), kdim, kdim, p, p + 8 * m, p + 16 * m,
+                                                p + 24 * m, tasks.shape[0], values.data_ptr(), s),
+                      "rkb_table_contract_fp64")
+        if stream is not None:
+            for x in (D, W, meta):
+                x.record_stream(stream)
+        g0 = g1
     return RkTables(plan=plan, ks=plan.ks, values=values, offsets={k: int(offs[i]) for i, k in enumerate(plan.ks)},
                     precision="cell")
 

@@ -448,6 +448,12 @@ int rkb_cell_densities(const double *d_c1, const double *d_c2, long ld, const lo
                        int n2, int ns_d, int ns_k, int ks, double *d_out, long out_ld, long col_off, void *stream);
 int rkb_gemm_nt_fp64(const double *d_A, long lda, const double *d_B, long ldb, double *d_C, long ldc, long M, long N,
                      long K, int accumulate, void *stream);
+
+/* Row ranges of A against a B each in one launch: C rows row0[g] ..
+ * row0[g+1]-1 = A rows times B[g]^T.  B (device pointers) and row0 (n_groups +
+ * 1 ascending values) are HOST arrays. */
+int rkb_gemm_nt_fp64_groups(const double *d_A, long lda, const void *const *B, const long *row0, int n_groups,
+                            long ldb, double *d_C, long ldc, long N, long K, void *stream);
 int rkb_cell_dots(const double *d_L, long l_ld, const double *d_W, long w_ld, long n, const long *d_il,
                   const long *d_iw, long n_ent, double *d_out, void *stream);
 int rkb_cell_exchange(const double *d_K, long ld, const long *d_kofs, const double *d_dens, long nbatch, int ns,

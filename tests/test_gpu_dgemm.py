@@ -61,3 +61,22 @@ def test_contraction_does_not_depend_on_the_tile(n):
     up = torch.triu(torch.ones(n, n, dtype=torch.bool, device="cuda"))
     err = (one[0] - g @ y.T).abs()
     assert bool((err <= 2.0 * (k + 1) * 2.0 ** -52 * (g.abs() @ y.abs().T))[up].all())
+
+
+@pytest.mark.parametrize("rows", [[5], [0, 33, 0, 64, 1], [700, 0, 900], [3] * 70])
+def test_grouped_gemm_equals_single_ones(rows):
+    """Empty groups, groups that share no tile, more groups than one launch takes."""
+    from atomx_b200 import _native
+    L = _native.require_device()
+    n, k = 1100, 32
+    r0 = np.concatenate([[0], np.cumsum(rows)]).astype(np.int64)
+    A, C = _rand(max(int(r0[-1]), 1), k, seed=3), torch.full((int(r0[-1]), n), float("nan"), dtype=torch.float64, device="cuda")
+    Bs = [_rand(n, k, seed=10 + i) for i in range(len(rows))]
+    ptrs = np.array([b.data_ptr() for b in Bs], dtype=np.int64)
+    _native.check(L.rkb_gemm_nt_fp64_groups(A.data_ptr(), k, ptrs.ctypes.data, r0.ctypes.data, len(rows), k, C.data_ptr(),
+                                            n, n, k, _native.stream_handle()), "rkb_gemm_nt_fp64_groups")
+    for g, b in enumerate(Bs):
+        one = torch.empty(rows[g], n, dtype=torch.float64, device="cuda")
+        _native.check(L.rkb_gemm_nt_fp64(A[int(r0[g]):].data_ptr(), k, b.data_ptr(), k, one.data_ptr(), n, rows[g], n, k,
+                                         0, _native.stream_handle()), "rkb_gemm_nt_fp64")
+        assert torch.equal(one, C[int(r0[g]):int(r0[g + 1])])
