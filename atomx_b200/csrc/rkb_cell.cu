@@ -578,8 +578,8 @@ __global__ void fock_exchange_density_kernel(const __grid_constant__ FockArgs f)
 // over blocks and multipoles are those of one block and multipole at a time.
 // Bound by the latency of the bank reads from L2.  A whole Fock step of 24 targets and
 // 8 multipoles at 120 splines took 6.0 ms in 226 launches, one target a thread (3.5 ms
-// of it in 32 exchange launches), and takes 2.67 ms with eight targets a thread; four
-// targets 3.07, twelve 3.65, four targets of two rows 4.1.
+// of it in 32 exchange launches), and took 2.67 ms with eight targets a thread (2.21 with
+// the grouped GEMM too); four targets 3.07, twelve 3.65, four targets of two rows 4.1.
 constexpr int FOCK_THREADS = 128;  // columns a block
 template <int BT>
 __global__ void __launch_bounds__(FOCK_THREADS, 5) fock_exchange_kernel(const __grid_constant__ FockArgs f) {

@@ -7,9 +7,10 @@
 //     I_in (i in cell m) = B_m + sum_{j in m} g_j r_j^-(k+1) mi[i][j]
 //     Y_i = r_i^-(k+1) I_out(i) + r_i^k I_in(i)
 // where A_m (B_m) is the sum of g r^k (g r^-(k+1)) over all cells left
-// (right) of m.  One warp owns one row: lane l owns cell 32c+l of chunk c,
+// (right) of m.  One warp owns one row, or one chunk of a row when there are few
+// rows (yk_row_block_kernel): lane l owns cell 32c+l of chunk c,
 // forms its cell's terms in registers, and the cell bases come from a
-// warp-shuffle scan plus a running carry across chunks.  Within a cell every
+// warp-shuffle scan plus the carry across chunks.  Within a cell every
 // product and sum is evaluated in the reference's order with round-to-nearest
 // intrinsics (no FMA contraction), so the only difference from the serial
 // reference is the association order of the cross-cell base sums.

@@ -4,10 +4,10 @@ For one ion on the device this builds, once per radial grid, the factored
 Green operator of every multipole (``split_plan.green_factor``), then per
 call runs
 
-* K2x ``rkb_split_rows``: one warp per (pair, k) row forms rho, the factored
-  row [X | Z] and its FP64 core correction vectors, scales the row by a power
+* K2x ``rkb_split_rows_cells_z`` (or another row kernel, see ``IonRows``):
+  every (pair, k) row forms rho, the factored row [X | Z] and its FP64 core correction vectors, scales the row by a power
   of two to ``bits`` bits and writes int8 residues for every CRT modulus;
-* K3s ``rkb_split_contract``: per multipole, the upper 128x128 tiles of the
+* K3s ``rkb_split_contract_z``: per multipole, the upper 128x128 tiles of the
   table as n_mod INT8 GEMMs on tcgen05 with int32 accumulators in TMEM,
   recombined in FP64 by the Chinese remainder theorem, scaled back and
   corrected by the FP64 core terms; tiles above the diagonal are also stored
@@ -45,7 +45,8 @@ KDIM_MAX = 3456
 #: the single-ion contraction takes each table's tiles in blocks of
 #: TASK_BLOCK x TASK_BLOCK (tables.tile_tasks): the tiles in flight then share
 #: their residue panels in L2.  On the Z=70 table 8 measured fastest (2.87
-#: against 2.92 ms row-major; 12 and 16 slower), with identical tables.
+#: against 2.92 ms row-major, of a contraction that takes 2.35 ms now; 12 and
+#: 16 slower), with identical tables.
 TASK_BLOCK = 8
 
 #: doubles per row of the row record (screen bounds, |[X|Z]|, R_aa)

@@ -453,7 +453,7 @@ def run_fp64(dev: IonDevice, ws: Fp64Workspace, out: torch.Tensor, stream=None) 
 class Fp64Recompute:
     """Plain FP64 tables for a set of (ion, k) groups, written at given
     offsets of an output buffer: one Y^k-rows launch per group into a shared
-    workspace, then one grouped persistent contraction over all of them.
+    workspace, then one grouped contraction over all of them.
     The split engines use it for the tables whose certificate fails; the plan
     (workspace, group and task lists) is built once and reused."""
 

@@ -171,7 +171,7 @@ int rkb_table_contract_fp64(const double *d_g, const double *d_y, long ld, long 
 
 /* As rkb_table_contract_fp64 with a contraction length per group,
  * d_grp_kdim[g] (each a multiple of 16 and <= max_kdim <= ld): one
- * persistent launch over the groups of many ions with different grids, whose
+ * launch over the groups of many ions with different grids, whose
  * rows share one (g, y) matrix of stride ld (atomx has no batched
  * counterpart; each group is a table of slater_rk_poisson values). */
 int rkb_table_contract_fp64_groups(const double *d_g, const double *d_y, long ld, long max_kdim,
