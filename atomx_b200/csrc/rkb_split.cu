@@ -42,7 +42,9 @@
 //      The fraction's rounding, 2^-64 of M, is 2^-50 or less of an entry's Schwarz
 //      scale at the default widths, some 4000 times below the split's own error.
 //      Every mbarrier wait is bounded; on timeout the kernel records
-//      RKB_ETIMEDOUT in *status and every role drains and returns.
+//      RKB_ETIMEDOUT in *status, every role gives up, waits (again with a limit) for
+//      the loads and MMAs that it has issued, and returns.  A non-finite entry is only
+//      recorded (its row has zero residues and a NaN scale): the launch runs to its end.
 #include <cuda.h>
 
 #include <cfloat>
@@ -918,15 +920,15 @@ __device__ __forceinline__ bool mbar_try(uint64_t *bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait: false (and status = ETIMEDOUT) after WAIT_LIMIT clock ticks,
-// or as soon as another role has recorded a failure.
+// Bounded wait: false (and status = ETIMEDOUT) after WAIT_LIMIT clock ticks, or as soon as
+// another wait has given up.  RKB_ENONFINITE in the status word ends no wait.
 __device__ __forceinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, int *status) {
     const long long t0 = clock64();
     while (true) {
 #pragma unroll 1
         for (int i = 0; i < 8; ++i)  // the status word is an L2 read: looked at between tries only
             if (mbar_try(bar, parity)) return true;
-        if (*(volatile int *)status != 0) return false;
+        if (*(volatile int *)status == (int)RKB_ETIMEDOUT) return false;
         if (clock64() - t0 > WAIT_LIMIT) {
             atomicExch(status, (int)RKB_ETIMEDOUT);
             return false;
@@ -936,6 +938,16 @@ __device__ __forceinline__ bool mbar_wait_slow(uint64_t *bar, uint32_t parity, i
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *status) {
     if (mbar_try(bar, parity)) return true;
     return mbar_wait_slow(bar, parity, status);
+}
+// The same by a whole warp, with one outcome for all its lanes: what follows a wait (shuffles,
+// .aligned instructions) wants every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, int *status) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, status));
+}
+// After a failure: wait for what is still in flight, whatever the status, with the same limit.
+__device__ __forceinline__ void mbar_drain(uint64_t *bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (!mbar_try(bar, parity) && clock64() - t0 <= WAIT_LIMIT) {}
 }
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -1022,8 +1034,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     TileInfo *info = (TileInfo *)(stage_out + EPI_WARPS * 32 * STG_LD);
     uint64_t *bars = (uint64_t *)(info + 2);
     uint64_t *full = bars, *empty = full + STAGES, *accf = empty + STAGES, *acce = accf + NACC;
-    uint64_t *inff = acce + NACC, *infe = inff + 2;
-    uint32_t *tmem_slot = (uint32_t *)(infe + 2);
+    uint64_t *inff = acce + NACC, *infe = inff + 2, *drain = infe + 2;
+    uint32_t *tmem_slot = (uint32_t *)(drain + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -1039,6 +1051,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             mbar_init(&inff[b], 2);
             mbar_init(&infe[b], EPI_WARPS);
         }
+        mbar_init(drain, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -1078,6 +1091,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                         }
                     }
                 }
+                // given up: the loads of the last STAGES steps may still be under way
+                if (!ok)
+                    for (uint32_t i = it > STAGES ? it - STAGES : 0u; i < it; ++i)
+                        mbar_drain(&full[i % STAGES], (i / STAGES) & 1u);
             }
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
@@ -1106,6 +1123,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                         if (++buf == NACC) { buf = 0; aph ^= 1u; }
                     }
                 }
+                if (!ok) {  // given up: wait for the MMAs issued
+                    mma_commit(drain);
+                    mbar_drain(drain, 0);
+                }
             }
         } else {
             // -------------------------------------------------------- tile records: warp 2 rows, warp 3 columns
@@ -1115,7 +1136,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int g = p.tasks[3 * t], ti = p.tasks[3 * t + 1], tj = p.tasks[3 * t + 2];
                 const long row0 = p.grp_row0[g];
                 const int n = (int)p.grp_n[g];
-                if (!mbar_wait(&infe[buf], ph ^ 1u, status)) break;
+                if (!mbar_wait_warp(&infe[buf], ph ^ 1u, status)) break;
                 TileInfo &I = info[buf];
                 double *rs = rows ? I.rs_row : I.rs_col, *mx = rows ? I.row_max[0] : I.col_max[0];
                 int i = (rows ? ti : tj) * BM + lane;
@@ -1219,7 +1240,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (a0 + rr + sub < n && bc + col < n)
                         I.out[(long)(a0 + rr + sub) * n + bc + col] = seg[rr * STG_LD];
             }
-            if (top == 0x7ff00000u) atomicExch(status, (int)RKB_ENONFINITE);
+            if (top == 0x7ff00000u) atomicCAS(status, 0, (int)RKB_ENONFINITE);
             __syncwarp();
         };
         uint32_t it = 0;  // accumulators taken
@@ -1229,7 +1250,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             // The chunks of the tile before wait for the first digit of this one, in whose
             // shadow (the MMAs run on) they are finished.
             int late = k ? 0 : EPI_COLS;
-            if (k && !mbar_wait(&inff[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, status)) break;
+            if (k && !mbar_wait_warp(&inff[(k - 1) & 1], (uint32_t)((k - 1) >> 1) & 1u, status)) { ok = false; break; }
 #pragma unroll 1
             for (int dg = 0, md = 0; dg < NDIG; ++dg) {
                 long long acc[EPI_COLS];  // the open digit's sum
@@ -1238,7 +1259,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const int end = p.dig_end[dg];
 #pragma unroll 1
                 for (; md < end; ++md, ++it) {
-                    if (!mbar_wait(&accf[it & 1u], (it >> 1) & 1u, status)) { ok = false; break; }
+                    if (!mbar_wait_warp(&accf[it & 1u], (it >> 1) & 1u, status)) { ok = false; break; }
                     tc_fence_after();
                     const int coef = p.coef[md];
                     const uint32_t src = tbase + (it & 1u) * (uint32_t)BN;
@@ -1293,11 +1314,13 @@ __global__ void __launch_bounds__(THREADS, 1)
             }
             if (!ok) break;
         }
-        if (ok && tiles > 0 && mbar_wait(&inff[(tiles - 1) & 1], (uint32_t)((tiles - 1) >> 1) & 1u, status)) {
+        if (ok && tiles > 0 && mbar_wait_warp(&inff[(tiles - 1) & 1], (uint32_t)((tiles - 1) >> 1) & 1u, status)) {
 #pragma unroll 1
             for (int c = 0; c < EPI_COLS; c += FC) finish(info[(tiles - 1) & 1], c);
         }
+        tmem_wait_st();
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (warp == 1) {
