@@ -75,7 +75,10 @@ int sm_count() {
 struct RhoRows {
     const double *rho;
     long ld;
-    static constexpr int BLOCKS = 7;  // of yk_rows_kernel per SM: more rows in flight, or more registers
+    // Blocks of yk_rows_kernel per SM (more rows in flight, or more registers) by node count, with
+    // and without a power table.  20 000 rows of 896 nodes, 7 / 5 / 3 blocks: 181, 214, 255 us at
+    // ng = 7, 253, 273, 372 at 11, and at ng = 16 335, 294, 372.
+    static constexpr int blocks(int ng, bool tab) { return tab ? (ng <= 5 ? 8 : ng <= 11 ? 7 : 5) : (ng <= 11 ? 8 : 4); }
     struct Row {
         const double *__restrict__ rho;
         __device__ __forceinline__ double at(long i) const { return __ldg(rho + i); }
@@ -86,7 +89,8 @@ struct RhoPairs {
     const double *P, *Q;
     long orb_ld;
     const long *pairs, *row_pair;
-    static constexpr int BLOCKS = 5;
+    // 5 / 4 / 3 blocks: 239, 239, 282 us at ng = 8, 341, 325, 345 at 16.
+    static constexpr int blocks(int ng, bool) { return ng <= 5 ? 7 : ng <= 11 ? 5 : 4; }
     struct Row {
         const double *__restrict__ pa, *__restrict__ pc, *__restrict__ qa, *__restrict__ qc;
         // rho = P_a P_c + Q_a Q_c (atomx slater_yk.py:193), each product rounded
@@ -284,7 +288,7 @@ __device__ __forceinline__ void yk_row(const Src &src, const Pow &pw, long q, co
 }
 
 template <int NG, class Src, bool TAB>
-__global__ void __launch_bounds__(128, NG > 0 ? Src::BLOCKS : 1) yk_rows_kernel(Src src, const int *__restrict__ row_k, int k_all, long nrows,
+__global__ void __launch_bounds__(128, NG > 0 ? Src::blocks(NG, TAB) : 1) yk_rows_kernel(Src src, const int *__restrict__ row_k, int k_all, long nrows,
                                                       const double *__restrict__ r, const double *__restrict__ w,
                                                       int nv, int ng, const double *__restrict__ mo,
                                                       const double *__restrict__ mi, double *__restrict__ yk,
@@ -320,7 +324,9 @@ __global__ void __launch_bounds__(128, NG > 0 ? Src::BLOCKS : 1) yk_rows_kernel(
 // is summed at once, the carries follow from the chunk totals in yk_row's order (so the
 // rows are the same to the bit), and both passes go on together.  Latency-bound: the
 // warp-per-row kernel walks 2 x nchunks chunks one after another (a single row of 238
-// nodes 18.5 us from cold caches, 14.9 us here).
+// nodes 18.5 us from cold caches, 14.9 us here).  The partial matrices are in shared memory:
+// as uniform loads from L1 they cost more than the chunks from 13 nodes a cell on (64 rows of
+// 896 nodes, ng = 8, 13, 17: 18, 35 and 57 us, 16, 25 and 35 us now; a warp a row 41, 43, 43).
 template <int NG, class Src>
 __global__ void __launch_bounds__(512) yk_row_block_kernel(Src src, const int *__restrict__ row_k, int k_all,
                                                            const double *__restrict__ r, const double *__restrict__ w,
@@ -329,7 +335,13 @@ __global__ void __launch_bounds__(512) yk_row_block_kernel(Src src, const int *_
                                                            long yk_ld, double *__restrict__ gout) {
     constexpr int GS = NG | 1;
     extern __shared__ double smem_chunk[];
+    constexpr int MS = (NG + 1) & ~1;
+    __shared__ __align__(16) double part[2 * NG * MS];
     __shared__ double total[2][16];
+    for (int i = threadIdx.x; i < NG * NG; i += blockDim.x) {  // read behind the barrier below
+        part[i / NG * MS + i % NG] = mo[i];
+        part[NG * MS + i / NG * MS + i % NG] = mi[i];
+    }
     const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
     double *cbuf = smem_chunk + (long)c * (32 * GS);
     const long n = (long)nv * NG, q = blockIdx.x;
@@ -393,19 +405,19 @@ __global__ void __launch_bounds__(512) yk_row_block_kernel(Src src, const int *_
     auto partial = [&](const double *M, const double (&x)[NG], double base, int i) {
         double s = base;
 #pragma unroll
-        for (int j = 0; j < NG; ++j) s = __dadd_rn(s, __dmul_rn(x[j], __ldg(M + i * NG + j)));
+        for (int j = 0; j < NG; ++j) s = __dadd_rn(s, __dmul_rn(x[j], M[i * MS + j]));
         return s;
     };
     const double base_o = base_of(0, incl_o), base_i = base_of(1, incl_i);
     if (live_o)
 #pragma unroll
-        for (int i = 0; i < NG; ++i) cbuf[lane * GS + i] = partial(mo, h, base_o, i);
+        for (int i = 0; i < NG; ++i) cbuf[lane * GS + i] = partial(part, h, base_o, i);
     __syncwarp();
     for (int t = lane; t < ne_o; t += 32) yrow[o0 + t] = cbuf[t / NG * GS + t % NG];  // I_out parked
     __syncwarp();
     if (live_i)
 #pragma unroll
-        for (int i = 0; i < NG; ++i) cbuf[cl * GS + i] = partial(mi, e, base_i, i);
+        for (int i = 0; i < NG; ++i) cbuf[cl * GS + i] = partial(part + NG * MS, e, base_i, i);
     __syncthreads();  // the whole row's I_out is in place
 #pragma unroll
     for (int u = 0; u < NG; ++u) {
@@ -419,9 +431,12 @@ __global__ void __launch_bounds__(512) yk_row_block_kernel(Src src, const int *_
     }
 }
 
-// Rows up to which a block takes a row: the warp-per-row kernel then leaves SMs idle
-// (two blocks of its four rows per SM).
-static long few_rows() { return 8L * sm_count(); }
+// Rows up to which a block takes a row, by what the warp-per-row kernel would run with.  Rows
+// of 896 nodes, block and warp kernel in us.  Without a power table at ng = 8: 1 185 rows 31 and
+// 48, 2 100 rows 43 and 54, 3 000 rows 59 and 59.  With one: 1 500 rows 37 and 46, 1 800 rows 41
+// and 46, 2 400 rows 51 and 48.  At ng = 17 without a table 1 184 rows 39 and 53, 1 185 rows 57
+// and 53; at ng = 13 with one 1 185 rows 45 and 46, 1 500 rows 57 and 48.
+static long few_rows(int ng, bool tab) { return (ng > 12 ? 8L : tab ? 12L : 16L) * sm_count(); }
 
 template <class Src>
 static int launch_yk(Src src, const int *d_row_k, int k_all, long nrows, const double *d_r, const double *d_w, int nv,
@@ -432,9 +447,11 @@ static int launch_yk(Src src, const int *d_row_k, int k_all, long nrows, const d
     const bool compiled = (ng >= 2 && ng <= 13) || ng == 16 || ng == 17;
     const int gsmax = compiled ? (ng | 1) : (RKB_MAX_NG | 1);
     const size_t chunk = (size_t)32 * gsmax * sizeof(double);  // one chunk buffer per warp, any grid length
-    const bool block = compiled && chunks <= 16 && nrows <= few_rows();
-    // A table of the powers pays for its own launch where rows outnumber multipoles.
-    const bool tab = !block && d_pow != nullptr && pow_k >= 0;
+    // A table of the powers pays for its own launch where rows outnumber multipoles (the caller's
+    // choice), but not below five nodes a cell (4 000 pair rows of 896 nodes at ng = 4: 61 us
+    // without, 79 with one).
+    const bool use = d_pow != nullptr && pow_k >= 0 && ng >= 5;
+    const bool block = compiled && chunks <= 16 && nrows <= few_rows(ng, use), tab = use && !block;
     if (tab) {
         const long n = (long)nv * ng;
         pow_table_kernel<<<dim3((unsigned)ceil_div(n, 128), (unsigned)(pow_k + 1)), 128, 0, st>>>(d_r, n, d_pow);

@@ -74,7 +74,10 @@ def _device_partials(ng: int):
     return _partials_on(int(ng), torch.cuda.current_device())
 
 
-#: rows per multipole from which the power table of rkb_yk_rows_pow is used
+#: rows per multipole from which the power table of rkb_yk_rows_pow is used.  Rows
+#: of 896 nodes and 101 multipoles at ng = 7, 8, 11, without and with the table:
+#: 1800 rows (18 a multipole) 41, 45, 55 and 40, 46, 54 us, 2400 rows (24) 59, 66,
+#: 75 and 42, 48, 56; 20 000 rows and 9 multipoles at ng = 8 266 and 220 us.
 POWER_TABLE_ROWS = 16
 
 
