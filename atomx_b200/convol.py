@@ -45,7 +45,7 @@ import numpy as np
 import torch
 
 from . import _native
-from .device import as_device, resident, to_host
+from .device import as_device, on_stream, resident, to_host, used_on
 
 __all__ = ["ConvolCache", "CellBank", "grid_bank_key", "shared_banks", "SEMISEPARABLE_DIRECT_NS",
            "compute_slater_rk_cell", "compute_slater_fk_cell", "compute_slater_gk_cell",
@@ -108,6 +108,8 @@ class CellBank:
     kq_pad: int
     K: torch.Tensor           # (kdim, kdim) block matrix, kdim = kp_pad + kq_pad
     moments: dict = field(default_factory=dict)   # ("p"|"q", "rising"|"falling") -> (kk, nv)
+    home: object = None       # the stream that built it
+    seen: set = field(default_factory=set)        # streams whose work comes after the build
 
     @property
     def kdim(self) -> int:
@@ -157,20 +159,35 @@ class ConvolCache:
 
     # ------------------------------------------------------------ building
     def bank(self, k: int, stream=None) -> CellBank:
-        k = int(k)
-        if k < 0:
-            raise ValueError("multipole rank must be a nonnegative integer")
-        dkey = (k, torch.cuda.current_device())
-        with self._lock:
-            hit = self._cache.get(dkey)
-            if hit is None:
-                hit = self._cache[dkey] = self._build(k, stream)
-        return hit
+        with on_stream(stream):
+            return self.banks((k,))[0]
 
-    def _build(self, k: int, stream=None) -> CellBank:
+    def banks(self, ks) -> list:
+        """The banks of the multipoles ``ks``, for use on the current stream."""
+        cur, dev, out = torch.cuda.current_stream(), torch.cuda.current_device(), []
+        handle = cur.cuda_stream
+        for k in ks:
+            k = int(k)
+            if k < 0:
+                raise ValueError("multipole rank must be a nonnegative integer")
+            with self._lock:
+                hit = self._cache.get((k, dev))
+                if hit is None:
+                    hit = self._build(k)
+                    hit.home = cur
+                    hit.seen.add(handle)
+                    self._cache[k, dev] = hit
+            if handle not in hit.seen:  # wait for the build, keep the memory for what runs here
+                cur.wait_stream(hit.home)
+                hit.K.record_stream(cur)
+                hit.seen.add(handle)
+            out.append(hit)
+        return out
+
+    def _build(self, k: int) -> CellBank:
         L = _native.require_device()
         bd = self.bsp_data
-        s = _native.stream_handle(stream)
+        s = _native.stream_handle()
         nv, ns = int(bd["nv"]), int(bd["ns"])
         gr, grw = resident(bd["gr"]), resident(bd["grw"])
         ng = int(gr.shape[1])
@@ -296,10 +313,17 @@ def cell_densities(bank: CellBank, P: torch.Tensor, Q: torch.Tensor, pairs, nsp:
     of the (a, b) rows of the coefficient stacks P, Q (atomx _density_sym with
     extents nsp and nsq, convol.py:713), in bank index order."""
     L = _native.load()
-    pr = torch.as_tensor(np.ascontiguousarray(np.asarray(pairs, dtype=np.int64).reshape(-1, 2)), device=P.device)
-    n = int(pr.shape[0])
+    pairs = np.ascontiguousarray(np.asarray(pairs, dtype=np.int64).reshape(-1, 2))
+    n = int(pairs.shape[0])
+    if stream is not None:
+        D = torch.empty((n, bank.kdim), dtype=torch.float64, device=P.device)
+        with on_stream(stream):
+            D.copy_(cell_densities(bank, P, Q, pairs, nsp, nsq))
+        used_on(stream, D, P, Q)
+        return D
+    pr = torch.as_tensor(pairs, device=P.device)
     D = torch.zeros((max(n, 1), bank.kdim), dtype=torch.float64, device=P.device)
-    s = _native.stream_handle(stream)
+    s = _native.stream_handle()
     ld = P.shape[1]
     for comp, C, nsd, ks, off in (("p", P, nsp, bank.ksp, 0), ("q", Q, nsq, bank.ksq, bank.kp_pad)):
         _native.check(L.rkb_cell_densities(C.data_ptr(), C.data_ptr(), ld, pr.data_ptr(), n, ld, ld,
@@ -308,7 +332,7 @@ def cell_densities(bank: CellBank, P: torch.Tensor, Q: torch.Tensor, pairs, nsp:
     return D[:n]
 
 
-def _potentials_of(banks, rows, D: torch.Tensor, stream=None) -> torch.Tensor:
+def _potentials_of(banks, rows, D: torch.Tensor) -> torch.Tensor:
     """W = D K_full^T, rows [rows[g], rows[g+1]) of D against banks[g], in one launch."""
     L = _native.load()
     kdim = banks[0].kdim
@@ -316,28 +340,28 @@ def _potentials_of(banks, rows, D: torch.Tensor, stream=None) -> torch.Tensor:
     ptrs = np.array([b.K.data_ptr() for b in banks], dtype=np.int64)
     r0 = np.ascontiguousarray(rows, dtype=np.int64)
     _native.check(L.rkb_gemm_nt_fp64_groups(D.data_ptr(), kdim, ptrs.ctypes.data, r0.ctypes.data, len(banks), kdim,
-                                            W.data_ptr(), kdim, kdim, kdim, _native.stream_handle(stream)),
+                                            W.data_ptr(), kdim, kdim, kdim, _native.stream_handle()),
                   "rkb_gemm_nt_fp64_groups")
     return W[:D.shape[0]]
 
 
-def _potentials(bank: CellBank, D: torch.Tensor, stream=None) -> torch.Tensor:
+def _potentials(bank: CellBank, D: torch.Tensor) -> torch.Tensor:
     """W = D K_full^T: row r is the pair potential of density r in bank order."""
     L = _native.load()
     n = D.shape[0]
     W = torch.empty((max(n, 1), bank.kdim), dtype=torch.float64, device=D.device)
     _native.check(L.rkb_gemm_nt_fp64(D.data_ptr(), bank.kdim, bank.K.data_ptr(), bank.kdim, W.data_ptr(), bank.kdim,
-                                     n, bank.kdim, bank.kdim, 0, _native.stream_handle(stream)), "rkb_gemm_nt_fp64")
+                                     n, bank.kdim, bank.kdim, 0, _native.stream_handle()), "rkb_gemm_nt_fp64")
     return W[:n]
 
 
-def _dots(Dl: torch.Tensor, W: torch.Tensor, il, iw, stream=None) -> torch.Tensor:
+def _dots(Dl: torch.Tensor, W: torch.Tensor, il, iw) -> torch.Tensor:
     L = _native.load()
     il = torch.as_tensor(np.ascontiguousarray(il, dtype=np.int64), device=Dl.device)
     iw = torch.as_tensor(np.ascontiguousarray(iw, dtype=np.int64), device=Dl.device)
     out = torch.empty(il.shape[0], dtype=torch.float64, device=Dl.device)
     _native.check(L.rkb_cell_dots(Dl.data_ptr(), Dl.shape[1], W.data_ptr(), W.shape[1], Dl.shape[1], il.data_ptr(),
-                                  iw.data_ptr(), il.shape[0], out.data_ptr(), _native.stream_handle(stream)),
+                                  iw.data_ptr(), il.shape[0], out.data_ptr(), _native.stream_handle()),
                   "rkb_cell_dots")
     return out
 
@@ -377,7 +401,7 @@ def compute_slater_rk_cell_batch(orbital_arrays, keys, bsp_data, cache=None):
     ab, cd = (np.fromiter((idx[key[i]] * n + idx[key[i + 1]] for key in keys), dtype=np.int64, count=len(keys))
               for i in (0, 2))
     ks, kpos = np.unique(kk, return_inverse=True)
-    banks = [cache.bank(int(k)) for k in ks]
+    banks = cache.banks(ks)
     kdim = banks[0].kdim
     # the distinct (multipole, pair) rows of each side, multipole by multipole
     lu, il = np.unique(kpos * (n * n) + ab, return_inverse=True)
@@ -423,7 +447,8 @@ def cell_tables(P, Q, kappa, bsp_data, k_max: int, cache=None, plan=None, stream
     """Whole cell-engine tables R^k(ac; bd) over every allowed pair (the
     TablePlan of atomx_b200.plan, same layout as the Poisson engine's
     RkTables): per multipole one density block D, one GEMM for the pair
-    potentials and one symmetric table contraction."""
+    potentials and one symmetric table contraction.  With ``stream`` the work
+    runs there, behind what the current stream holds at the call."""
     from .plan import make_plan
     from .tables import RkTables, tile_tasks
     L = _native.require_device()
@@ -431,36 +456,35 @@ def cell_tables(P, Q, kappa, bsp_data, k_max: int, cache=None, plan=None, stream
     plan = plan or make_plan(np.asarray(kappa), k_max)
     ns, nsp, nsq = _sizes(bsp_data)
     dev = torch.device("cuda", torch.cuda.current_device())
-    Pd = P if isinstance(P, torch.Tensor) and P.is_cuda else _stack(list(np.asarray(P)), ns, dev)
-    Qd = Q if isinstance(Q, torch.Tensor) and Q.is_cuda else _stack(list(np.asarray(Q)), ns, dev)
     sizes = [plan.n_of_k(k) for k in plan.ks]
     offs = np.concatenate([[0], np.cumsum(np.asarray(sizes, dtype=np.int64) ** 2)])
     values = torch.empty(int(offs[-1]), dtype=torch.float64, device=dev)
-    s = _native.stream_handle(stream)
-    banks = [cache.bank(k, stream) for k in plan.ks]
-    g0 = 0
-    while g0 < len(plan.ks):  # multipoles together as long as their rows stay below _CELL_BYTES
-        kdim, g1, rows = banks[g0].kdim, g0 + 1, sizes[g0]
-        while g1 < len(plan.ks) and 2 * (rows + sizes[g1]) * kdim * 8 <= _CELL_BYTES:
-            rows += sizes[g1]
-            g1 += 1
-        row0 = np.concatenate([[0], np.cumsum(sizes[g0:g1])]).astype(np.int64)
-        pairs = np.concatenate([plan.pairs[plan.pairs_of_k[k]] for k in plan.ks[g0:g1]])
-        D = cell_densities(banks[g0], Pd, Qd, pairs, nsp, nsq, stream)
-        W = _potentials_of(banks[g0:g1], row0, D, stream)
-        m, tasks = g1 - g0, tile_tasks(sizes[g0:g1])
-        host = np.zeros(3 * m + (tasks.size + 1) // 2, dtype=np.int64)
-        host[:3 * m] = np.concatenate([row0[:-1], sizes[g0:g1], offs[g0:g1]])
-        host[3 * m:].view(np.int32)[:tasks.size] = tasks.reshape(-1)
-        meta = torch.from_numpy(host).to(dev)
-        p = meta.data_ptr()
-        _native.check(L.rkb_table_contract_fp64(D.data_ptr(), W.data_ptr(), kdim, kdim, p, p + 8 * m, p + 16 * m,
-                                                p + 24 * m, tasks.shape[0], values.data_ptr(), s),
-                      "rkb_table_contract_fp64")
-        if stream is not None:
-            for x in (D, W, meta):
-                x.record_stream(stream)
-        g0 = g1
+    with on_stream(stream):
+        Pd = P if isinstance(P, torch.Tensor) and P.is_cuda else _stack(list(np.asarray(P)), ns, dev)
+        Qd = Q if isinstance(Q, torch.Tensor) and Q.is_cuda else _stack(list(np.asarray(Q)), ns, dev)
+        banks = cache.banks(plan.ks)
+        g0 = 0
+        while g0 < len(plan.ks):  # multipoles together as long as their rows stay below _CELL_BYTES
+            kdim, g1, rows = banks[g0].kdim, g0 + 1, sizes[g0]
+            while g1 < len(plan.ks) and 2 * (rows + sizes[g1]) * kdim * 8 <= _CELL_BYTES:
+                rows += sizes[g1]
+                g1 += 1
+            row0 = np.concatenate([[0], np.cumsum(sizes[g0:g1])]).astype(np.int64)
+            pairs = np.concatenate([plan.pairs[plan.pairs_of_k[k]] for k in plan.ks[g0:g1]])
+            D = cell_densities(banks[g0], Pd, Qd, pairs, nsp, nsq)
+            W = _potentials_of(banks[g0:g1], row0, D)
+            m, tasks = g1 - g0, tile_tasks(sizes[g0:g1])
+            host = np.zeros(3 * m + (tasks.size + 1) // 2, dtype=np.int64)
+            host[:3 * m] = np.concatenate([row0[:-1], sizes[g0:g1], offs[g0:g1]])
+            host[3 * m:].view(np.int32)[:tasks.size] = tasks.reshape(-1)
+            meta = torch.from_numpy(host).to(dev)
+            p = meta.data_ptr()
+            _native.check(L.rkb_table_contract_fp64(D.data_ptr(), W.data_ptr(), kdim, kdim, p, p + 8 * m, p + 16 * m,
+                                                    p + 24 * m, tasks.shape[0], values.data_ptr(),
+                                                    _native.stream_handle()),
+                          "rkb_table_contract_fp64")
+            g0 = g1
+    used_on(stream, values, P, Q)
     return RkTables(plan=plan, ks=plan.ks, values=values, offsets={k: int(offs[i]) for i, k in enumerate(plan.ks)},
                     precision="cell")
 
@@ -531,7 +555,7 @@ def compute_slater_rk_table(M, CP_l, CQ_l, CP_r, CQ_r):
 
 
 # --------------------------------------------------- direct and exchange
-def _full_from_banded(bank: CellBank, Wrow: torch.Tensor, stream=None):
+def _full_from_banded(bank: CellBank, Wrow: torch.Tensor):
     """(J_PP, J_QQ) device: banded potentials of one W row to full matrices."""
     L = _native.load()
     ns = bank.ns
@@ -539,7 +563,7 @@ def _full_from_banded(bank: CellBank, Wrow: torch.Tensor, stream=None):
     for off, ks in ((0, bank.ksp), (bank.kp_pad, bank.ksq)):
         V = torch.zeros((ns, ns), dtype=torch.float64, device=Wrow.device)
         v = Wrow[off:off + ks * ns].contiguous()
-        _native.check(L.rkb_cell_banded_to_full(v.data_ptr(), ns, ks, 1, V.data_ptr(), _native.stream_handle(stream)),
+        _native.check(L.rkb_cell_banded_to_full(v.data_ptr(), ns, ks, 1, V.data_ptr(), _native.stream_handle()),
                       "rkb_cell_banded_to_full")
         out.append(V)
     return out
@@ -558,12 +582,12 @@ def compute_direct_potential_cell(orb_P, orb_Q, bsp_data, k, cache=None):
     return tuple(to_host(m) for m in _full_from_banded(bank, W[0]))
 
 
-def _exchange_blocks(bank: CellBank, left: dict, right: dict, blocks, symmetric_pairs, stream=None):
+def _exchange_blocks(bank: CellBank, left: dict, right: dict, blocks, symmetric_pairs):
     """Device exchange contractions of outer-product densities left[a] x right[b]."""
     L = _native.load()
     ns, dev = bank.ns, bank.K.device
     one = torch.ones(1, dtype=torch.float64, device=dev)
-    s = _native.stream_handle(stream)
+    s = _native.stream_handle()
     out = {}
     for a, b in blocks:
         dens = torch.empty((ns, ns), dtype=torch.float64, device=dev)
@@ -614,7 +638,8 @@ def build_hf_matrices_dbsr(targets, P_stack, Q_stack, angular_direct, angular_ex
     contraction (case 4) into its block; then symmetrised and divided by the
     target's norm.  P_stack/Q_stack: (n_orb, ns) coefficients;
     angular_*: (n_orb, n_orb, k_max+1); k_values: the multipoles to visit.
-    Returns a device tensor (n_targets, 4, ns, ns)."""
+    Returns a device tensor (n_targets, 4, ns, ns).  With ``stream`` the work
+    runs there, behind what the current stream holds at the call."""
     L = _native.require_device()
     cache = cache if isinstance(cache, ConvolCache) else ConvolCache(bsp_data)
     ns = int(bsp_data["ns"])
@@ -622,51 +647,47 @@ def build_hf_matrices_dbsr(targets, P_stack, Q_stack, angular_direct, angular_ex
     targets = np.asarray(targets, dtype=np.int64).reshape(-1)
     nt = targets.shape[0]
     n_orb = int(np.asarray(P_stack).shape[0])
-    P = _stack(list(np.asarray(P_stack)), ns, dev)
-    Q = _stack(list(np.asarray(Q_stack)), ns, dev)
     ks = [int(k) for k in k_values]
     nk = len(ks)
-    banks = [cache.bank(k, stream) for k in ks]
-    s = _native.stream_handle(stream)
     out = torch.empty((nt, 4, ns, ns), dtype=torch.float64, device=dev)
-    if nt == 0:
-        return out
-    norms = np.asarray(norms, dtype=np.float64).reshape(-1)
-    if norms.shape[0] < nt:
-        raise ValueError(f"{nt} targets need as many norms (got {norms.shape[0]})")
-    # [multipole][target][orbital], as the kernels read them
-    ad = np.asarray(angular_direct, dtype=np.float64)[targets][:, :, ks].transpose(2, 0, 1)
-    ax = np.asarray(angular_exchange, dtype=np.float64)[targets][:, :, ks].transpose(2, 0, 1)
-    if banks:
-        ld, q_off, ks_p, ks_q = banks[0].kdim, banks[0].kp_pad, banks[0].ksp, banks[0].ksq
-    else:
-        ld, q_off, ks_p, ks_q = 2 * _round16(ns), _round16(ns), 1, 1
-    dd_ld = max(q_off, ld - q_off)
-    # targets in groups whose exchange densities stay below _FOCK_BYTES
-    group = min(nt, max(1, min(_FOCK_BYTES // (32 * max(nk, 1) * ns * ns), 65535 // (4 * max(nk, 1)))))
-    work = torch.empty(group * nk * (2 * dd_ld + 2 * ld + 4 * ns * ns) + group * 4 * ns * ns, dtype=torch.float64,
-                       device=dev)
-    kptr = np.array([b.K.data_ptr() for b in banks] + [0], dtype=np.int64)
-    for g0 in range(0, nt, group):
-        g1 = min(nt, g0 + group)
-        m = g1 - g0
-        # angular coefficients, norms, targets and bank addresses in one copy
-        parts = [ad[:, g0:g1], ax[:, g0:g1], norms[g0:g1], kptr.view(np.float64),
-                 np.concatenate([targets[g0:g1].astype(np.int32), np.zeros(m % 2, dtype=np.int32)]).view(np.float64)]
-        host = np.concatenate([np.ascontiguousarray(x).reshape(-1) for x in parts])
-        d = torch.from_numpy(host).to(dev)
-        p = [d.data_ptr() + 8 * int(x) for x in np.concatenate([[0], np.cumsum([x.size for x in parts])])]
-        w = [work.data_ptr() + 8 * int(x) for x in np.cumsum([0, 2 * m * nk * dd_ld, 2 * m * nk * ld,
-                                                               4 * m * nk * ns * ns])]
-        _native.check(L.rkb_fock_blocks(kptr.ctypes.data, p[3], ld, q_off, nk, ns, ks_p, ks_q, P.data_ptr(),
-                                        Q.data_ptr(), P.shape[1], n_orb, p[0], p[1], p[4], m, p[2],
-                                        int(bool(skip_pq_exchange)), w[0], dd_ld, w[1], w[2], w[3],
-                                        out[g0:g1].data_ptr(), s), "rkb_fock_blocks")
-        if stream is not None:  # the copy's memory is in use there
-            d.record_stream(stream)
-    if stream is not None:
-        for x in (work, P, Q):
-            x.record_stream(stream)
+    with on_stream(stream):
+        P = _stack(list(np.asarray(P_stack)), ns, dev)
+        Q = _stack(list(np.asarray(Q_stack)), ns, dev)
+        banks = cache.banks(ks)
+        if nt == 0:
+            return out
+        norms = np.asarray(norms, dtype=np.float64).reshape(-1)
+        if norms.shape[0] < nt:
+            raise ValueError(f"{nt} targets need as many norms (got {norms.shape[0]})")
+        # [multipole][target][orbital], as the kernels read them
+        ad = np.asarray(angular_direct, dtype=np.float64)[targets][:, :, ks].transpose(2, 0, 1)
+        ax = np.asarray(angular_exchange, dtype=np.float64)[targets][:, :, ks].transpose(2, 0, 1)
+        if banks:
+            ld, q_off, ks_p, ks_q = banks[0].kdim, banks[0].kp_pad, banks[0].ksp, banks[0].ksq
+        else:
+            ld, q_off, ks_p, ks_q = 2 * _round16(ns), _round16(ns), 1, 1
+        dd_ld = max(q_off, ld - q_off)
+        # targets in groups whose exchange densities stay below _FOCK_BYTES
+        group = min(nt, max(1, min(_FOCK_BYTES // (32 * max(nk, 1) * ns * ns), 65535 // (4 * max(nk, 1)))))
+        work = torch.empty(group * nk * (2 * dd_ld + 2 * ld + 4 * ns * ns) + group * 4 * ns * ns, dtype=torch.float64,
+                           device=dev)
+        kptr = np.array([b.K.data_ptr() for b in banks] + [0], dtype=np.int64)
+        for g0 in range(0, nt, group):
+            g1 = min(nt, g0 + group)
+            m = g1 - g0
+            # angular coefficients, norms, targets and bank addresses in one copy
+            parts = [ad[:, g0:g1], ax[:, g0:g1], norms[g0:g1], kptr.view(np.float64),
+                     np.concatenate([targets[g0:g1].astype(np.int32), np.zeros(m % 2, dtype=np.int32)]).view(np.float64)]
+            host = np.concatenate([np.ascontiguousarray(x).reshape(-1) for x in parts])
+            d = torch.from_numpy(host).to(dev)
+            p = [d.data_ptr() + 8 * int(x) for x in np.concatenate([[0], np.cumsum([x.size for x in parts])])]
+            w = [work.data_ptr() + 8 * int(x) for x in np.cumsum([0, 2 * m * nk * dd_ld, 2 * m * nk * ld,
+                                                                   4 * m * nk * ns * ns])]
+            _native.check(L.rkb_fock_blocks(kptr.ctypes.data, p[3], ld, q_off, nk, ns, ks_p, ks_q, P.data_ptr(),
+                                            Q.data_ptr(), P.shape[1], n_orb, p[0], p[1], p[4], m, p[2],
+                                            int(bool(skip_pq_exchange)), w[0], dd_ld, w[1], w[2], w[3],
+                                            out[g0:g1].data_ptr(), _native.stream_handle()), "rkb_fock_blocks")
+    used_on(stream, out)
     return out
 
 

@@ -3,6 +3,7 @@ for the read-only basis arrays (grid nodes, weights, B-spline values, partial
 matrices) so repeated calls on the same basis do not re-upload them."""
 from __future__ import annotations
 
+import contextlib
 import hashlib
 import threading
 from collections import OrderedDict
@@ -12,7 +13,8 @@ import torch
 
 from . import _native
 
-__all__ = ["as_device", "resident", "to_host", "is_device_tensor", "device", "wait_for"]
+__all__ = ["as_device", "resident", "to_host", "is_device_tensor", "device", "wait_for", "on_stream",
+           "used_on"]
 
 _cache: OrderedDict = OrderedDict()
 _cache_lock = threading.Lock()
@@ -73,3 +75,26 @@ def wait_for(stream) -> None:
     ev = torch.cuda.Event(blocking=True)
     ev.record(stream)
     ev.synchronize()
+
+
+@contextlib.contextmanager
+def on_stream(stream):
+    """Run the block on ``stream`` (None, or the current stream: as it is):
+    its allocations, fills, copies and launches all go there, after everything
+    that the current stream holds so far (the block's inputs)."""
+    if stream is None or stream == torch.cuda.current_stream():
+        yield
+        return
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        yield
+
+
+def used_on(stream, *tensors) -> None:
+    """Tensors of the current stream that work queued on ``stream`` still uses:
+    their memory is not handed out again before that work is done."""
+    if stream is None or stream == torch.cuda.current_stream():
+        return
+    for t in tensors:
+        if isinstance(t, torch.Tensor) and t.is_cuda:
+            t.record_stream(stream)
