@@ -219,7 +219,11 @@ class SplitBatch(_Graphable):
         self.total = int(offs[-1])
         tasks = batch_tasks(g_n, g_kdim, order)
         self.n_tasks = int(tasks.shape[0])
-        # the group records and the task list in one host-to-device copy
+        #: [contraction status, number of tables whose certificate failed]
+        self.status = torch.zeros(2, dtype=torch.int32, device=d)
+        self.est = torch.zeros(len(g_n), dtype=torch.float64, device=d)
+        # the group records and the task list in one host-to-device copy; the upload waits
+        # for the fills above, so that a run on any stream comes behind them
         ng_ = len(g_n)
         host = np.empty(4 * ng_ + (tasks.size + ng_ + 1) // 2, dtype=np.int64)
         host[:4 * ng_] = np.concatenate([g_row0, g_n, g_kdim, offs[:-1]]).astype(np.int64)
@@ -230,9 +234,6 @@ class SplitBatch(_Graphable):
         self.grp_row0, self.grp_n, self.grp_kdim, self.grp_out = (arr[i * ng_:(i + 1) * ng_] for i in range(4))
         words_d = arr[4 * ng_:].view(torch.int32)
         self.tasks, self.grp_zc = words_d[:tasks.size], words_d[tasks.size:tasks.size + ng_]
-        #: [contraction status, number of tables whose certificate failed]
-        self.status = torch.zeros(2, dtype=torch.int32, device=d)
-        self.est = torch.zeros(len(g_n), dtype=torch.float64, device=d)
         self.cert_limit = float(cert_limit)
         #: (ion, k) tables recomputed in FP64 by the last check_status()
         self.escalated: list = []

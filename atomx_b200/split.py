@@ -422,8 +422,13 @@ class SplitEngine:
         # task range of each group (tasks are grouped by multipole) for streaming
         bounds = np.searchsorted(tasks[:, 0], np.arange(len(sizes) + 1))
         self.task_range = [(int(bounds[i]), int(bounds[i + 1])) for i in range(len(sizes))]
+        #: [contraction status, number of tables whose certificate failed]
+        self.status = torch.zeros(2, dtype=torch.int32, device=d)
+        #: certificate estimate of every multipole table (Schwarz-relative error)
+        self.est = torch.zeros(len(sizes), dtype=torch.float64, device=d)
         # the group records (and the zero offsets of the streaming path) and the
-        # task list, in one host-to-device copy
+        # task list, in one host-to-device copy; the upload waits
+        # for the fills above, so that a run on any stream comes behind them
         ng_ = len(sizes)
         host = np.zeros(5 * ng_ + (tasks.size + ng_ + 1) // 2, dtype=np.int64)
         host[:4 * ng_] = np.concatenate([[plan.k_row_offset[k] for k in plan.ks], sizes,
@@ -436,10 +441,6 @@ class SplitEngine:
             arr[i * ng_:(i + 1) * ng_] for i in range(5))
         words_d = arr[5 * ng_:].view(torch.int32)
         self.tasks, self.grp_zc = words_d[:tasks.size], words_d[tasks.size:tasks.size + ng_]
-        #: [contraction status, number of tables whose certificate failed]
-        self.status = torch.zeros(2, dtype=torch.int32, device=d)
-        #: certificate estimate of every multipole table (Schwarz-relative error)
-        self.est = torch.zeros(len(sizes), dtype=torch.float64, device=d)
         self.cert_limit = float(cert_limit)
         #: multipoles recomputed in FP64 by the last check_status()
         self.escalated: list = []

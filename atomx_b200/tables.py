@@ -609,12 +609,12 @@ def stream_tables(dev: IonDevice, sink, precision: str = "fp64", stream=None, **
         held = eng.held_bytes
     else:
         L = _native.load()
+        zero = torch.zeros(len(plan.ks), dtype=torch.int64, device=dev.Pv.device)  # done before the upload of:
         ws = Fp64Workspace(dev)
         h = _native.stream_handle(s)
         _fp64_rows(dev, ws, h)
         nmax = max(plan.n_of_k(k) for k in plan.ks)
         bufs = [torch.empty(nmax * nmax, dtype=torch.float64, device=dev.Pv.device) for _ in range(2)]
-        zero = torch.zeros(len(plan.ks), dtype=torch.int64, device=dev.Pv.device)
         held = (ws.g.numel() + ws.y.numel() + 2 * nmax * nmax) * 8
         for gi, k in enumerate(plan.ks):
             nk = plan.n_of_k(k)
