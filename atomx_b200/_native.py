@@ -74,6 +74,7 @@ _SIGNATURES = {
                         _vp, _vp, _vp, _vp],
     "rkb_split_contract": [_vp, _vp, _l, _l, _i, _vp, _vp, _vp, _vp, _d, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _vp,
                            _vp, _vp, _vp, _l, _vp, _vp, _vp],
+    "rkb_split_crt_weights": [_vp, _i, _vp, _vp, _vp, _vp],
     "rkb_split_contract_z": [_vp, _vp, _l, _l, _l, _i, _vp, _d, _vp, _vp, _vp, _vp, _d, _i, _i, _vp, _vp, _vp, _vp,
                              _vp, _vp, _l, _vp, _vp, _vp],
 }

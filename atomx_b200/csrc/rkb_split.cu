@@ -29,8 +29,9 @@
 //      warps 4-19: epilogue (4 TMEM lane quarters x 4 column groups).  Per modulus
 //              one IMAD.WIDE an entry folds the int32 accumulator, unreduced, into
 //              the open digit's 64-bit sum; three times a tile the digit is reduced
-//              (FP64 quotient) and its CRT weight added to the entry's 64-bit
-//              fraction x / M in TMEM columns 256..511.  A finished tile's scaling,
+//              (FP64 quotient) and its CRT weight added to the entry's 72-bit
+//              fraction x / M, 64 bits of it in TMEM columns 256..511 and a byte in
+//              shared memory.  A finished tile's scaling,
 //              core correction (when it is not screened out) and stores (the tile and
 //              its transpose) run in four chunks between the next tile's first moduli,
 //              so that the MMAs do not wait for them.
@@ -38,9 +39,10 @@
 //      residue and merging residues in pairs took about 13 instructions per entry and
 //      modulus (IMAD.HI issues at a quarter rate), spilled registers went through L2,
 //      and the MMAs stood still during the final phase.  Z=70 table (kdim 1024): 2.88
-//      ms before, 2.35 ms now; N=2112 table (kdim 2176): 2.58 and 2.41 ms.
-//      The fraction's rounding, 2^-64 of M, is 2^-50 or less of an entry's Schwarz
-//      scale at the default widths, some 4000 times below the split's own error.
+//      ms before, 2.47 ms now; N=2112 table (kdim 2176): 2.58 and 2.49 ms.
+//      The fraction is off by 3 x 2^-73 of M at most (one rounding per digit), less than
+//      the 2^-70 of a recombination in doubles; with 64 bits it would be 2^-63.4, more than
+//      a split narrow for its moduli is off by itself.  The eight more bits take 0.10 ms.
 //      Every mbarrier wait is bounded; on timeout the kernel records
 //      RKB_ETIMEDOUT in *status, every role gives up, waits (again with a limit) for
 //      the loads and MMAs that it has issued, and returns.  A non-finite entry is only
@@ -871,6 +873,7 @@ constexpr int NACC = 2;     // int32 accumulator tiles in TMEM (128 columns each
 constexpr int NDIG = 3;     // CRT digits, of up to four moduli each
 constexpr int FC = 8;       // columns per chunk of the final phase
 constexpr int STG_LD = FC + 1;  // doubles per staged row
+constexpr int LOW_WORDS = EPI_WARPS * EPI_COLS / 4 * 32;  // the fractions' lowest bytes, four columns a word
 // What the epilogue needs to know of a tile, fetched ahead of it by two control warps.
 struct __align__(16) TileInfo {
     double rs_row[BM], rs_col[BN];         // row scales
@@ -880,7 +883,8 @@ struct __align__(16) TileInfo {
     int n, ti, tj, pad;
 };
 constexpr size_t SMEM_BYTES = 1024 /*align slack*/ + (size_t)STAGES * STAGE_BYTES +
-                              (size_t)EPI_WARPS * 32 * STG_LD * sizeof(double) + 2 * sizeof(TileInfo) + 256 /*barriers*/;
+                              (size_t)EPI_WARPS * 32 * STG_LD * sizeof(double) + 2 * sizeof(TileInfo) +
+                              LOW_WORDS * sizeof(uint32_t) + 256 /*barriers*/;
 constexpr long long WAIT_LIMIT = 4000000000LL;  // clock64 ticks (~2 s)
 constexpr uint32_t IDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
                            ((uint32_t)(BM >> 4) << 24);
@@ -898,8 +902,8 @@ struct CrtArgs {
     int n_mod;
     // The CRT in two steps. Consecutive moduli (up to dig_end[g]) make a digit modulo
     // D_g < 2^32: d_g = sum_i x_i coef_i mod D_g. Then x / M = sum_g d_g F_g mod 1 with
-    // F_g = f_hi 2^-32 + f_mid 2^-64 + f_lo 2^-96.
-    int dig_end[NDIG], coef[MAXMOD], D[NDIG], f_hi[NDIG], f_mid[NDIG], f_lo[NDIG];
+    // F_g = f_hi 2^-32 + f_mid 2^-64 + f_lo 2^-96 + f_end 2^-112 (f_end of 16 bits).
+    int dig_end[NDIG], coef[MAXMOD], D[NDIG], f_hi[NDIG], f_mid[NDIG], f_lo[NDIG], f_end[NDIG];
     double inv_D[NDIG], inv_D32[NDIG];  // 1/D, 2^32/D
     double M;  // the product of the moduli, times 2^-32
 };
@@ -1017,6 +1021,10 @@ __device__ __forceinline__ double int_to_double(int v) {
 __device__ __forceinline__ double uint_to_double(uint32_t v) {
     return __dadd_rn(__hiloint2double(0x43300000, (int)v), -4503599627370496.0);
 }
+// 2^8 v plus a byte
+__device__ __forceinline__ double uint40_to_double(uint32_t v, uint32_t byte) {
+    return __dadd_rn(__hiloint2double((int)(0x43300000u | (v >> 24)), (int)((v << 8) | byte)), -4503599627370496.0);
+}
 // acc mod D nearest zero. |acc| < 2^59 and D < 2^32, so the quotient's rounding error is
 // far below 1 and |result| <= D/2 (1 + 2^-25).
 __device__ __forceinline__ int mod_near(long long acc, int D, double inv_D, double inv_D32) {
@@ -1032,7 +1040,8 @@ __global__ void __launch_bounds__(THREADS, 1)
     unsigned char *ring = base;
     double *stage_out = (double *)(ring + (size_t)STAGES * STAGE_BYTES);
     TileInfo *info = (TileInfo *)(stage_out + EPI_WARPS * 32 * STG_LD);
-    uint64_t *bars = (uint64_t *)(info + 2);
+    uint32_t *low_all = (uint32_t *)(info + 2);
+    uint64_t *bars = (uint64_t *)(low_all + LOW_WORDS);
     uint64_t *full = bars, *empty = full + STAGES, *accf = empty + STAGES, *acce = accf + NACC;
     uint64_t *inff = acce + NACC, *infe = inff + 2, *drain = infe + 2;
     uint32_t *tmem_slot = (uint32_t *)(drain + 1);
@@ -1174,7 +1183,10 @@ __global__ void __launch_bounds__(THREADS, 1)
         const uint32_t tbase = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cgrp * EPI_COLS);
         double *stg = stage_out + (size_t)ew * 32 * STG_LD;
         const int tiles = (int)((p.n_tasks - blockIdx.x + gridDim.x - 1) / gridDim.x);
-        const uint32_t park = tbase + (uint32_t)(NACC * BN);  // x / M mod 1: low words, high words BN columns on
+        // x / M mod 1 of this thread's row: words of 2^-64 and, BN columns on, of 2^-32 in TMEM, and the
+        // bytes of 2^-72 of four columns in a word of shared memory that no other thread touches
+        const uint32_t park = tbase + (uint32_t)(NACC * BN);
+        uint32_t *low = low_all + ew * (EPI_COLS / 4 * 32) + lane;
         double *row = stg + lane * STG_LD;
         // One chunk of FC columns of a finished tile: scaling, correction and stores.
         auto finish = [&](const TileInfo &I, int c) {
@@ -1187,11 +1199,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                 int lo[4], hi[4];
                 tmem_ld4(park + (uint32_t)(c + h), lo);
                 tmem_ld4(park + (uint32_t)(BN + c + h), hi);
+                const uint32_t bytes = low[(c + h) * 8];
                 tmem_wait_ld();
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    row[h + j] = __fma_rn(uint_to_double((uint32_t)lo[j]), 0x1p-32, int_to_double(hi[j])) *
-                                 (rs_a * rs_b[h + j]);
+                    row[h + j] = __fma_rn(uint40_to_double((uint32_t)lo[j], (bytes >> (8 * j)) & 0xffu), 0x1p-40,
+                                          int_to_double(hi[j])) * (rs_a * rs_b[h + j]);
             }
             // Correction screen for this warp's 32 x EPI_COLS block: with per-row bounds
             // relative to each row's scale, |left_a . right_b| <= 2^(e_a+e_b) *
@@ -1287,29 +1300,36 @@ __global__ void __launch_bounds__(THREADS, 1)
                     for (; late < EPI_COLS; late += FC) finish(info[(k - 1) & 1], late);
                     if (lane == 0) mbar_arrive(&infe[(k - 1) & 1]);
                 }
-                // f += d F mod 1, rounded to 2^-64
-                const int D = p.D[dg], fh = p.f_hi[dg], fm = p.f_mid[dg], fl = p.f_lo[dg];
+                // f += d F mod 1, rounded to 2^-72
+                const int D = p.D[dg], fh = p.f_hi[dg], fm = p.f_mid[dg], fl = p.f_lo[dg], fe = p.f_end[dg];
                 const double inv_D = p.inv_D[dg], inv_D32 = p.inv_D32[dg];
                 tmem_wait_st();
 #pragma unroll
                 for (int c = 0; c < EPI_COLS; c += 4) {
                     int lo[4] = {0, 0, 0, 0}, hi[4] = {0, 0, 0, 0};
+                    uint32_t bytes = 0u, t[4];
                     if (dg) {
                         tmem_ld4(park + (uint32_t)c, lo);
                         tmem_ld4(park + (uint32_t)(BN + c), hi);
+                        bytes = low[c * 8];
                         tmem_wait_ld();
                     }
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int d = mod_near(acc[c + j], D, inv_D, inv_D32);
+                        // units of 2^-96: the byte so far in bits 24..31, half a unit of it below; the product
+                        // with the weight's end needs d to 16 bits only (off by 2^-81)
+                        long long e = (long long)(d >> 16) * fe + __byte_perm(bytes, 0x00800000u, 0x0644u | (j << 12));
+                        e += (long long)d * fl;
                         long long f = ((long long)hi[j] << 32) | (uint32_t)lo[j];
-                        f += (long long)d * fm + ((long long)((uint32_t)d * (uint32_t)fh) << 32) +
-                             (((long long)d * fl + 0x80000000LL) >> 32);
+                        f += (long long)d * fm + ((long long)((uint32_t)d * (uint32_t)fh) << 32) + (e >> 32);
                         lo[j] = (int)f;
                         hi[j] = (int)(f >> 32);
+                        t[j] = (uint32_t)e;
                     }
                     tmem_st4(park + (uint32_t)c, lo);
                     tmem_st4(park + (uint32_t)(BN + c), hi);
+                    low[c * 8] = __byte_perm(__byte_perm(t[0], t[1], 0x0073), __byte_perm(t[2], t[3], 0x0073), 0x5410);
                 }
             }
             if (!ok) break;
@@ -1372,7 +1392,10 @@ static void crt_weights(const int *moduli, int n_mod, CrtArgs &p) {
         // F = ((M/D)^-1 mod D) / D in [-1/2, 1/2)
         const __int128 cs = 2 * c >= D ? (__int128)c - (__int128)D : (__int128)c, Ds = (__int128)D;
         const __int128 f = one / Ds * cs + one % Ds * cs / Ds;
-        const __int128 w = (f + ((__int128)1 << 29)) >> 30;  // 96 bits; the two lower words are read as signed
+        // 112 bits; every word but the first is read as signed
+        const __int128 v = (f + ((__int128)1 << 13)) >> 14;
+        p.f_end[g] = (int)(int16_t)(uint16_t)v;
+        const __int128 w = (v - p.f_end[g]) >> 16;
         p.f_lo[g] = (int)(uint32_t)w;
         const uint64_t t = (uint64_t)(w >> 32) + ((uint32_t)w >> 31);
         p.f_mid[g] = (int)(uint32_t)t;
@@ -1605,6 +1628,21 @@ extern "C" int rkb_split_rows_fused(const double *d_Pv, const double *d_Qv, long
         default: split_rows_fused_kernel<11><<<grid, block, 0, st>>>(a); break;
     }
     RKB_LAUNCHED("split_rows_fused_kernel");
+    return RKB_OK;
+}
+
+extern "C" int rkb_split_crt_weights(const int *moduli, int n_mod, int *dig_end, int *coef, unsigned *digit, int *weight) {
+    RKB_CHECK_ARG(n_mod >= 4 && n_mod <= MAXMOD, "split contraction takes 4..%d moduli (got %d)", MAXMOD, n_mod);
+    for (int i = 0; i < n_mod; ++i) RKB_CHECK_ARG(moduli[i] >= 2 && moduli[i] <= 256, "moduli must lie in [2, 256]");
+    CrtArgs p;
+    crt_weights(moduli, n_mod, p);
+    for (int i = 0; i < n_mod; ++i) coef[i] = p.coef[i];
+    for (int g = 0; g < NDIG; ++g) {
+        dig_end[g] = p.dig_end[g];
+        digit[g] = (unsigned)p.D[g];
+        const int w[4] = {p.f_hi[g], p.f_mid[g], p.f_lo[g], p.f_end[g]};
+        for (int i = 0; i < 4; ++i) weight[4 * g + i] = w[i];
+    }
     return RKB_OK;
 }
 

@@ -45,7 +45,7 @@ KDIM_MAX = 3456
 #: the single-ion contraction takes each table's tiles in blocks of
 #: TASK_BLOCK x TASK_BLOCK (tables.tile_tasks): the tiles in flight then share
 #: their residue panels in L2.  On the Z=70 table 8 measured fastest (2.87
-#: against 2.92 ms row-major, of a contraction that takes 2.35 ms now; 12 and
+#: against 2.92 ms row-major, of a contraction that takes 2.47 ms now; 12 and
 #: 16 slower), with identical tables.
 TASK_BLOCK = 8
 

@@ -243,7 +243,7 @@ int rkb_exchange_matrix(const double *d_fb, const double *d_bsp, const double *d
  * rkb_split_contract: for every task (group, tile_i, tile_j >= tile_i) the
  * 128 x 128 tile of R_g is computed as n_mod residue GEMMs of length
  * d_grp_kdim[g] (multiple of 128, <= 3456) on the tensor cores, CRT-recombined
- * to 64 bits of x / M (M, the product of the moduli, as a double; the CRT
+ * to 72 bits of x / M (M, the product of the moduli, as a double; the CRT
  * weights follow from the moduli, and pair_inv, f_hi and f_lo are not read),
  * scaled and corrected, and written (and
  * mirrored) into the n x n block at d_out + d_grp_out[g], as
@@ -375,6 +375,13 @@ int rkb_split_contract_z(const signed char *d_resA, const signed char *d_resB, l
                          const long *d_grp_row0, const long *d_grp_n, const long *d_grp_kdim,
                          const int *d_grp_zchunk, const long *d_grp_out, const int *d_tasks,
                          long n_tasks, double *d_out, int *d_status, void *stream);
+/* Host-only: the constants with which the contraction recombines the residues
+ * of n_mod (4..12) moduli.  The moduli up to dig_end[g] (g < 3) make a digit
+ * modulo digit[g], d_g = sum_i x_i coef[i] mod digit[g], nearest zero (x_i: any
+ * integer of the residue class), and x / M = sum_g d_g F_g mod 1 with F_g =
+ * weight[4g] 2^-32 + weight[4g+1] 2^-64 + weight[4g+2] 2^-96 + weight[4g+3]
+ * 2^-112.  The kernel rounds each product to 2^-72. */
+int rkb_split_crt_weights(const int *moduli, int n_mod, int *dig_end, int *coef, unsigned *digit, int *weight);
 
 /* rkb_split_certify: per table g (rows d_grp_row0[g] .. + d_grp_n[g]) the
  * estimate d_est[g] = max_a h_a / sqrt|R_aa| * max_b |[X|Z]_b| / sqrt|R_bb|
