@@ -52,6 +52,7 @@
 #include <cfloat>
 
 #include <mutex>
+#include <numeric>
 
 #include "rkb_common.cuh"
 
@@ -1366,14 +1367,24 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-static int inverse_mod(int a, int m) {  // by trial (m <= 256); 0 when there is none
-    for (int x = 1; x < m; ++x)
-        if (a % m * x % m == 1 % m) return x;
-    return 0;
+static int inverse_mod(int a, int m) {  // a and m coprime, m >= 2 (extended Euclid)
+    int r0 = m, r1 = a % m, t0 = 0, t1 = 1;
+    while (r1 > 1) {
+        const int q = r0 / r1, r2 = r0 - q * r1, t2 = t0 - q * t1;
+        r0 = r1, r1 = r2, t0 = t1, t1 = t2;
+    }
+    return t1 < 0 ? t1 + m : t1;
 }
 
-// The CRT constants of the contraction (CrtArgs).
-static void crt_weights(const int *moduli, int n_mod, CrtArgs &p) {
+// The CRT constants of the contraction (CrtArgs); 4..MAXMOD pairwise coprime moduli in [2, 256].
+static int crt_weights(const int *moduli, int n_mod, CrtArgs &p) {
+    RKB_CHECK_ARG(n_mod >= 4 && n_mod <= MAXMOD, "split contraction takes 4..%d moduli (got %d)", MAXMOD, n_mod);
+    for (int i = 0; i < n_mod; ++i) {
+        RKB_CHECK_ARG(moduli[i] >= 2 && moduli[i] <= 256, "moduli must lie in [2, 256]");
+        for (int j = 0; j < i; ++j)
+            RKB_CHECK_ARG(std::gcd(moduli[j], moduli[i]) == 1, "moduli %d and %d have a common factor", moduli[j],
+                          moduli[i]);
+    }
     const __int128 one = (__int128)1 << 126;
     for (int g = 0, i0 = 0; g < NDIG; ++g) {
         const int i1 = i0 + (n_mod - i0 + NDIG - g - 1) / (NDIG - g);  // 4 to 12 moduli in three even parts
@@ -1405,6 +1416,7 @@ static void crt_weights(const int *moduli, int n_mod, CrtArgs &p) {
         p.inv_D32[g] = 4294967296.0 / (double)D;
         p.dig_end[g] = i0 = i1;
     }
+    return RKB_OK;
 }
 
 static int make_map(CUtensorMap *map, const void *ptr, long kpad, long rows) {
@@ -1632,10 +1644,9 @@ extern "C" int rkb_split_rows_fused(const double *d_Pv, const double *d_Qv, long
 }
 
 extern "C" int rkb_split_crt_weights(const int *moduli, int n_mod, int *dig_end, int *coef, unsigned *digit, int *weight) {
-    RKB_CHECK_ARG(n_mod >= 4 && n_mod <= MAXMOD, "split contraction takes 4..%d moduli (got %d)", MAXMOD, n_mod);
-    for (int i = 0; i < n_mod; ++i) RKB_CHECK_ARG(moduli[i] >= 2 && moduli[i] <= 256, "moduli must lie in [2, 256]");
     CrtArgs p;
-    crt_weights(moduli, n_mod, p);
+    const int rc = crt_weights(moduli, n_mod, p);
+    if (rc) return rc;
     for (int i = 0; i < n_mod; ++i) coef[i] = p.coef[i];
     for (int g = 0; g < NDIG; ++g) {
         dig_end[g] = p.dig_end[g];
@@ -1663,23 +1674,26 @@ extern "C" int rkb_split_contract_z(const signed char *d_resA, const signed char
     RKB_CHECK_ARG(cw <= cwp, "cw must be <= cwp");
     RKB_CHECK_ARG(d_cbound != nullptr && corr_floor >= 0.0, "correction bounds and a nonnegative floor are required");
     if (n_tasks == 0) return RKB_OK;
+    CrtArgs p;
+    int rc = crt_weights(moduli, n_mod, p);
+    if (rc) return rc;
+    double prod = 1.0;
+    for (int i = 0; i < n_mod; ++i) prod *= moduli[i];
+    RKB_CHECK_ARG(M >= prod * (1.0 - 1e-14) && M <= prod * (1.0 + 1e-14), "M (%g) is not the product of the moduli (%g)",
+                  M, prod);
     CUtensorMap mA, mB;
-    int rc = make_map(&mA, d_resA, kpad, (long)n_mod * nrows_total);
+    rc = make_map(&mA, d_resA, kpad, (long)n_mod * nrows_total);
     if (rc) return rc;
     rc = d_resB ? make_map(&mB, d_resB, b_ld, (long)n_mod * nrows_total) : make_map(&mB, d_resA, kpad, (long)n_mod * nrows_total);
     if (rc) return rc;
-    CrtArgs p;
     p.rowscale = d_rowscale; p.left = d_left; p.right = d_right; p.cbound = d_cbound; p.corr_floor = corr_floor;
     p.cwp = cwp; p.cw = cw;
     p.grp_row0 = d_grp_row0; p.grp_n = d_grp_n; p.grp_kdim = d_grp_kdim; p.grp_out = d_grp_out;
     p.grp_zc = d_resB ? d_grp_zchunk : nullptr;
     p.tasks = d_tasks; p.n_tasks = n_tasks; p.nrows_total = nrows_total; p.out = d_out; p.status = d_status;
     p.n_mod = n_mod; p.M = M * 0x1p-32;
-    for (int i = 0; i < n_mod; ++i) RKB_CHECK_ARG(moduli[i] >= 2 && moduli[i] <= 256, "moduli must lie in [2, 256]");
-    crt_weights(moduli, n_mod, p);
     long grid = n_tasks < sm_count() ? n_tasks : sm_count();
     cudaStream_t st = as_stream(stream);
-    RKB_CHECK_ARG(n_mod >= 4, "split contraction takes 4..%d moduli (got %d)", MAXMOD, n_mod);
     RKB_CUDA(set_smem(crt_syrk_kernel, (int)SMEM_BYTES));
     crt_syrk_kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, st>>>(mA, mB, p);
     RKB_LAUNCHED("crt_syrk_kernel");

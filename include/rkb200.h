@@ -238,7 +238,8 @@ int rkb_exchange_matrix(const double *d_fb, const double *d_bsp, const double *d
  * x kpad doubles that receives the FP64 rows [X | Z | 0] before they are
  * rounded.  A row with a non-finite value gets a NaN scale and zero residues,
  * so every entry it reaches comes out NaN.
- * `moduli` is a HOST array of n_mod pairwise-coprime ints <= 256.
+ * `moduli` is a HOST array of n_mod pairwise-coprime ints <= 256; the
+ * contraction refuses others, and an M that is not their product (RKB_EINVAL).
  *
  * rkb_split_contract: for every task (group, tile_i, tile_j >= tile_i) the
  * 128 x 128 tile of R_g is computed as n_mod residue GEMMs of length

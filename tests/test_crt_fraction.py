@@ -37,3 +37,34 @@ def test_fraction_of_every_size(n_mod):
             err = abs(Fraction(w.fraction(v), 1 << 72) - Fraction(x, M))
             worst = max(worst, min(err, 1 - err))
     assert worst <= Fraction(3, 1 << 73) + Fraction(3, 1 << 81) < Fraction(1, 1 << 70)
+
+
+def _contract(moduli, M):
+    """Status of a contraction call that is refused before it looks at a device."""
+    import ctypes
+
+    import numpy as np
+    from atomx_b200 import _native
+    ms, some = np.ascontiguousarray(moduli, dtype=np.int32), 256
+    return _native.load().rkb_split_contract_z(
+        some, 0, 128, 128, 128, len(ms), ms.ctypes.data_as(ctypes.c_void_p), float(M), some, some, some, some, 0.0, 9,
+        10, some, some, some, 0, some, some, 1, some, some, 0)
+
+
+@pytest.mark.parametrize("moduli,scale", [
+    ((256, 255, 254, 251), 1.0),       # 256 and 254
+    ((256, 255, 253, 251, 51), 1.0),   # 255 and 51, in different digits
+    ((13, 13, 17, 19), 1.0),
+    ((256, 255, 253, 251), 1.0 + 1e-12),
+    ((256, 255, 253, 251), 0.5),
+    ((256, 255, 253, 251), float("nan")),
+])
+def test_wrong_moduli_or_product_is_refused(moduli, scale):
+    import math
+
+    from atomx_b200 import _native
+    assert _contract(moduli, math.prod(moduli) * scale) == 1
+    assert b"moduli" in _native.load().rkb_last_error()
+    if scale == 1.0:
+        with pytest.raises(ValueError):
+            Weights(moduli)
