@@ -83,6 +83,12 @@ __device__ __forceinline__ double transfer_at(const Tables &T, long p) {  // of 
     return q < T.ncuts - 1 && T.cuts[q] == p ? T.transfer[q - 1] : 1.0;
 }
 
+// A factor >= 0, kept above zero: the product of many frames' factors may underflow where the
+// serial scan, which applies them one by one, keeps an infinite sum infinite.
+__device__ __forceinline__ double above_zero(double m) {
+    return __hiloint2double(max(__double2hiint(m), 0x00100000), __double2loint(m));
+}
+
 // x -> m x + s composed along the lanes: lane l receives the map of lanes 0..l in order
 // (UP), or of lanes 31..l (down).
 template <bool UP>
@@ -93,7 +99,7 @@ __device__ __forceinline__ void scan_maps(double &m, double &s, int lane) {
         const double s2 = UP ? __shfl_up_sync(FULL, s, o) : __shfl_down_sync(FULL, s, o);
         if (UP ? lane >= o : lane + o < 32) {
             s = fma(s2, m, s);
-            m *= m2;
+            m = above_zero(m * m2);
         }
     }
 }
@@ -186,7 +192,8 @@ __device__ __forceinline__ void tile_y(const Tables &T, const Dens &rho, long ba
         double above = __shfl_down_sync(FULL, s, 1);
         if (lane == 31) above = A;
         A = __shfl_sync(FULL, s, 0);
-        y[c] = rk[c] * fma(hr[c], b[c], t * above);
+        // nothing lies behind the last point (and its h_i = 0 times an infinite density is no zero)
+        y[c] = EDGE && base + 32 * c + lane + 1 >= T.n ? 0.0 : rk[c] * fma(hr[c], b[c], t * above);
     }
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
@@ -219,7 +226,7 @@ __device__ void carry_scan(const Tables &T, double *sums, int ntiles, int lane) 
             s = sums[i];
             // outward: frame starts in [base, base + TILE); inward: in (base, base + TILE]
             const long first = (long)i * TILE + (UP ? 0 : 1);
-            for (long q = frame_from(T, first); q < T.ncuts - 1 && T.cuts[q] < first + TILE; ++q) m *= T.transfer[q - 1];
+            for (long q = frame_from(T, first); q < T.ncuts - 1 && T.cuts[q] < first + TILE; ++q) m = above_zero(m * T.transfer[q - 1]);
         }
         scan_maps<UP>(m, s, lane);
         const double after = fma(m, carry, s);  // the value behind this lane's tile
