@@ -356,16 +356,25 @@ static int grid_common_checks(long n, long ncuts, long ntr, long i_cut) {
 template <bool DOTS>
 static int launch_rows(const grid::BatchArgs &a, cudaStream_t st) {
     auto kern = grid::grid_rows_kernel<DOTS>;
-    const long ctas = a.nrows < 8L * sm_count() ? a.nrows : 8L * sm_count();
+    long ctas = a.nrows < 8L * sm_count() ? a.nrows : 8L * sm_count();
     const size_t bytes = sizeof(double) * 2 * (size_t)ceil_div(a.n, grid::TILE);  // the tiles' sums and carries
     double *scratch = nullptr;
-    const bool fits = bytes <= 200 * 1024;  // above 3.2 million points they go to device memory
-    if (fits) RKB_CUDA(set_smem(kern, (int)bytes));
-    else RKB_CUDA(cudaMallocAsync(reinterpret_cast<void **>(&scratch), bytes * ctas, st));
+    const bool fits = bytes <= 200 * 1024;
+    if (fits) {
+        RKB_CUDA(set_smem(kern, (int)bytes));
+    } else {  // above 1 638 400 points they go to device memory (n / 8 bytes a CTA): fewer CTAs where that is short
+        cudaError_t e;
+        while ((e = cudaMallocAsync(reinterpret_cast<void **>(&scratch), bytes * ctas, st)) == cudaErrorMemoryAllocation &&
+               ctas > 1) {
+            cudaGetLastError();
+            ctas = (ctas + 3) / 4;
+        }
+        RKB_CUDA(e);
+    }
     kern<<<(unsigned)ctas, grid::THREADS, fits ? bytes : 0, st>>>(a, scratch);
-    const cudaError_t e = cudaGetLastError();
-    if (scratch) cudaFreeAsync(scratch, st);
+    const cudaError_t e = cudaGetLastError(), f = scratch ? cudaFreeAsync(scratch, st) : cudaSuccess;
     if (e != cudaSuccess) return cuda_status(e, "grid_rows_kernel");
+    RKB_CUDA(f);
     return RKB_OK;
 }
 

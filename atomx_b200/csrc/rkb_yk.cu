@@ -35,6 +35,7 @@ void set_error(const char *fmt, ...) {
 }
 
 int cuda_status(cudaError_t err, const char *what) {
+    cudaGetLastError();  // reported here: the next launch check must not find it again
     set_error("CUDA error in %s: %s (%s)", what, cudaGetErrorName(err), cudaGetErrorString(err));
     return RKB_ECUDA;
 }
