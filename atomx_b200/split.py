@@ -610,7 +610,7 @@ class SplitEngine:
                     else:
                         self._contract(self.grp_out, *self.task_range[gi], self.out, s)
             if shipper is not None:
-                shipper.ship([(k, self.out.data_ptr() + 8 * self.offsets[k]) for k in ks], s)
+                shipper.ship_run([(k, self.out.data_ptr() + 8 * self.offsets[k]) for k in ks], s)
                 continue
             ev = torch.cuda.Event()
             ev.record(s)

@@ -367,20 +367,27 @@ def ship_groups(plan: TablePlan, n_tasks) -> list:
 
 
 class PackedShipper:
-    """Ships finished tables to a pinned host buffer in packed form: a run of
-    consecutive tables is packed on the compute stream into one of two rotating
-    device buffers and copied on the copy stream while the next are computed."""
+    """Ships finished tables to a pinned host buffer in packed form: a table, or a
+    run of consecutive tables, is packed on the compute stream into one of two
+    rotating device buffers and copied on the copy stream while the next are
+    computed.  ``groups``: the runs [(first, stop)] that will be shipped (each
+    table by itself by default); the buffers hold the largest."""
 
-    def __init__(self, plan: TablePlan, host: torch.Tensor, device, copy_stream, groups):
+    def __init__(self, plan: TablePlan, host: torch.Tensor, device, copy_stream, groups=None):
         self.plan, self.host, self.cs = plan, host, copy_stream
         self.offsets = packed_offsets(plan)
         self.size = {k: plan.n_of_k(k) * (plan.n_of_k(k) + 1) // 2 for k in plan.ks}
+        if groups is None:
+            groups = [(i, i + 1) for i in range(len(plan.ks))]
         nmax = max((sum(self.size[k] for k in plan.ks[a:b]) for a, b in groups), default=1)
         self.bufs = [torch.empty(nmax, dtype=torch.float64, device=device) for _ in range(2)]
         self.free = [None, None]
         self.i = 0
 
-    def ship(self, tables, stream) -> None:
+    def ship(self, k: int, table_ptr: int, stream) -> None:
+        self.ship_run([(k, table_ptr)], stream)
+
+    def ship_run(self, tables, stream) -> None:
         """``tables``: [(k, device address)] of consecutive multipoles."""
         L = _native.load()
         b = self.i % 2
@@ -515,7 +522,7 @@ def fp64_tables_to_host(dev: IonDevice, ws: Fp64Workspace, out: torch.Tensor, ho
                                                 ws.nk.data_ptr(), ws.out_off.data_ptr(), ws.tasks.data_ptr() + 12 * t0,
                                                 t1 - t0, out.data_ptr(), h), "rkb_table_contract_fp64")
         if shipper is not None:
-            shipper.ship([(k, out.data_ptr() + 8 * ws.offsets[k]) for k in ks], s)
+            shipper.ship_run([(k, out.data_ptr() + 8 * ws.offsets[k]) for k in ks], s)
             continue
         ev = torch.cuda.Event()
         ev.record(s)
