@@ -239,7 +239,7 @@ def tile_tasks(sizes, tile: int = TILE, order=None, block: int | None = None):
     whole tile row of column panels (more than L2 holds on large tables)."""
     if block is not None:
         return _blocked_tasks(tuple(int(s) for s in np.asarray(sizes).reshape(-1)), tile,
-                              None if order is None else tuple(int(o) for o in order), int(block))
+                              None if order is None else tuple(int(o) for o in order), int(block)).copy()
     nt = (np.asarray(sizes, dtype=np.int64).reshape(-1) + tile - 1) // tile
     groups = np.arange(nt.shape[0]) if order is None else np.asarray(order, dtype=np.int64)
     groups = groups[nt[groups] > 0]
