@@ -186,13 +186,13 @@ class SplitBatch(_Graphable):
         self.b_col0 = [r.b_col0 if cells else 0 for r in self.ions]
         self.b_ld = max(r.kmax_dim - c for r, c in zip(self.ions, self.b_col0)) if cells else self.kpad
         self.resA = _alloc(ws, (self.n_mod, self.rows_alloc, self.kpad), torch.int8, d)
-        self.resB = (_alloc(ws, (self.n_mod, self.rows_alloc, self.b_ld), torch.int8, d)
-                     if any(r.has_z for r in self.ions) and self.b_ld > 0 else None)
+        self._resB = (_alloc(ws, (self.n_mod, self.rows_alloc, self.b_ld), torch.int8, d)
+                      if any(r.has_z for r in self.ions) and self.b_ld > 0 else None)
         # The cell and two-kernel row paths write every column of their rows;
         # the fused kernel only its own.  Padding rows are read by the last
         # tiles (their entries are never stored) and are zeroed all the same.
         full_zero = any(r.kind == "fused" for r in self.ions)
-        for res in (self.resA, self.resB):
+        for res in (self.resA, self._resB):
             if res is not None:
                 (res if full_zero else res[:, nrows:, :]).zero_()
         self.rowscale = _alloc(ws, (nrows,), torch.float64, d)
@@ -242,6 +242,18 @@ class SplitBatch(_Graphable):
         self._c = np.ctypeslib.as_ctypes(np.ascontiguousarray(self.moduli, dtype=np.int32))
 
     @property
+    def resB(self) -> torch.Tensor | None:
+        """The whole B operand, [modulus][row][kpad] like ``resA`` (each ion's
+        columns before its ``b_col0`` are A's), assembled for inspection."""
+        if self._resB is None or not any(self.b_col0):
+            return self._resB
+        out = self.resA.clone()
+        for i, c0 in enumerate(self.b_col0):
+            rows, w = slice(int(self.row_base[i]), int(self.row_base[i + 1])), min(self.b_ld, self.kpad - c0)
+            out[:, rows, c0:c0 + w] = self._resB[:, rows, :w]
+        return out
+
+    @property
     def launches_per_step(self) -> int:
         """Row kernels of every ion, the certificate and the contraction."""
         return sum(2 if r.kind == "two" else 1 for r in self.ions) + 2
@@ -279,7 +291,7 @@ class SplitBatch(_Graphable):
                 if ls not in used:
                     ls.wait_event(fork)
                     used.add(ls)
-            r.launch(self.ion_bits[i], self.n_mod, self._c, self.resA, self.resB, self.kpad, int(self.row_base[i]),
+            r.launch(self.ion_bits[i], self.n_mod, self._c, self.resA, self._resB, self.kpad, int(self.row_base[i]),
                      self.rows_alloc, self.rowscale, self.left, self.right, self.cbound, self.cwp, self.xwork, ls,
                      self.b_col0[i], self.b_ld)
         for ls in used:
@@ -290,7 +302,7 @@ class SplitBatch(_Graphable):
 
     def contract(self, stream=None) -> None:
         L = _native.load()
-        _native.check(L.rkb_split_contract_z(self.resA.data_ptr(), _native.ptr(self.resB), self.kpad, self.b_ld,
+        _native.check(L.rkb_split_contract_z(self.resA.data_ptr(), _native.ptr(self._resB), self.kpad, self.b_ld,
                                              self.rows_alloc, self.n_mod, self._c, self.M,
                                              self.rowscale.data_ptr(), self.left.data_ptr(), self.right.data_ptr(),
                                              self.cbound.data_ptr(), self.corr_floor, self.cw, self.cwp,
