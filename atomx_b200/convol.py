@@ -159,6 +159,8 @@ class ConvolCache:
 
     # ------------------------------------------------------------ building
     def bank(self, k: int, stream=None) -> CellBank:
+        if stream is None:
+            return self.banks((k,))[0]
         with on_stream(stream):
             return self.banks((k,))[0]
 
@@ -173,7 +175,7 @@ class ConvolCache:
             with self._lock:
                 hit = self._cache.get((k, dev))
                 if hit is None:
-                    hit = self._build(k)
+                    hit = self._build(k, handle)
                     hit.home = cur
                     hit.seen.add(handle)
                     self._cache[k, dev] = hit
@@ -184,10 +186,9 @@ class ConvolCache:
             out.append(hit)
         return out
 
-    def _build(self, k: int) -> CellBank:
+    def _build(self, k: int, s: int) -> CellBank:
         L = _native.require_device()
         bd = self.bsp_data
-        s = _native.stream_handle()
         nv, ns = int(bd["nv"]), int(bd["ns"])
         gr, grw = resident(bd["gr"]), resident(bd["grw"])
         ng = int(gr.shape[1])
@@ -376,6 +377,26 @@ def _sizes(bd):
 _CELL_BYTES = 2 << 30
 
 
+def _in_groups(costs, run) -> None:
+    """``run(first, stop)`` over all of ``costs`` in runs of consecutive items
+    whose costs (bytes) add up to _CELL_BYTES at most, or of one item; where the
+    device memory does not hold a run, one item at a time from there on."""
+    limit, a = _CELL_BYTES, 0
+    while a < len(costs):
+        b, size = a + 1, costs[a]
+        while b < len(costs) and size + costs[b] <= limit:
+            size += costs[b]
+            b += 1
+        try:
+            run(a, b)
+        except torch.cuda.OutOfMemoryError:
+            if b == a + 1:
+                raise
+            limit = 0
+            continue
+        a = b
+
+
 def compute_slater_rk_cell_batch(orbital_arrays, keys, bsp_data, cache=None):
     """R^k(ab, cd) for many (a, b, c, d, k) keys (atomx convol.py:2084).
 
@@ -408,18 +429,16 @@ def compute_slater_rk_cell_batch(orbital_arrays, keys, bsp_data, cache=None):
     ru, ir = np.unique(kpos * (n * n) + cd, return_inverse=True)
     lb, rb = (np.searchsorted(u, np.arange(len(ks) + 1) * (n * n)) for u in (lu, ru))
     result = np.empty(len(keys))
-    g0 = 0
-    while g0 < len(ks):  # multipoles together as long as their rows stay below _CELL_BYTES
-        g1 = g0 + 1
-        while g1 < len(ks) and (lb[g1 + 1] - lb[g0] + 2 * (rb[g1 + 1] - rb[g0])) * kdim * 8 <= _CELL_BYTES:
-            g1 += 1
+
+    def run(g0, g1):
         nl, nr = int(lb[g1] - lb[g0]), int(rb[g1] - rb[g0])
         pairs = np.concatenate([lu[lb[g0]:lb[g1]], ru[rb[g0]:rb[g1]]]) % (n * n)
         D = cell_densities(banks[g0], P, Q, np.stack([pairs // n, pairs % n], axis=1), nsp, nsq)
         W = _potentials_of(banks[g0:g1], rb[g0:g1 + 1] - rb[g0], D[nl:nl + nr])
         ents = np.flatnonzero((kpos >= g0) & (kpos < g1))
         result[ents] = to_host(_dots(D[:nl], W, il[ents] - lb[g0], ir[ents] - rb[g0]))
-        g0 = g1
+
+    _in_groups([int(x) * kdim * 8 for x in np.diff(lb) + 2 * np.diff(rb)], run)
     return result.tolist()
 
 
@@ -463,12 +482,9 @@ def cell_tables(P, Q, kappa, bsp_data, k_max: int, cache=None, plan=None, stream
         Pd = P if isinstance(P, torch.Tensor) and P.is_cuda else _stack(list(np.asarray(P)), ns, dev)
         Qd = Q if isinstance(Q, torch.Tensor) and Q.is_cuda else _stack(list(np.asarray(Q)), ns, dev)
         banks = cache.banks(plan.ks)
-        g0 = 0
-        while g0 < len(plan.ks):  # multipoles together as long as their rows stay below _CELL_BYTES
-            kdim, g1, rows = banks[g0].kdim, g0 + 1, sizes[g0]
-            while g1 < len(plan.ks) and 2 * (rows + sizes[g1]) * kdim * 8 <= _CELL_BYTES:
-                rows += sizes[g1]
-                g1 += 1
+        kdim = banks[0].kdim
+
+        def run(g0, g1):
             row0 = np.concatenate([[0], np.cumsum(sizes[g0:g1])]).astype(np.int64)
             pairs = np.concatenate([plan.pairs[plan.pairs_of_k[k]] for k in plan.ks[g0:g1]])
             D = cell_densities(banks[g0], Pd, Qd, pairs, nsp, nsq)
@@ -483,7 +499,8 @@ def cell_tables(P, Q, kappa, bsp_data, k_max: int, cache=None, plan=None, stream
                                                     p + 24 * m, tasks.shape[0], values.data_ptr(),
                                                     _native.stream_handle()),
                           "rkb_table_contract_fp64")
-            g0 = g1
+
+        _in_groups([2 * n * kdim * 8 for n in sizes], run)
     used_on(stream, values, P, Q)
     return RkTables(plan=plan, ks=plan.ks, values=values, offsets={k: int(offs[i]) for i, k in enumerate(plan.ks)},
                     precision="cell")
@@ -669,8 +686,15 @@ def build_hf_matrices_dbsr(targets, P_stack, Q_stack, angular_direct, angular_ex
         dd_ld = max(q_off, ld - q_off)
         # targets in groups whose exchange densities stay below _FOCK_BYTES
         group = min(nt, max(1, min(_FOCK_BYTES // (32 * max(nk, 1) * ns * ns), 65535 // (4 * max(nk, 1)))))
-        work = torch.empty(group * nk * (2 * dd_ld + 2 * ld + 4 * ns * ns) + group * 4 * ns * ns, dtype=torch.float64,
-                           device=dev)
+        work = None
+        while work is None:
+            try:
+                work = torch.empty(group * (nk * (2 * dd_ld + 2 * ld + 4 * ns * ns) + 4 * ns * ns),
+                                   dtype=torch.float64, device=dev)
+            except torch.cuda.OutOfMemoryError:  # fewer targets at a time
+                if group == 1:
+                    raise
+                group = (group + 1) // 2
         kptr = np.array([b.K.data_ptr() for b in banks] + [0], dtype=np.int64)
         for g0 in range(0, nt, group):
             g1 = min(nt, g0 + group)
