@@ -284,23 +284,18 @@ def _fp64_engine(dev, stream):
 
 
 def _fp64_rows_rate(dev, ws, stream, flush, reps: int = 5) -> dict:
-    """The plain engine's Y^k row kernel alone (g and Y^k rows of the whole
-    table): CUDA events on the launch stream after an L2 flush, median of
-    ``reps``, against the HBM peak.  Algorithmic bytes: the orbital values
-    read once and the g and Y rows written."""
-    import torch
-
+    """The plain engine's Y^k rows alone (g and Y^k rows of the whole table, as
+    the engine launches them, with the power table they read): CUDA events on
+    the launch stream after an L2 flush, median of ``reps``, against the HBM
+    peak.  Algorithmic bytes: the orbital values read once and the g and Y
+    rows written."""
     from atomx_b200 import _native
-    L = _native.load()
+    from atomx_b200 import tables as T
     plan = dev.plan
     h = _native.stream_handle(stream)
 
     def launch():
-        _native.check(L.rkb_table_rows_fp64(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
-                                            dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows,
-                                            dev.r.data_ptr(), dev.w.data_ptr(), dev.nv, dev.ng, dev.mo.data_ptr(),
-                                            dev.mi.data_ptr(), ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, h),
-                      "rkb_table_rows_fp64")
+        T._fp64_rows(dev, ws, h)
 
     launch()
     ms = float(statistics.median(_time_steps(launch, reps, flush, stream)))
@@ -330,13 +325,11 @@ def _fp64_roofline(dev, ws, out, stream, flush):
     import torch
 
     from atomx_b200 import _native
+    from atomx_b200 import tables as T
     L = _native.load()
     plan = dev.plan
     s = _native.stream_handle(stream)
-    _native.check(L.rkb_table_rows_fp64(dev.Pv.data_ptr(), dev.Qv.data_ptr(), dev.n, dev.pairs.data_ptr(),
-                                        dev.row_pair.data_ptr(), dev.row_k.data_ptr(), plan.n_rows, dev.r.data_ptr(),
-                                        dev.w.data_ptr(), dev.nv, dev.ng, dev.mo.data_ptr(), dev.mi.data_ptr(),
-                                        ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, s), "rkb_table_rows_fp64")
+    T._fp64_rows(dev, ws, s)
 
     def contract():
         _native.check(L.rkb_table_contract_fp64(ws.g.data_ptr(), ws.y.data_ptr(), ws.ld, ws.ld, ws.row0.data_ptr(),
@@ -431,7 +424,7 @@ def run_gpu(args):
         launches_per_step = eng.launches_per_step
     else:
         step, out64, ws = _fp64_engine(dev, stream)
-        launches_per_step = 2
+        launches_per_step = 2 + (ws.pow is not None)  # the rows and the powers they read, the contraction
 
     for _ in range(args.warmup):
         step()
