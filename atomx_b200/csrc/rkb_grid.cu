@@ -24,9 +24,9 @@
 // The reference runs them serially per row.  Here one CTA owns a row and cuts it into
 // tiles of TILE points, a warp per tile: a first pass sums every tile's terms, a scan over
 // the tiles gives each its two carries, and a second pass scans inside the tiles and
-// forms y and its dots with up to FUSED consumers (a row with more takes the second
-// pass again).  No tile waits for another, the batch stores no y, and all loads are
-// coalesced (consecutive lanes, consecutive points).  Sums are formed without
+// forms y and its dots with up to FUSED consumers; a row with more puts y into shared
+// memory, and a warp per consumer dots it from there.  No tile waits for another, and all
+// loads are coalesced (consecutive lanes, consecutive points).  Sums are formed without
 // subtractions: a difference of partial sums would cancel on grids whose terms grow
 // along the row.  The summation order differs from the serial one, so results agree
 // with the reference to rounding, not bit for bit.
@@ -34,15 +34,20 @@
 // Bound by instruction issue (two passes of nine loads and about fifteen FP64
 // operations a point, two warp scans in the second).  4000 rows x 20 000 points with 2
 // consumers: tile after tile with block-wide scans and y in memory 2.87 ms, this form
-// 1.10 ms (tiles of 64, 192, 256 points: 1.2 to 1.4 ms).
+// 1.07 ms (tiles of 64, 192, 256 points: 1.2 to 1.4 ms).  More consumers than FUSED by
+// taking the second pass again: 4000 rows x 300 points with 40 841 us, 500 rows x 20 000
+// points with 64 2.27 ms, from shared memory 131 us and 0.72 ms (from device memory, tile
+// after tile, 0.49 and 1.99 ms).  A block takes a warp per tile, up to eight: 4000 rows x
+// 300 points with 2 consumers 77 us, with eight warps 135 us.
 #include "rkb_common.cuh"
 
 namespace rkb {
 namespace grid {
 
-constexpr int THREADS = 256, WARPS = THREADS / 32;
+constexpr int THREADS = 256, WARPS = THREADS / 32;  // at most; a short row takes a warp per tile
 constexpr int CH = 4, TILE = 32 * CH;  // chunks of 32 points per tile
 constexpr int FUSED = 4;               // consumers dotted in one second pass
+constexpr int Y_TILES = 64;            // tiles of y that shared memory holds for more consumers
 constexpr unsigned FULL = 0xffffffffu;
 
 struct Tables {
@@ -252,15 +257,17 @@ struct BatchArgs {
     double *val;  // consumer dots
     double *y;    // y rows (ld y_ld) when W is null
     long y_ld;
+    int y_tiles;  // rows with more than FUSED consumers take y through shared memory, that many tiles at a time (or 0)
 };
 
 template <bool DOTS>
 __global__ void __launch_bounds__(THREADS, 3) grid_rows_kernel(const __grid_constant__ BatchArgs a, double *scratch) {
     extern __shared__ double tiles_sh[];
     __shared__ double dots_sh[WARPS * FUSED];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int ntiles = (int)((a.n + TILE - 1) / TILE), live = (int)(a.i_cut / TILE) + 1;  // tiles with an output
     double *in = scratch ? scratch + 2L * ntiles * blockIdx.x : tiles_sh, *out = in + ntiles;
+    double *y_sh = tiles_sh + (scratch ? 0 : 2 * ntiles);
     for (long m = blockIdx.x; m < a.nrows; m += gridDim.x) {
         if (a.rows_ok && !a.rows_ok[m]) continue;
         const long s0 = DOTS ? a.cons_ptr[m] : 0, s1 = DOTS ? a.cons_ptr[m + 1] : 1;
@@ -281,7 +288,7 @@ __global__ void __launch_bounds__(THREADS, 3) grid_rows_kernel(const __grid_cons
             return q < T.ncuts - 1 && T.cuts[q] <= base + TILE;
         };
         // ---- the tiles' sums
-        for (int c = warp; c < ntiles; c += WARPS) {
+        for (int c = warp; c < ntiles; c += warps) {
             const long base = (long)c * TILE;
             const bool cut = has_cut(base);
             double si, so;
@@ -296,6 +303,33 @@ __global__ void __launch_bounds__(THREADS, 3) grid_rows_kernel(const __grid_cons
         if (warp == 0) carry_scan<false>(T, in, ntiles, lane);
         if (warp == 1) carry_scan<true>(T, out, ntiles, lane);
         __syncthreads();
+        // ---- many consumers: y into shared memory, and a warp per consumer
+        if (DOTS && a.y_tiles && s1 - s0 > FUSED) {
+            for (int c0 = 0; c0 < live; c0 += a.y_tiles) {
+                for (int c = c0 + warp; c < min(live, c0 + a.y_tiles); c += warps) {
+                    const long base = (long)c * TILE;
+                    const bool cut = has_cut(base);
+                    double y[CH];
+                    if (cut || base == 0 || base + TILE >= T.n) tile_y<true>(T, rho, base, cut, lane, in[c], out[c], y);
+                    else tile_y<false>(T, rho, base, false, lane, in[c], out[c], y);
+#pragma unroll
+                    for (int j = 0; j < CH; ++j) y_sh[(c - c0) * TILE + 32 * j + lane] = y[j];
+                }
+                __syncthreads();
+                const long first = (long)c0 * TILE;
+                const int pts = (int)min((long)a.y_tiles * TILE, a.i_cut + 1 - first);
+                for (long s = s0 + warp; s < s1; s += warps) {
+                    const double *w = a.W + a.cons_rho[s] * a.w_ld + first;
+                    double part = 0.0;
+#pragma unroll 4
+                    for (int i = lane; i < pts; i += 32) part = fma(__ldg(w + i), y_sh[i], part);
+                    part = warp_sum(part);
+                    if (lane == 0) a.val[s] = c0 ? a.val[s] + part : part;
+                }
+                __syncthreads();
+            }
+            continue;
+        }
         // ---- y, and its dots with FUSED consumers at a time
         for (long s = s0; s < s1; s += FUSED) {
             const double *w[FUSED];
@@ -306,7 +340,7 @@ __global__ void __launch_bounds__(THREADS, 3) grid_rows_kernel(const __grid_cons
                     w[q] = a.W + a.cons_rho[s + q < s1 ? s + q : s] * a.w_ld + lane;
                     part[q] = 0.0;
                 }
-            for (int c = warp; c < live; c += WARPS) {
+            for (int c = warp; c < live; c += warps) {
                 const long base = (long)c * TILE;
                 const bool cut = has_cut(base);
                 double y[CH];
@@ -332,7 +366,7 @@ __global__ void __launch_bounds__(THREADS, 3) grid_rows_kernel(const __grid_cons
             __syncthreads();
             if (threadIdx.x < FUSED && s + threadIdx.x < s1) {
                 double v = 0.0;
-                for (int x = 0; x < WARPS; ++x) v += dots_sh[x * FUSED + threadIdx.x];
+                for (int x = 0; x < warps; ++x) v += dots_sh[x * FUSED + threadIdx.x];
                 a.val[s + threadIdx.x] = v;
             }
             __syncthreads();
@@ -353,16 +387,29 @@ static int grid_common_checks(long n, long ncuts, long ntr, long i_cut) {
     return RKB_OK;
 }
 
+// max_cons: the most consumers of a row, or -1 if that is not known here.
 template <bool DOTS>
-static int launch_rows(const grid::BatchArgs &a, cudaStream_t st) {
+static int launch_rows(grid::BatchArgs &a, long max_cons, cudaStream_t st) {
     auto kern = grid::grid_rows_kernel<DOTS>;
-    long ctas = a.nrows < 8L * sm_count() ? a.nrows : 8L * sm_count();
-    const size_t bytes = sizeof(double) * 2 * (size_t)ceil_div(a.n, grid::TILE);  // the tiles' sums and carries
-    double *scratch = nullptr;
+    const long tiles = ceil_div(a.n, grid::TILE);
+    const int warps = tiles < 2 ? 2 : tiles < grid::WARPS ? (int)tiles : grid::WARPS;  // the carries take two
+    const long most = 8L * sm_count() * grid::WARPS / warps;
+    long ctas = a.nrows < most ? a.nrows : most;
+    size_t bytes = sizeof(double) * 2 * (size_t)tiles;  // the tiles' sums and carries
     const bool fits = bytes <= 200 * 1024;
-    if (fits) {
-        RKB_CUDA(set_smem(kern, (int)bytes));
-    } else {  // above 1 638 400 points they go to device memory (n / 8 bytes a CTA): fewer CTAs where that is short
+    // Shared memory for y costs L1 (4000 rows x 5000 points with two consumers: 457 us, 477 with it), so it is
+    // taken where rows have, or may have, more consumers than one second pass serves.
+    const long live = a.i_cut / grid::TILE + 1;
+    const int y_tiles = live < grid::Y_TILES ? (int)live : grid::Y_TILES;
+    const size_t y_bytes = sizeof(double) * grid::TILE * (size_t)y_tiles;
+    size_t smem = fits ? bytes : 0;
+    if (DOTS && (max_cons < 0 || max_cons > grid::FUSED) && smem + y_bytes <= 200 * 1024) {
+        a.y_tiles = y_tiles;
+        smem += y_bytes;
+    }
+    double *scratch = nullptr;
+    RKB_CUDA(set_smem(kern, (int)smem));
+    if (!fits) {  // above 1 638 400 points they go to device memory (n / 8 bytes a CTA): fewer CTAs where that is short
         cudaError_t e;
         while ((e = cudaMallocAsync(reinterpret_cast<void **>(&scratch), bytes * ctas, st)) == cudaErrorMemoryAllocation &&
                ctas > 1) {
@@ -371,7 +418,7 @@ static int launch_rows(const grid::BatchArgs &a, cudaStream_t st) {
         }
         RKB_CUDA(e);
     }
-    kern<<<(unsigned)ctas, grid::THREADS, fits ? bytes : 0, st>>>(a, scratch);
+    kern<<<(unsigned)ctas, 32 * warps, smem, st>>>(a, scratch);
     const cudaError_t e = cudaGetLastError(), f = scratch ? cudaFreeAsync(scratch, st) : cudaSuccess;
     if (e != cudaSuccess) return cuda_status(e, "grid_rows_kernel");
     RKB_CUDA(f);
@@ -390,7 +437,29 @@ extern "C" int rkb_grid_yk_rows(const double *d_rho, long rho_ld, const long *d_
     a.rho = d_rho; a.rho_ld = rho_ld; a.rows_k = d_rows_k; a.nrows = nrows;
     a.r = d_r; a.RK = d_RK; a.inverse = d_inverse; a.transfers = d_transfers; a.cuts = d_cuts;
     a.n = n; a.ncuts = ncuts; a.ntr = ntr; a.i_cut = i_cut; a.y = d_y; a.y_ld = y_ld;
-    return launch_rows<false>(a, as_stream(stream));
+    return launch_rows<false>(a, 0, as_stream(stream));
+}
+
+extern "C" int rkb_grid_pair_dot_batch_cons(const double *d_PA, const double *d_QA, const double *d_PB,
+                                       const double *d_QB, long ld, const long *d_rows_a, const long *d_rows_b,
+                                       const long *d_rows_k, const unsigned char *d_rows_ok, long nrows,
+                                       const double *d_W, long w_ld, const long *d_cons_ptr,
+                                       const long *d_cons_rho, const double *d_r, long n, const double *d_RK,
+                                       const double *d_inverse, const long *d_cuts, long ncuts,
+                                       const double *d_transfers, long ntr, long i_cut, double *d_val,
+                                       long max_cons, void *stream) {
+    int st = grid_common_checks(n, ncuts, ntr, i_cut);
+    if (st != RKB_OK) return st;
+    RKB_CHECK_ARG(ld >= n && w_ld >= i_cut + 1, "row strides too small (ld=%ld, w_ld=%ld)", ld, w_ld);
+    RKB_CHECK_ARG(max_cons >= -1, "invalid number of consumers");
+    if (nrows == 0) return RKB_OK;
+    grid::BatchArgs a = {};
+    a.PA = d_PA; a.QA = d_QA; a.PB = d_PB; a.QB = d_QB; a.ld = ld; a.rows_a = d_rows_a; a.rows_b = d_rows_b;
+    a.rows_k = d_rows_k; a.rows_ok = d_rows_ok; a.nrows = nrows; a.W = d_W; a.w_ld = w_ld;
+    a.cons_ptr = d_cons_ptr; a.cons_rho = d_cons_rho; a.r = d_r; a.RK = d_RK; a.inverse = d_inverse;
+    a.transfers = d_transfers; a.cuts = d_cuts; a.n = n; a.ncuts = ncuts; a.ntr = ntr; a.i_cut = i_cut;
+    a.val = d_val;
+    return launch_rows<true>(a, max_cons, as_stream(stream));
 }
 
 extern "C" int rkb_grid_pair_dot_batch(const double *d_PA, const double *d_QA, const double *d_PB,
@@ -401,16 +470,8 @@ extern "C" int rkb_grid_pair_dot_batch(const double *d_PA, const double *d_QA, c
                                        const double *d_inverse, const long *d_cuts, long ncuts,
                                        const double *d_transfers, long ntr, long i_cut, double *d_val,
                                        double *d_work, long work_rows, void *stream) {
-    int st = grid_common_checks(n, ncuts, ntr, i_cut);
-    if (st != RKB_OK) return st;
-    RKB_CHECK_ARG(ld >= n && w_ld >= i_cut + 1, "row strides too small (ld=%ld, w_ld=%ld)", ld, w_ld);
     RKB_CHECK_ARG(d_work != nullptr && work_rows >= 1, "a work area of at least one row is required");
-    if (nrows == 0) return RKB_OK;
-    grid::BatchArgs a = {};
-    a.PA = d_PA; a.QA = d_QA; a.PB = d_PB; a.QB = d_QB; a.ld = ld; a.rows_a = d_rows_a; a.rows_b = d_rows_b;
-    a.rows_k = d_rows_k; a.rows_ok = d_rows_ok; a.nrows = nrows; a.W = d_W; a.w_ld = w_ld;
-    a.cons_ptr = d_cons_ptr; a.cons_rho = d_cons_rho; a.r = d_r; a.RK = d_RK; a.inverse = d_inverse;
-    a.transfers = d_transfers; a.cuts = d_cuts; a.n = n; a.ncuts = ncuts; a.ntr = ntr; a.i_cut = i_cut;
-    a.val = d_val;
-    return launch_rows<true>(a, as_stream(stream));
+    return rkb_grid_pair_dot_batch_cons(d_PA, d_QA, d_PB, d_QB, ld, d_rows_a, d_rows_b, d_rows_k, d_rows_ok, nrows, d_W,
+                                        w_ld, d_cons_ptr, d_cons_rho, d_r, n, d_RK, d_inverse, d_cuts, ncuts,
+                                        d_transfers, ntr, i_cut, d_val, -1, stream);
 }

@@ -7,10 +7,10 @@ The Green action r_<^k / r_>^(k+1) is applied by two cumulative trapezoid
 scans in block-scaled frames (``coulomb_tables``, after quadrature.py:190-231:
 within a frame the powers are taken relative to the frame's first radius,
 and carried moments change frame by a factor <= 1). The scans run on the GPU
-(``rkb_grid_yk_rows`` / ``rkb_grid_pair_dot_batch``): one CTA per row, with
-block-wide prefix sums inside each frame. Rows are independent. The
-summation order inside a frame differs from atomx's serial loop, so values
-agree with it to rounding.
+(``rkb_grid_yk_rows`` / ``rkb_grid_pair_dot_batch_cons``): one CTA per row,
+which is cut into tiles of points whose sums, and the carries between them, are
+formed side by side. Rows are independent. The summation order differs from
+atomx's serial loop, so values agree with it to rounding.
 
 Inputs may be numpy arrays (results come back as numpy, like atomx) or CUDA
 tensors (results stay on the device). Errors follow atomx: a non-increasing,
@@ -186,14 +186,15 @@ def yk_pair_dot_batch_on_grid(PA, QA, PB, QB, rows_a, rows_b, rows_k, rows_ok, R
     ok = torch.as_tensor(np.asarray(rows_ok.cpu() if is_device_tensor(rows_ok) else rows_ok, dtype=np.uint8),
                          device=dev)
     nrows = int(rows_k_h.shape[0])
-    _native.check(L.rkb_grid_pair_dot_batch(mats[0].data_ptr(), mats[1].data_ptr(), mats[2].data_ptr(),
-                                            mats[3].data_ptr(), ld, idx[0].data_ptr(), idx[1].data_ptr(),
-                                            idx[2].data_ptr(), ok.data_ptr(), nrows, W.data_ptr(), W.shape[1],
-                                            idx[3].data_ptr(), idx[4].data_ptr(), tab.r.data_ptr(), n,
-                                            tab.RK.data_ptr(), tab.inverse.data_ptr(), tab.cuts.data_ptr(),
-                                            tab.ncuts, tab.transfers.data_ptr(), tab.ntr, ic, val.data_ptr(),
-                                            val.data_ptr(), 1, _native.stream_handle()),
-                  "rkb_grid_pair_dot_batch")
+    most = int(np.diff(cons_ptr_h).max(initial=0))
+    _native.check(L.rkb_grid_pair_dot_batch_cons(mats[0].data_ptr(), mats[1].data_ptr(), mats[2].data_ptr(),
+                                                 mats[3].data_ptr(), ld, idx[0].data_ptr(), idx[1].data_ptr(),
+                                                 idx[2].data_ptr(), ok.data_ptr(), nrows, W.data_ptr(), W.shape[1],
+                                                 idx[3].data_ptr(), idx[4].data_ptr(), tab.r.data_ptr(), n,
+                                                 tab.RK.data_ptr(), tab.inverse.data_ptr(), tab.cuts.data_ptr(),
+                                                 tab.ncuts, tab.transfers.data_ptr(), tab.ntr, ic, val.data_ptr(),
+                                                 most, _native.stream_handle()),
+                  "rkb_grid_pair_dot_batch_cons")
     return val if on_dev else val.cpu().numpy()
 
 

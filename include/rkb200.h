@@ -123,7 +123,7 @@ int rkb_slater_direct(const double *d_rho13, const double *d_rho24, const double
  * 0..i_cut and, for each consumer slot s in [d_cons_ptr[m], d_cons_ptr[m+1]),
  * writes d_val[s] = sum_i W[d_cons_rho[s]][i] Y_i (W rows of stride w_ld).
  * Rows with d_rows_ok[m] == 0 leave their slots untouched (zero them first).
- * d_work (not null) and work_rows (>= 1) are not used: y is not stored.
+ * d_work (not null) and work_rows (>= 1) are not used.
  * ------------------------------------------------------------------------- */
 int rkb_grid_yk_rows(const double *d_rho, long rho_ld, const long *d_rows_k, long nrows,
                      const double *d_r, long n, const double *d_RK, const double *d_inverse,
@@ -138,6 +138,16 @@ int rkb_grid_pair_dot_batch(const double *d_PA, const double *d_QA, const double
                             const double *d_inverse, const long *d_cuts, long ncuts,
                             const double *d_transfers, long ntr, long i_cut, double *d_val,
                             double *d_work, long work_rows, void *stream);
+/* The same told the largest number of consumers of a row (or -1), by which the
+ * launch chooses how much shared memory it takes. */
+int rkb_grid_pair_dot_batch_cons(const double *d_PA, const double *d_QA, const double *d_PB,
+                            const double *d_QB, long ld, const long *d_rows_a, const long *d_rows_b,
+                            const long *d_rows_k, const unsigned char *d_rows_ok, long nrows,
+                            const double *d_W, long w_ld, const long *d_cons_ptr,
+                            const long *d_cons_rho, const double *d_r, long n, const double *d_RK,
+                            const double *d_inverse, const long *d_cuts, long ncuts,
+                            const double *d_transfers, long ntr, long i_cut, double *d_val,
+                            long max_cons, void *stream);
 
 /* ---------------------------------------------------------------------------
  * Plain FP64 table engine (all arithmetic in FP64).
