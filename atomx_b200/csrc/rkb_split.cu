@@ -832,16 +832,19 @@ __device__ __forceinline__ void cell_rows_body(const RowsArgs &a, const ResidueA
     }
 }
 
-template <int NG>
+template <int NG, int R>
 __global__ void __launch_bounds__(256, 2) split_rows_cell_kernel(const __grid_constant__ RowsArgs a,
                                                               const __grid_constant__ ResidueArgs f,
                                                               const double *__restrict__ ktab_t,
                                                               const long *__restrict__ koff_t, int zmax) {
-    constexpr int R = cell_rows(NG);
     extern __shared__ __align__(16) double sm[];
     double *img = sm;                                          // [R][cell_image]
     double *red = sm + R * cell_image(NG, a.nv, zmax);           // block scratch (cell_scratch doubles)
     const long q0 = (long)blockIdx.x * R;
+    if (R == 1) {
+        cell_rows_body<NG, 1>(a, f, ktab_t, koff_t, q0, zmax, img, red);
+        return;
+    }
     bool same = q0 + R <= a.nrows;
     for (int r = 1; same && r < R; ++r) same = a.row_k[q0 + r] == a.row_k[q0];
     if (same) {
@@ -855,7 +858,7 @@ __global__ void __launch_bounds__(256, 2) split_rows_cell_kernel(const __grid_co
     }
 }
 // doubles of block scratch: warp sums and maxima, the core vectors and moments, the scales
-constexpr int cell_scratch(int ng) { return cell_rows(ng) * (8 * 4 + 2 * ng + 2 + 1); }
+constexpr int cell_scratch(int ng, int rows) { return rows * (8 * 4 + 2 * ng + 2 + 1); }
 
 // =========================================================================
 // K3s — tcgen05 INT8 residue SYRK with CRT epilogue
@@ -1510,6 +1513,12 @@ extern "C" int rkb_split_rows(const double *d_Pv, const double *d_Qv, long orb_l
     return RKB_OK;
 }
 
+// Rows up to which a block takes one: with R at a time fewer blocks than SMs are left, and blocks at
+// a change of multipole take their rows one after another.  R rows and one row a block in us: ng = 8
+// (R = 4, 105 cells) 114 rows 36 and 17, 801 rows 38 and 28, 1 656 rows 38 and 38, 3 114 rows 56 and
+// 63; ng = 11 (R = 2, 142 cells) 32 and 21, 36 and 36, 52 and 59, 89 and 96.
+static long cell_single(int ng) { return 2L * cell_rows(ng) * sm_count(); }
+
 extern "C" int rkb_split_rows_cells_z(const double *d_Pv, const double *d_Qv, long orb_ld, const long *d_pairs,
                                       const long *d_row_pair, const int *d_row_k, long nrows, const double *d_w,
                                       int nv, int ng, const double *d_ktab, const long *d_koff,
@@ -1551,8 +1560,8 @@ extern "C" int rkb_split_rows_cells_z(const double *d_Pv, const double *d_Qv, lo
     a.resA = d_resA; a.resB = d_resB; a.kpad = kpad; a.row_base = row_base; a.nrows_total = nrows_total;
     a.rowscale = d_rowscale; a.left = d_left; a.right = d_right; a.cbound = d_cbound; a.cwp = cwp;
     RKB_CHECK_ARG(d_ktab_t != nullptr && d_koff_t != nullptr, "the cell-minor factor tables are required");
-    const int rows = cell_rows(ng);
-    const size_t smem = sizeof(double) * (size_t)(rows * cell_image(ng, nv, max_z) + cell_scratch(ng));
+    const int rows = nrows <= cell_single(ng) ? 1 : cell_rows(ng);
+    const size_t smem = sizeof(double) * (size_t)(rows * cell_image(ng, nv, max_z) + cell_scratch(ng, rows));
     RKB_CHECK_ARG(smem <= 200 * 1024, "row images too large for shared memory");
     ResidueArgs f = {};
     for (int i = 0; i < n_mod; ++i) {
@@ -1562,10 +1571,14 @@ extern "C" int rkb_split_rows_cells_z(const double *d_Pv, const double *d_Qv, lo
     }
     cudaStream_t st = as_stream(stream);
     const dim3 grid((unsigned)ceil_div(nrows, rows)), block((unsigned)threads);
-#define RKB_CELL_CASE(NGV)                                                                      \
-    case NGV:                                                                                   \
-        RKB_CUDA(set_smem(split_rows_cell_kernel<NGV>, (int)smem));                             \
-        split_rows_cell_kernel<NGV><<<grid, block, smem, st>>>(a, f, d_ktab_t, d_koff_t, max_z); \
+#define RKB_CELL_LAUNCH(NGV, RV)                                                                        \
+    {                                                                                                   \
+        RKB_CUDA(set_smem(split_rows_cell_kernel<NGV, RV>, (int)smem));                                 \
+        split_rows_cell_kernel<NGV, RV><<<grid, block, smem, st>>>(a, f, d_ktab_t, d_koff_t, max_z);    \
+    }
+#define RKB_CELL_CASE(NGV)                                                                              \
+    case NGV:                                                                                           \
+        if (rows == 1) RKB_CELL_LAUNCH(NGV, 1) else RKB_CELL_LAUNCH(NGV, cell_rows(NGV))                \
         break;
     switch (ng) {
         RKB_CELL_CASE(5) RKB_CELL_CASE(6) RKB_CELL_CASE(7) RKB_CELL_CASE(8) RKB_CELL_CASE(9) RKB_CELL_CASE(10)
@@ -1573,6 +1586,7 @@ extern "C" int rkb_split_rows_cells_z(const double *d_Pv, const double *d_Qv, lo
             RKB_CELL_CASE(11)
     }
 #undef RKB_CELL_CASE
+#undef RKB_CELL_LAUNCH
     RKB_LAUNCHED("split_rows_cell_kernel");
     return RKB_OK;
 }
