@@ -597,7 +597,7 @@ class SplitEngine:
         fp64 = set(self._failing(self.est.cpu().numpy())) if flagged else set()
         self.escalated = sorted(fp64)
         # failing tables go to FP64 before the split ones around them are shipped
-        groups = ship_groups(plan, [t1 - t0 for t0, t1 in self.task_range])
+        groups = ship_groups([t1 - t0 for t0, t1 in self.task_range])
         shipper = PackedShipper(plan, host, self.out.device, cs, groups) if packed else None
         for a, b in groups:
             ks = plan.ks[a:b]

@@ -351,11 +351,11 @@ class HostPackedTables:
         return self.plan.unique_entries
 
 
-def ship_groups(plan: TablePlan, n_tasks) -> list:
-    """Runs of consecutive multipoles [(first, stop)] (indices into plan.ks) to
-    contract in one launch and copy together: small tables share a launch that
-    fills the GPU, a large one goes alone so that its copy overlaps the next.
-    ``n_tasks[i]``: 128 x 128 tiles of table i."""
+def ship_groups(n_tasks) -> list:
+    """Runs of consecutive tables [(first, stop)] to contract in one launch and
+    copy together: a run ends with the table that brings it to two tiles per SM,
+    so that small tables share a launch that fills the GPU and the copy of a run
+    overlaps the next.  ``n_tasks[i]``: 128 x 128 tiles of table i."""
     full = 2 * torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
     out, first, tiles = [], 0, 0
     for i, m in enumerate(n_tasks):
@@ -513,7 +513,7 @@ def fp64_tables_to_host(dev: IonDevice, ws: Fp64Workspace, out: torch.Tensor, ho
     h = _native.stream_handle(s)
     plan = dev.plan
     _fp64_rows(dev, ws, h)
-    groups = ship_groups(plan, [t1 - t0 for t0, t1 in ws.task_range])
+    groups = ship_groups([t1 - t0 for t0, t1 in ws.task_range])
     shipper = PackedShipper(plan, host, out.device, cs, groups) if packed else None
     for a, b in groups:
         t0, t1 = ws.task_range[a][0], ws.task_range[b - 1][1]

@@ -258,7 +258,7 @@ int rkb_exchange_matrix(const double *d_fb, const double *d_bsp, const double *d
  * weights follow from the moduli, and pair_inv, f_hi and f_lo are not read),
  * scaled and corrected, and written (and
  * mirrored) into the n x n block at d_out + d_grp_out[g], as
- * rkb_table_contract_fp64 does.  The FP64 core correction of a 32 x 64 block
+ * rkb_table_contract_fp64 does.  The FP64 core correction of a 32 x 32 block
  * is skipped when its bound from d_cbound (relative to 2^(e_a + e_b), which
  * the Schwarz scale of every entry exceeds) is <= corr_floor; pass 0 to
  * always apply it.  Device waits are bounded; *d_status (device
